@@ -994,6 +994,145 @@ __device__ __forceinline__ bool in_box(const float4 b, float px, float py) {
     return px >= b.x && px <= b.z && py >= b.y && py <= b.w;
 }
 
+// ---------------------------------------------------------------- pixel groups
+// A CTA composites a square of side 8 (64 threads) or 16 (256 threads) pixels; warp w owns an 8x4 block of it and
+// each 8 lanes of the warp a 4x2 group of that block, so neighbouring lanes stay neighbouring pixels.  Each group
+// walks its own list of the staged splats that can reach it, so the four groups of a warp evaluate four different
+// splats at once.  A splat of a few pixels meets 1.6 of the eight 4x2 groups of an 8x8 tile it is listed in on
+// average, against 1.1 of its two 8x4 warps, of whose lanes 14 % then hold a valid pair (1M-splat mixture,
+// 1600x1200): the warps execute 0.49 evaluations per listed splat instead of 1.13.  Smaller groups save little
+// more (2x2: 0.43, one pixel: 0.37) and give up the broadcast reads of the staged records.
+constexpr int kGroupLanes = 8;
+
+struct PixelSlot {
+    int x, y;  // pixel within the CTA's square
+};
+__device__ __forceinline__ PixelSlot pixel_slot(int tid, int side) {
+    const int lane = tid & 31, warp = tid >> 5, per_row = side >> 3;
+    const int wy = warp / per_row, wx = warp - wy * per_row;
+    return PixelSlot{wx * 8 + ((lane >> 3) & 1) * 4 + (lane & 3), wy * 4 + (lane >> 4) * 2 + ((lane >> 2) & 1)};
+}
+
+// Bits of the 4x2 groups of row band k (two pixel rows) whose columns are set in `cols`, in the order
+// group = warp * 4 + (lane >> 3) of pixel_slot.
+__device__ __forceinline__ uint32_t band_bits(uint32_t cols, int k, int side) {
+    if (side == 8) return cols << (2 * k);
+    return ((cols & 3u) | ((cols >> 2) << 4)) << ((k >> 1) * 8 + (k & 1) * 2);
+}
+
+// The groups of the square with corner pixel (X0, Y0) that a splat can reach: a superset of the groups holding a
+// pixel whose pair is valid.  The region of validity is the one cull_box bounds by a box -- the image of a UV
+// square, united with a disk around the projected centre; here it is intersected with each two-row band, which
+// drops the corners of the box that a turned square does not cover (a third of the (warp, splat) pairs the box
+// keeps).  The quadrilateral is widened by a quarter pixel plus terms for its extent and for its distance from
+// the origin (FP32 rounding of the pair evaluation: its error is a few units of the pixel coordinate's last
+// place).  A square seen so obliquely that the homography's denominator varies more than tenfold over it keeps
+// the whole box.
+__device__ __forceinline__ uint32_t group_mask(const float4 xyo, const float4 m0, const float4 m1, const float4 m2,
+                                               bool textured, float range_x, float range_y, float g_weight,
+                                               bool tex_square, int X0, int Y0, int side) {
+    const int bands = side >> 1, cols = side >> 2;
+    const uint32_t all = side == 8 ? 0xffu : 0xffffffffu;
+    const float4 box = cull_box(xyo, m0, m1, m2, textured, range_x, range_y, g_weight, tex_square);
+    if (box.x == -INFINITY) return all;  // unbounded
+    const float fx0 = (float)X0 + 0.5f, fy0 = (float)Y0 + 0.5f, last = (float)(side - 1);
+    if (box.z < fx0 || box.x > fx0 + last || box.w < fy0 || box.y > fy0 + last) return 0u;
+    // cull_box found a bound, so these are finite and the denominators have one sign
+    const float opac = xyo.z;
+    const float K = (textured ? (1.f / (255.f * opac) - 0.998f + g_weight) / g_weight : 1.f / (255.f * opac)) * 0.999f;
+    const float sig1 = K >= 1.f ? 0.f : -logf(K) * 1.001f + 1e-3f;
+    const float rs = sqrtf(2.f * sig1), rd = sqrtf(sig1);
+    const float hx = textured && tex_square ? fmaxf(rs, range_x) : rs;
+    const float hy = textured && tex_square ? fmaxf(rs, range_y) : rs;
+    float qx[4], qy[4], sl[4];
+    float zmin = INFINITY, zmax = 0.f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {  // in order around the square
+        const float u = (c == 1 || c == 2) ? hx : -hx, v = c >= 2 ? hy : -hy;
+        const float Z = m2.x * u + m2.y * v + m2.z, iz = 1.f / Z;
+        qx[c] = (m0.x * u + m0.y * v + m0.z) * iz;
+        qy[c] = (m1.x * u + m1.y * v + m1.z) * iz;
+        zmin = fminf(zmin, fabsf(Z));
+        zmax = fmaxf(zmax, fabsf(Z));
+    }
+    const bool tight = zmin > 0.1f * zmax;
+    const float mg = 0.25f + 1e-3f * ((box.z - box.x) + (box.w - box.y)) +
+                     2e-6f * (fmaxf(fabsf(box.x), fabsf(box.z)) + fmaxf(fabsf(box.y), fabsf(box.w)));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float dy = qy[(i + 1) & 3] - qy[i];
+        sl[i] = dy != 0.f ? (qx[(i + 1) & 3] - qx[i]) / dy : 0.f;  // (a level edge's corners end its neighbours)
+    }
+    const float r = rd + mg, r2 = r * r;
+    uint32_t mask = 0u;
+    for (int k = 0; k < bands; ++k) {
+        const float ya = fy0 + (float)(2 * k), yb = ya + 1.f;  // the band's pixel centres
+        float lo = INFINITY, hi = -INFINITY;
+        if (tight) {
+            const float a = ya - mg, b = yb + mg;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float y0 = qy[i], y1 = qy[(i + 1) & 3];
+                const float e0 = fminf(y0, y1), e1 = fmaxf(y0, y1);
+                if (e1 < a || e0 > b) continue;
+                const float xa = qx[i] + (fminf(fmaxf(a, e0), e1) - y0) * sl[i];
+                const float xb = qx[i] + (fminf(fmaxf(b, e0), e1) - y0) * sl[i];
+                lo = fminf(lo, fminf(xa, xb));
+                hi = fmaxf(hi, fmaxf(xa, xb));
+            }
+            lo -= mg;
+            hi += mg;
+            const float d = fmaxf(fmaxf(ya - xyo.y, xyo.y - yb), 0.f);  // the disk around the projected centre
+            if (d <= r) {
+                const float h = sqrtf(r2 - d * d);
+                lo = fminf(lo, xyo.x - h);
+                hi = fmaxf(hi, xyo.x + h);
+            }
+        } else if (!(box.w < ya || box.y > yb)) {
+            lo = box.x;
+            hi = box.z;
+        }
+        // columns of four pixels: centres fx0 + 4c .. fx0 + 4c + 3
+        const float c0 = ceilf((lo - fx0 - 3.f) * 0.25f), c1 = floorf((hi - fx0) * 0.25f);
+        const int i0 = (int)fminf(fmaxf(c0, 0.f), (float)cols), i1 = (int)fminf(fmaxf(c1, -1.f), (float)(cols - 1));
+        if (i1 >= i0) mask |= band_bits((2u << i1) - (1u << i0), k, side);
+    }
+    return mask;
+}
+
+// Bit matrix transpose over the warp: lane r holds row r, returns column `lane`.
+__device__ __forceinline__ uint32_t transpose32(uint32_t x) {
+    const int lane = threadIdx.x & 31;
+    uint32_t m = 0x0000ffffu;
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1, m ^= m << j) {
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+        x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y & m) << j));
+    }
+    return x;
+}
+
+// Writes the lists of a warp's 32 slots (mask: the calling lane's slot over the groups) as one word per group,
+// words[group * n_words + word].
+__device__ __forceinline__ void store_group_words(uint32_t mask, uint32_t* words, int n_words, int word, int side) {
+    const int lane = threadIdx.x & 31;
+    if (side == 8) {
+        uint32_t w = 0;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            const uint32_t b = __ballot_sync(0xffffffffu, (mask >> g) & 1u);
+            if (lane == g) w = b;
+        }
+        if (lane < 8) words[lane * n_words + word] = w;
+    } else {
+        words[lane * n_words + word] = transpose32(mask);
+    }
+}
+
+// CTA side of a tile: 32x32 tiles are composited as four 16x16 squares (each its own work item).
+__host__ __device__ __forceinline__ int square_side(int tile_size) { return tile_size == 8 ? 8 : 16; }
+__host__ __device__ __forceinline__ int squares_per_tile(int tile_size) { return tile_size == 32 ? 4 : 1; }
+
 // Texture contribution to colour channel k (channels >= 4 have none).
 template <int NT>
 __device__ __forceinline__ float tex_color(const PairEvalT<NT>& e, int k) {

@@ -35,239 +35,250 @@ namespace tg {
 #ifndef TG_FWD_MIN_CTAS_ANISO
 #define TG_FWD_MIN_CTAS_ANISO TG_FWD_MIN_CTAS
 #endif
-template <int PPT, class Filt>
+template <class Filt>
 struct FwdBounds {
-    static constexpr int kMinCtas = PPT == 1 ? (Filt::kAniso ? TG_FWD_MIN_CTAS_ANISO : TG_FWD_MIN_CTAS) : 1;
+    static constexpr int kMinCtas = Filt::kAniso ? TG_FWD_MIN_CTAS_ANISO : TG_FWD_MIN_CTAS;
 };
 
-// One work item (tile) of the forward; every early return is uniform over the CTA.
-template <int D, class Tex, int PPT, class Filt = FiltBilinear>
+// Staged splats: four float4 records, the colour (four channels in a vector, a fifth apart), the texture scale
+// (FP8 only), the contribution statistics and the groups' list words.
+template <int D, class Tex>
+struct FwdSmem {
+    static constexpr bool kScale = Tex::kFormat == TG_TEX_FP8_E4M3;
+    float4 *m0, *m1, *m2, *nrm, *col;
+    float *col5, *scale;
+    uint32_t *csum, *ccnt, *words;
+    float4* extra;  // anisotropic_bilinear: the boundary integration's per-warp areas
+    __device__ __forceinline__ FwdSmem(float4* base, int bs, int side) {
+        m0 = base; m1 = m0 + bs; m2 = m1 + bs; nrm = m2 + bs; col = nrm + bs;
+        csum = reinterpret_cast<uint32_t*>(col + bs);
+        ccnt = csum + bs;
+        words = ccnt + bs;
+        scale = reinterpret_cast<float*>(words + (side * side / kGroupLanes) * (bs / 32));
+        col5 = scale + (kScale ? bs : 0);
+        extra = reinterpret_cast<float4*>(col5 + (D == 5 ? bs : 0));
+    }
+    static size_t bytes(int bs, int side) {
+        return (size_t)bs * (5 * sizeof(float4) + 8 + (kScale ? 4 : 0) + (D == 5 ? 4 : 0)) +
+               (size_t)(side * side / kGroupLanes) * (bs / 32) * 4;
+    }
+};
+
+// One work item (a tile, or a quarter of a 32x32 tile) of the forward; every early return is uniform over the CTA.
+template <int D, class Tex, class Filt = FiltBilinear>
 __device__ __forceinline__ void fwd_tile(const tg_raster_fwd_args& a, const int bs, const int64_t item) {
     constexpr bool kTextured = Tex::kFormat != TG_TEX_NONE;
+    constexpr unsigned kFull = 0xffffffffu;
     extern __shared__ float4 smem4[];
-    const int nt = blockDim.x;  // threads: tile_size^2 / PPT; bs = splats staged per batch
-    float4* s_box = smem4;  // per-splat cull box (see cull_box)
-    float4* s_xyo = s_box + bs;
-    float4* s_m0 = s_xyo + bs;
-    float4* s_m1 = s_m0 + bs;
-    float4* s_m2 = s_m1 + bs;
-    float4* s_nrm = s_m2 + bs;
-    float* s_col = reinterpret_cast<float*>(s_nrm + bs);
-    int* s_row = reinterpret_cast<int*>(s_col + bs * D);
-    // anisotropic_bilinear: the boundary integration's per-warp area (16-byte aligned: bs is a multiple of 32)
-    float4* s_aniso = Filt::kAniso ? reinterpret_cast<float4*>(s_row + bs) + (threadIdx.x >> 5) * kAnisoWarpF4
-                                   : nullptr;
+    const int nt = blockDim.x;  // one thread per pixel of the square; bs = splats staged per batch
+    const int ts = a.tile_size, side = square_side(ts), subs = squares_per_tile(ts);
+    const FwdSmem<D, Tex> S(smem4, bs, side);
+    float4* s_aniso = Filt::kAniso ? S.extra + (threadIdx.x >> 5) * kAnisoWarpF4 : nullptr;
 
-    const unsigned wmask = __activemask();
-    const TileWork tc = tile_work(a, item);
+    const TileWork tc = tile_work(a, subs == 1 ? item : item / subs);
     if (!tc.valid) return;  // uniform over the CTA
     const int tr = threadIdx.x, lane = tr & 31;
-    const int ts = a.tile_size;
-
-    int64_t pix[PPT];
-    bool inside[PPT], done[PPT];
-    float px[PPT], py[PPT];
-#pragma unroll
-    for (int q = 0; q < PPT; ++q) {
-        const int local = tr + q * nt;
-        const int i = tc.ty * ts + local / ts;
-        const int j = tc.tx * ts + local % ts;
-        pix[q] = pixel_index(tc, i, j);
-        inside[q] = pix[q] >= 0;
-        px[q] = (float)j + 0.5f;
-        py[q] = (float)i + 0.5f;
-        done[q] = !inside[q];
-    }
+    const int sub = subs == 1 ? 0 : (int)(item % subs);
+    const int X0 = tc.tx * ts + (sub & 1) * side, Y0 = tc.ty * ts + (sub >> 1) * side;
+    const PixelSlot ps = pixel_slot(tr, side);
+    const int j = X0 + ps.x, i = Y0 + ps.y;
+    const int64_t pix = pixel_index(tc, i, j);
+    const bool inside = pix >= 0;
+    const float px = (float)j + 0.5f, py = (float)i + 0.5f;
+    bool done = !inside;
 
     if (a.masks != nullptr && !a.masks[tc.t]) {
+        if (!inside) return;
 #pragma unroll
-        for (int q = 0; q < PPT; ++q) {
-            if (!inside[q]) continue;
-            const int64_t p = pix[q];
-#pragma unroll
-            for (int k = 0; k < D; ++k) a.out_colors[p * D + k] = a.backgrounds ? a.backgrounds[tc.c * D + k] : 0.f;
-            a.out_alphas[p] = 0.f;
-            a.out_normals[p * 3] = a.out_normals[p * 3 + 1] = a.out_normals[p * 3 + 2] = 0.f;
-            a.out_distort[p] = 0.f;
-            a.out_median[p] = 0.f;
-            a.last_ids[p] = 0;
-            a.median_ids[p] = 0;
-        }
+        for (int k = 0; k < D; ++k) a.out_colors[pix * D + k] = a.backgrounds ? a.backgrounds[tc.c * D + k] : 0.f;
+        a.out_alphas[pix] = 0.f;
+        a.out_normals[pix * 3] = a.out_normals[pix * 3 + 1] = a.out_normals[pix * 3 + 2] = 0.f;
+        a.out_distort[pix] = 0.f;
+        a.out_median[pix] = 0.f;
+        a.last_ids[pix] = 0;
+        a.median_ids[pix] = 0;
         return;
     }
 
-    // pixel-centre rectangle covered by this warp (for the warp-level cull)
-    float wx0 = INFINITY, wx1 = -INFINITY, wy0 = INFINITY, wy1 = -INFINITY;
-#pragma unroll
-    for (int q = 0; q < PPT; ++q) {
-        const int local = tr + q * nt;
-        const float cx = (float)(tc.tx * ts + local % ts) + 0.5f, cy = (float)(tc.ty * ts + local / ts) + 0.5f;
-        wx0 = fminf(wx0, cx); wx1 = fmaxf(wx1, cx); wy0 = fminf(wy0, cy); wy1 = fmaxf(wy1, cy);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        wx0 = fminf(wx0, __shfl_xor_sync(wmask, wx0, o)); wx1 = fmaxf(wx1, __shfl_xor_sync(wmask, wx1, o));
-        wy0 = fminf(wy0, __shfl_xor_sync(wmask, wy0, o)); wy1 = fmaxf(wy1, __shfl_xor_sync(wmask, wy1, o));
-    }
     const int32_t range_start = tc.range_start;
     const int32_t range_end = tc.range_end;
     const int num_batches = (range_end - range_start + bs - 1) / bs;
     const int64_t tex_stride = (int64_t)a.tex_ry * a.tex_rx;
     const int mip_clen = Filt::kMip ? ((1 << (2 * a.mip_levels)) - 1) / 3 : 0;
+    const int n_words = bs >> 5;
+    // the calling lane's list: its 4x2 group's, or (anisotropic_bilinear, which integrates one splat's footprints
+    // over the whole warp) the union of its warp's four
+    const uint32_t* words = S.words + (size_t)(Filt::kAniso ? (tr >> 5) * 4 : tr >> 3) * n_words;
+    auto list_word = [&](int w) -> uint32_t {
+        if constexpr (Filt::kAniso) return words[w] | words[w + n_words] | words[w + 2 * n_words] | words[w + 3 * n_words];
+        else return words[w];
+    };
 
-    float T[PPT], pix_out[PPT][D], nrm_out[PPT][3], distort[PPT], accum_vis_depth[PPT], median_depth[PPT];
-    int32_t cur_idx[PPT], median_idx[PPT];
+    float T = 1.f, pix_out[D], nrm_out[3] = {0.f, 0.f, 0.f}, distort = 0.f, accum_vis_depth = 0.f, median_depth = 0.f;
+    int32_t cur_idx = 0, median_idx = 0;
     // anisotropic_bilinear records: footprint integrals computed so far, and those up to the last contributor
-    int32_t rec_n[PPT], rec_last[PPT];
+    int32_t rec_n = 0, rec_last = 0;
     const bool records = Filt::kAniso && a.aniso_records != nullptr;
 #pragma unroll
-    for (int q = 0; q < PPT; ++q) {
-        T[q] = 1.f;
-#pragma unroll
-        for (int k = 0; k < D; ++k) pix_out[q][k] = 0.f;
-        nrm_out[q][0] = nrm_out[q][1] = nrm_out[q][2] = 0.f;
-        distort[q] = accum_vis_depth[q] = median_depth[q] = 0.f;
-        cur_idx[q] = median_idx[q] = 0;
-        rec_n[q] = rec_last[q] = 0;
-    }
+    for (int k = 0; k < D; ++k) pix_out[k] = 0.f;
+    for (int slot = tr; slot < bs; slot += nt) S.csum[slot] = S.ccnt[slot] = 0u;
+
+    // adds a staged slot's statistics to its Gaussian's (by the thread that stages the slot)
+    auto flush_stats = [&](int slot) {
+        const uint32_t c = S.ccnt[slot];
+        if (c == 0u) return;
+        const int row = __float_as_int(S.nrm[slot].w);
+        atomicAdd(a.contrib_sum + row, (float)S.csum[slot] * (1.f / 16777216.f));
+        atomicAdd(a.contrib_count + row, (float)c);
+        S.csum[slot] = S.ccnt[slot] = 0u;
+    };
 
     for (int b = 0; b < num_batches; ++b) {
-        bool all_done = true;
-#pragma unroll
-        for (int q = 0; q < PPT; ++q) all_done &= done[q];
-        if (__syncthreads_count(all_done) >= nt) break;
+        if (__syncthreads_count(done) >= nt) break;
         const int32_t batch_start = range_start + bs * b;
-        for (int slot = tr; slot < bs; slot += nt) {
+        for (int slot = tr; slot < bs; slot += nt) {  // (whole warps: bs and nt are multiples of 32)
+            flush_stats(slot);
             const int32_t idx = batch_start + slot;
+            uint32_t reach = 0u;
             if (idx < range_end) {
                 const int32_t g = a.flatten_ids[idx];
                 const float2 xy = reinterpret_cast<const float2*>(a.means2d)[g];
                 const int32_t row = a.gaussian_ids ? (int32_t)a.gaussian_ids[g] : g % a.N;
-                const float scale = (Tex::kFormat == TG_TEX_FP8_E4M3) ? a.tex_scales[row] : 1.f;
-                s_xyo[slot] = make_float4(xy.x, xy.y, a.opacities[g], scale);
+                const float op = a.opacities[g];
                 const float* m = a.ray_transforms + 9 * (int64_t)g;
-                s_m0[slot] = make_float4(m[0], m[1], m[2], 0.f);
-                s_m1[slot] = make_float4(m[3], m[4], m[5], 0.f);
-                s_m2[slot] = make_float4(m[6], m[7], m[8], 0.f);
-                s_box[slot] = cull_box(s_xyo[slot], s_m0[slot], s_m1[slot], s_m2[slot], kTextured, a.range_x, a.range_y,
-                                       a.g_weight, !Filt::kAniso);
+                const float4 m0 = make_float4(m[0], m[1], m[2], xy.x), m1 = make_float4(m[3], m[4], m[5], xy.y),
+                             m2 = make_float4(m[6], m[7], m[8], op);
+                S.m0[slot] = m0;
+                S.m1[slot] = m1;
+                S.m2[slot] = m2;
                 const float* n = a.normals + 3 * (int64_t)g;
-                s_nrm[slot] = make_float4(n[0], n[1], n[2], 0.f);
-#pragma unroll
-                for (int k = 0; k < D; ++k) s_col[slot * D + k] = a.colors[(int64_t)g * D + k];
-                s_row[slot] = row;
+                S.nrm[slot] = make_float4(n[0], n[1], n[2], __int_as_float(row));
+                const float* c = a.colors + (int64_t)g * D;
+                S.col[slot] = make_float4(c[0], D > 1 ? c[D > 1 ? 1 : 0] : 0.f, D > 2 ? c[D > 2 ? 2 : 0] : 0.f,
+                                          D > 3 ? c[D > 3 ? 3 : 0] : 0.f);
+                if constexpr (D == 5) S.col5[slot] = c[4];
+                if constexpr (FwdSmem<D, Tex>::kScale) S.scale[slot] = a.tex_scales[row];
+                reach = group_mask(make_float4(xy.x, xy.y, op, 1.f), m0, m1, m2, kTextured, a.range_x, a.range_y,
+                                   a.g_weight, !Filt::kAniso, X0, Y0, side);
             }
+            store_group_words(reach, S.words, n_words, slot >> 5, side);
         }
         __syncthreads();
-        const int batch_size = min(bs, range_end - batch_start);
-        for (int t = 0; t < batch_size; ++t) {
-            bool warp_done = true;
-#pragma unroll
-            for (int q = 0; q < PPT; ++q) warp_done &= done[q];
-            if (__all_sync(wmask, warp_done)) break;
-            const float4 box = s_box[t];
-            if (box.z < wx0 || box.x > wx1 || box.w < wy0 || box.y > wy1) continue;  // no pixel of this warp can be valid
-            const float4 xyo = s_xyo[t], m0 = s_m0[t], m1 = s_m1[t], m2 = s_m2[t];
-            const int row = s_row[t];
-            const int64_t tex_base = (int64_t)row * tex_stride;
-            float csum = 0.f;
-            int ccount = 0;
-#pragma unroll
-            for (int q = 0; q < PPT; ++q) {
-                const bool act = !done[q] && in_box(box, px[q], py[q]);
+        int w = 0;
+        uint32_t bits = list_word(0);
+        for (;;) {
+            const unsigned live = __ballot_sync(kFull, !done);
+            const bool group_live = Filt::kAniso ? live != 0u : ((live >> (lane & 24)) & 0xffu) != 0u;
+            if (!group_live) bits = 0u;
+            else
+                while (bits == 0u && w + 1 < n_words) bits = list_word(++w);
+            if (!__any_sync(kFull, bits != 0u)) break;
+            const bool act = bits != 0u && !done;
+            const int t = w * 32 + (bits != 0u ? __ffs(bits) - 1 : 0);
+            bits &= bits - 1u;
+            uint32_t stat = 0u;  // the pair's alpha in 2^-24 fixed point
+            if (Filt::kAniso || act) {
+                const float4 m0 = S.m0[t], m1 = S.m1[t], m2 = S.m2[t];
+                const float4 nn = S.nrm[t];
+                const int row = __float_as_int(nn.w);
+                const int64_t tex_base = (int64_t)row * tex_stride;
+                const float4 xyo = make_float4(m0.w, m1.w, m2.w, FwdSmem<D, Tex>::kScale ? S.scale[t] : 1.f);
                 PairOf<Filt> e;
                 if constexpr (Filt::kAniso) {  // every lane takes part: the warp integrates footprints together
-                    eval_aniso_coop<Tex>(e, act, px[q], py[q], xyo, m0, m1, m2, a.textures, tex_base, a.tex_rx,
-                                         a.tex_ry, a.range_x, a.range_y, a.g_weight, wmask,
+                    eval_aniso_coop<Tex>(e, act, px, py, xyo, m0, m1, m2, a.textures, tex_base, a.tex_rx, a.tex_ry,
+                                         a.range_x, a.range_y, a.g_weight, kFull,
                                          a.aniso_prefix ? reinterpret_cast<const float4*>(a.aniso_prefix) + tex_base
                                                         : nullptr,
                                          s_aniso);
-                    if (!act) continue;
-                    if (records && e.tex_valid) {  // every integral, in order, whether or not the pair is kept
-                        if (rec_n[q] < a.aniso_record_cap)
-                            reinterpret_cast<float4*>(a.aniso_records)[pix[q] * a.aniso_record_cap + rec_n[q]] =
-                                e.tsum;
-                        ++rec_n[q];
+                    if (act && records && e.tex_valid) {  // every integral, in order, whether or not the pair is kept
+                        if (rec_n < a.aniso_record_cap)
+                            reinterpret_cast<float4*>(a.aniso_records)[pix * a.aniso_record_cap + rec_n] = e.tsum;
+                        ++rec_n;
                     }
                 } else {
-                    if (!act) continue;
-                    eval_pair<Tex, Filt>(e, px[q], py[q], xyo, m0, m1, m2, a.textures, tex_base, a.tex_rx, a.tex_ry,
-                                         a.range_x, a.range_y, a.g_weight,
+                    eval_pair<Tex, Filt>(e, px, py, xyo, m0, m1, m2, a.textures, tex_base, a.tex_rx, a.tex_ry, a.range_x,
+                                         a.range_y, a.g_weight,
                                          MipSrc{a.tex_coarse, (int64_t)row * mip_clen, mip_clen, a.mip_levels});
                 }
-                if (!e.valid) continue;
-                const float next_T = T[q] * (1.f - e.alpha);
-                if (next_T <= 1e-4f) {
-                    done[q] = true;
-                    continue;
-                }
-                const float vis = e.alpha * T[q];
-                const float* cp = s_col + t * D;
+                if (act && e.valid) {
+                    const float next_T = T * (1.f - e.alpha);
+                    if (next_T <= 1e-4f) {
+                        done = true;
+                    } else {
+                        const float vis = e.alpha * T;
+                        const float4 c4 = S.col[t];
+                        const float c5 = D == 5 ? S.col5[t] : 0.f;
+                        float depth = 0.f;
 #pragma unroll
-                for (int k = 0; k < D; ++k) pix_out[q][k] += (cp[k] + (kTextured ? tex_color(e, k) : 0.f)) * vis;
-                const float4 nn = s_nrm[t];
-                nrm_out[q][0] += nn.x * vis;
-                nrm_out[q][1] += nn.y * vis;
-                nrm_out[q][2] += nn.z * vis;
-                const float depth = cp[D - 1];
-                distort[q] += 2.f * (vis * depth * (1.f - T[q]) - vis * accum_vis_depth[q]);
-                accum_vis_depth[q] += vis * depth;
-                if (T[q] > 0.5f) {
-                    median_depth[q] = depth;
-                    median_idx[q] = batch_start + t;
-                }
-                cur_idx[q] = batch_start + t;
-                rec_last[q] = rec_n[q];
-                T[q] = next_T;
-                if (e.alpha > a.contrib_threshold) {
-                    csum += e.alpha;
-                    ++ccount;
+                        for (int k = 0; k < D; ++k) {
+                            const float ck = k < 4 ? f4get(c4, k) : c5;
+                            pix_out[k] += (ck + (kTextured ? tex_color(e, k) : 0.f)) * vis;
+                            if (k == D - 1) depth = ck;
+                        }
+                        nrm_out[0] += nn.x * vis;
+                        nrm_out[1] += nn.y * vis;
+                        nrm_out[2] += nn.z * vis;
+                        distort += 2.f * (vis * depth * (1.f - T) - vis * accum_vis_depth);
+                        accum_vis_depth += vis * depth;
+                        if (T > 0.5f) {
+                            median_depth = depth;
+                            median_idx = batch_start + t;
+                        }
+                        cur_idx = batch_start + t;
+                        rec_last = rec_n;
+                        T = next_T;
+                        // counted in the top four bits: eight lanes' alphas (each < 1) fit below them
+                        if (e.alpha > a.contrib_threshold) stat = __float2uint_rn(e.alpha * 16777216.f) | (1u << 28);
+                    }
                 }
             }
-            if (__any_sync(wmask, ccount > 0)) {
-                // one-instruction warp sums: the alphas (each < 1, at most PPT per lane) in 2^-24 fixed point,
-                // so 32 lanes' sums fit in 32 bits; the quantisation is at the FP32 rounding level of the sum
-                const unsigned s = __reduce_add_sync(wmask, __float2uint_rn(csum * 16777216.f));
-                const unsigned c = __reduce_add_sync(wmask, (unsigned)ccount);
-                if (lane == __ffs(wmask) - 1) {
-                    atomicAdd(a.contrib_sum + row, (float)s * (1.f / 16777216.f));
-                    atomicAdd(a.contrib_count + row, (float)c);
+            // the group's sum of alphas and count, into the slot's integer statistics (32-bit integer adds to shared
+            // memory are single instructions; a square's 256 alphas below 0.999 fit in 32 bits)
+            if constexpr (Filt::kAniso) {
+                const uint32_t s = __reduce_add_sync(kFull, stat & 0x0fffffffu), c = __reduce_add_sync(kFull, stat >> 28);
+                if (lane == 0 && c != 0u) {
+                    atomicAdd(S.csum + t, s);
+                    atomicAdd(S.ccnt + t, c);
+                }
+            } else {
+                stat += __shfl_xor_sync(kFull, stat, 4);
+                stat += __shfl_xor_sync(kFull, stat, 2);
+                stat += __shfl_xor_sync(kFull, stat, 1);
+                if ((lane & 7) == 0 && stat != 0u) {
+                    atomicAdd(S.csum + t, stat & 0x0fffffffu);
+                    atomicAdd(S.ccnt + t, stat >> 28);
                 }
             }
         }
-        if (a.t_checkpoints != nullptr) {  // every pixel's transmittance at the end of this batch
-            float* ck = a.t_checkpoints + ((int64_t)tc.t + range_start / bs + b) * (int64_t)(nt * PPT);
-#pragma unroll
-            for (int q = 0; q < PPT; ++q) ck[tr + q * nt] = T[q];
-        }
+        if (a.t_checkpoints != nullptr)  // every pixel's transmittance at the end of this batch
+            a.t_checkpoints[((int64_t)tc.t + range_start / bs + b) * (int64_t)(ts * ts) +
+                            (i - tc.ty * ts) * ts + (j - tc.tx * ts)] = T;
     }
+    __syncthreads();
+    for (int slot = tr; slot < bs; slot += nt) flush_stats(slot);
+    if (!inside) return;
+    a.out_alphas[pix] = 1.f - T;
 #pragma unroll
-    for (int q = 0; q < PPT; ++q) {
-        if (!inside[q]) continue;
-        const int64_t p = pix[q];
-        a.out_alphas[p] = 1.f - T[q];
-#pragma unroll
-        for (int k = 0; k < D; ++k)
-            a.out_colors[p * D + k] = a.backgrounds ? pix_out[q][k] + T[q] * a.backgrounds[tc.c * D + k] : pix_out[q][k];
-        a.out_normals[p * 3] = nrm_out[q][0];
-        a.out_normals[p * 3 + 1] = nrm_out[q][1];
-        a.out_normals[p * 3 + 2] = nrm_out[q][2];
-        a.last_ids[p] = cur_idx[q];
-        a.out_distort[p] = distort[q];
-        a.out_median[p] = median_depth[q];
-        a.median_ids[p] = median_idx[q];
-        if (records) a.aniso_record_count[p] = rec_last[q];
-    }
+    for (int k = 0; k < D; ++k)
+        a.out_colors[pix * D + k] = a.backgrounds ? pix_out[k] + T * a.backgrounds[tc.c * D + k] : pix_out[k];
+    a.out_normals[pix * 3] = nrm_out[0];
+    a.out_normals[pix * 3 + 1] = nrm_out[1];
+    a.out_normals[pix * 3 + 2] = nrm_out[2];
+    a.last_ids[pix] = cur_idx;
+    a.out_distort[pix] = distort;
+    a.out_median[pix] = median_depth;
+    a.median_ids[pix] = median_idx;
+    if (records) a.aniso_record_count[pix] = rec_last;
 }
 
 // CTA per work item, or (work_queue != NULL) a persistent grid whose CTAs take
 // items from the queue counter until none is left.
-template <int D, class Tex, int PPT, bool kPersistent, class Filt = FiltBilinear>
-__global__ void __launch_bounds__(256, FwdBounds<PPT, Filt>::kMinCtas) raster_fwd_kernel(const tg_raster_fwd_args a,
-                                                                                   const int bs,
-                                                                                   const int64_t n_items) {
+template <int D, class Tex, bool kPersistent, class Filt = FiltBilinear>
+__global__ void __launch_bounds__(256, FwdBounds<Filt>::kMinCtas) raster_fwd_kernel(const tg_raster_fwd_args a,
+                                                                                    const int bs,
+                                                                                    const int64_t n_items) {
     if constexpr (!kPersistent) {
-        fwd_tile<D, Tex, PPT, Filt>(a, bs, blockIdx.x);
+        fwd_tile<D, Tex, Filt>(a, bs, blockIdx.x);
         return;
     }
     else {
@@ -278,62 +289,43 @@ __global__ void __launch_bounds__(256, FwdBounds<PPT, Filt>::kMinCtas) raster_fw
             const int64_t item = s_item;
             __syncthreads();  // s_item read by all before it is rewritten
             if (item >= n_items) return;
-            fwd_tile<D, Tex, PPT, Filt>(a, bs, item);
+            fwd_tile<D, Tex, Filt>(a, bs, item);
         }
     }
 }
 
-size_t fwd_smem_bytes(int D, int bs) { return (size_t)bs * (6 * sizeof(float4) + D * sizeof(float) + sizeof(int)); }
-
-// mipmapped2 / anisotropic_bilinear filters: one pixel per thread (8x8 / 16x16 tiles), one CTA per tile
-template <int D, class Tex, class Filt>
-cudaError_t launch_fwd_filter(const tg_raster_fwd_args& a, cudaStream_t s) {
-    const int tile_px = a.tile_size * a.tile_size;
-    const int bs = a.batch_depth > 0 ? a.batch_depth : tile_px;
-    const size_t smem = fwd_smem_bytes(D, bs) + (Filt::kAniso ? (size_t)(tile_px / 32) * kAnisoWarpF4 * 16 : 0);
-    const int64_t blocks = a.views ? a.n_tiles : (int64_t)a.C * a.tile_width * a.tile_height;
-    if (blocks == 0) return cudaSuccess;
-    cudaError_t err = cudaFuncSetAttribute(raster_fwd_kernel<D, Tex, 1, false, Filt>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <int D, class Tex, bool kPersistent, class Filt>
+cudaError_t launch_fwd_kernel(const tg_raster_fwd_args& a, cudaStream_t s) {
+    const int side = square_side(a.tile_size), threads = side * side;
+    const int bs = a.batch_depth > 0 ? a.batch_depth : a.tile_size * a.tile_size;
+    const size_t smem = FwdSmem<D, Tex>::bytes(bs, side) + (Filt::kAniso ? (size_t)(threads / 32) * kAnisoWarpF4 * 16 : 0);
+    const int64_t tiles = a.views ? a.n_tiles : (int64_t)a.C * a.tile_width * a.tile_height;
+    const int64_t items = tiles * squares_per_tile(a.tile_size);
+    if (items == 0) return cudaSuccess;
+    if (items > 0x7fffffff) return cudaErrorInvalidValue;
+    const auto fn = raster_fwd_kernel<D, Tex, kPersistent, Filt>;
+    cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
-    raster_fwd_kernel<D, Tex, 1, false, Filt><<<(unsigned)blocks, tile_px, smem, s>>>(a, bs, blocks);
+    int64_t grid = items;
+    if (kPersistent) {
+        if ((err = cudaMemsetAsync(a.work_queue, 0, sizeof(uint32_t), s)) != cudaSuccess) return err;
+        if ((err = persistent_grid((const void*)fn, threads, smem, items, grid)) != cudaSuccess) return err;
+    }
+    fn<<<(unsigned)grid, threads, smem, s>>>(a, bs, items);
     note_launches(1);
     return cudaGetLastError();
 }
 
 template <int D, class Tex>
 cudaError_t launch_fwd_t(const tg_raster_fwd_args& a, cudaStream_t s) {
+    // mipmapped2 / anisotropic_bilinear filters: FP32 / BF16 storage, 3 or 4 channels, 8x8 / 16x16 tiles, one CTA per tile
     if constexpr ((D == 3 || D == 4) && (Tex::kFormat == TG_TEX_F32 || Tex::kFormat == TG_TEX_BF16)) {
-        if (a.mip_levels > 0) return launch_fwd_filter<D, Tex, FiltMip2>(a, s);
-        if (a.filter == TG_FILTER_ANISO_BILINEAR) return launch_fwd_filter<D, Tex, FiltAniso>(a, s);
+        if (a.mip_levels > 0) return launch_fwd_kernel<D, Tex, false, FiltMip2>(a, s);
+        if (a.filter == TG_FILTER_ANISO_BILINEAR) return launch_fwd_kernel<D, Tex, false, FiltAniso>(a, s);
     }
     if (a.mip_levels > 0 || a.filter != TG_FILTER_BILINEAR) return cudaErrorInvalidValue;
-    const int tile_px = a.tile_size * a.tile_size;
-    const int bs = a.batch_depth > 0 ? a.batch_depth : tile_px;
-    const size_t smem = fwd_smem_bytes(D, bs);
-    const int64_t blocks = a.views ? a.n_tiles : (int64_t)a.C * a.tile_width * a.tile_height;
-    if (blocks == 0) return cudaSuccess;
-    const bool four = tile_px > 256;  // 32x32 tiles: four pixels per thread, 256 threads
-    const bool pers = a.work_queue != nullptr;
-    const void* fn = four ? (pers ? (const void*)raster_fwd_kernel<D, Tex, 4, true>
-                                  : (const void*)raster_fwd_kernel<D, Tex, 4, false>)
-                          : (pers ? (const void*)raster_fwd_kernel<D, Tex, 1, true>
-                                  : (const void*)raster_fwd_kernel<D, Tex, 1, false>);
-    const int threads = four ? tile_px / 4 : tile_px;
-    cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return err;
-    int64_t grid = blocks;
-    if (pers) {
-        if ((err = cudaMemsetAsync(a.work_queue, 0, sizeof(uint32_t), s)) != cudaSuccess) return err;
-        if ((err = persistent_grid(fn, threads, smem, blocks, grid)) != cudaSuccess) return err;
-    }
-    const dim3 g((unsigned)grid), b((unsigned)threads);
-    if (four && pers) raster_fwd_kernel<D, Tex, 4, true><<<g, b, smem, s>>>(a, bs, blocks);
-    else if (four) raster_fwd_kernel<D, Tex, 4, false><<<g, b, smem, s>>>(a, bs, blocks);
-    else if (pers) raster_fwd_kernel<D, Tex, 1, true><<<g, b, smem, s>>>(a, bs, blocks);
-    else raster_fwd_kernel<D, Tex, 1, false><<<g, b, smem, s>>>(a, bs, blocks);
-    note_launches(1);
-    return cudaGetLastError();
+    return a.work_queue != nullptr ? launch_fwd_kernel<D, Tex, true, FiltBilinear>(a, s)
+                                   : launch_fwd_kernel<D, Tex, false, FiltBilinear>(a, s);
 }
 
 template <class Tex>
