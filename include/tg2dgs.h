@@ -427,17 +427,23 @@ typedef struct {
      * instead of cell by cell as the reference does; the same integral up to
      * FP32 rounding.  No counterpart in the reference. */
     const float* aniso_prefix;
-    /* With aniso_prefix: records of the footprint integrals the forward
-     * computes, per pixel in the order it computes them: aniso_records
-     * [n_pixels, aniso_record_cap, 4] FP32 (the first aniso_record_cap of
-     * each pixel's) and aniso_record_count [n_pixels] int32 (how many of them
-     * the pixel had up to its last contributor).  Given the same pointers the
-     * adjoint reads these integrals instead of integrating the footprints
-     * again (those past the capacity it integrates again).  NULL / 0: none.
-     * No counterpart in the reference. */
+    /* With aniso_prefix: records of the footprint integrals of each pixel's
+     * contributors, in order: aniso_records [n_pixels, aniso_record_cap, 4]
+     * FP32 (the first aniso_record_cap of each pixel's) and aniso_record_count
+     * [n_pixels] int32 (how many contributors the pixel has).  Given the same
+     * pointers and contrib_masks the adjoint reads these integrals instead of
+     * integrating the footprints again (those past the capacity it integrates
+     * again).  NULL / 0: none.  No counterpart in the reference. */
     float* aniso_records;
     int32_t* aniso_record_count;
     int32_t aniso_record_cap;
+    /* One bit per (pixel, listed splat), written by the forward where the pair
+     * was composited; given the same pointer the adjoint visits only those
+     * pairs.  [n_tiles + n_isects / 32 + 1, tile_size^2] uint32 (integer
+     * division): row t + tile_offsets[t] / 32 + k holds the pixels' bits for
+     * splats 32 k .. 32 k + 31 of tile t's list.  NULL: none (the adjoint then
+     * tests every pair again).  No counterpart in the reference. */
+    uint32_t* contrib_masks;
 } tg_raster_fwd_args;
 TG_API int tg_rasterize_fwd(const tg_raster_fwd_args* a, tg_stream_t stream);
 
@@ -473,6 +479,11 @@ typedef struct {
      * [G,ry,rx,4] FP32 scratch for the gradient of the row-prefix table; the
      * call zeroes it and folds it into v_textures after the accumulation. */
     float* v_aniso_prefix;
+    /* Scratch [E,24] FP32, 16-byte aligned, or NULL: the entries' gradients are
+     * then accumulated in contiguous rows of it and written to the arrays
+     * above by one pass, instead of one add per value and array.  With it any
+     * of the upstream gradients v_render_* may be NULL, meaning zero. */
+    float* v_packed;
 } tg_raster_bwd_args;
 TG_API int tg_rasterize_bwd(const tg_raster_bwd_args* a, tg_stream_t stream);
 

@@ -82,7 +82,8 @@ class RasterFwdArgs(ctypes.Structure):
                 ("views", P), ("tile_view", P), ("n_tiles", I64), ("n_pixels", I64), ("n_isects_dev", P),
                 ("batch_depth", I32), ("work_queue", P), ("mip_levels", I32), ("tex_coarse", P),
                 ("filter", I32), ("t_checkpoints", P), ("aniso_prefix", P),
-                ("aniso_records", P), ("aniso_record_count", P), ("aniso_record_cap", I32)]
+                ("aniso_records", P), ("aniso_record_count", P), ("aniso_record_cap", I32),
+                ("contrib_masks", P)]
 
 
 class RasterBwdArgs(ctypes.Structure):
@@ -91,7 +92,7 @@ class RasterBwdArgs(ctypes.Structure):
                 ("v_render_distort", P), ("v_render_median", P), ("adjoint", I32), ("n_elems", I64),
                 ("v_means2d", P), ("v_means2d_abs", P), ("v_ray_transforms", P), ("v_colors", P),
                 ("v_opacities", P), ("v_normals", P), ("v_textures", P), ("v_densify", P), ("v_tex_coarse", P),
-                ("v_aniso_prefix", P)]
+                ("v_aniso_prefix", P), ("v_packed", P)]
 
 
 _lib = None

@@ -35,6 +35,7 @@ cudaError_t launch_offset_encode_views(const int64_t* keys, int64_t n, int C, in
                                        cudaStream_t s);
 cudaError_t launch_raster_fwd(const tg_raster_fwd_args& a, cudaStream_t s);
 cudaError_t launch_raster_bwd(const tg_raster_bwd_args& a, cudaStream_t s);
+int bwd_slots(const tg_raster_bwd_args& a);
 cudaError_t launch_sh_fwd(int64_t n, int64_t rows, int degree, int K, const float* dirs, const float* coeffs,
                           const uint8_t* masks, float* colors, cudaStream_t s);
 cudaError_t launch_sh_bwd(int64_t n, int64_t rows, int degree, int K, const float* dirs, const float* coeffs,
@@ -439,9 +440,12 @@ int tg_rasterize_bwd(const tg_raster_bwd_args* a, tg_stream_t stream) {
         TG_REQUIRE(a->v_tex_coarse && aligned(a->v_tex_coarse, 16), TG_ERR_INVALID_ARG,
                    "mipmapped2 texture gradients need v_tex_coarse");
     TG_REQUIRE(a->n_elems >= 0, TG_ERR_INVALID_ARG, "negative n_elems");
-    TG_REQUIRE(a->render_colors && a->render_alphas && a->last_ids && a->median_ids && a->v_render_colors &&
-                   a->v_render_alphas && a->v_render_normals && a->v_render_distort && a->v_render_median,
+    TG_REQUIRE(a->render_colors && a->render_alphas && a->last_ids && a->median_ids &&
+                   (a->v_packed || (a->v_render_colors && a->v_render_alphas && a->v_render_normals &&
+                                    a->v_render_distort && a->v_render_median)),
                TG_ERR_INVALID_ARG, "null forward output or upstream gradient");
+    TG_REQUIRE(a->v_packed == nullptr || (aligned(a->v_packed, 16) && aligned(a->v_densify, 8)), TG_ERR_INVALID_ARG,
+               "v_packed must be 16-byte and v_densify 8-byte aligned");
     TG_REQUIRE(a->v_means2d && a->v_ray_transforms && a->v_colors && a->v_opacities && a->v_normals && a->v_densify,
                TG_ERR_INVALID_ARG, "null gradient output");
     if (a->v_textures) TG_REQUIRE(aligned(a->v_textures, 16), TG_ERR_INVALID_ARG, "v_textures must be 16-byte aligned");
@@ -456,11 +460,14 @@ int tg_rasterize_bwd(const tg_raster_bwd_args* a, tg_stream_t stream) {
     const size_t tex_bytes = a->f.tex_format == TG_TEX_NONE || a->v_textures == nullptr
                                  ? 0
                                  : sizeof(float) * 4 * (size_t)a->f.tex_ry * a->f.tex_rx * (size_t)a->f.n_contrib;
+    // with the packed rows the per-entry arrays are written whole from them
+    const size_t F = a->v_packed ? 0 : sizeof(float);
     struct Z { void* p; size_t n; } zs[] = {
-        {a->v_means2d, sizeof(float) * 2 * E}, {a->v_ray_transforms, sizeof(float) * 9 * E},
-        {a->v_colors, sizeof(float) * D * E},  {a->v_opacities, sizeof(float) * E},
-        {a->v_normals, sizeof(float) * 3 * E}, {a->v_means2d_abs, a->v_means2d_abs ? sizeof(float) * 2 * E : 0},
-        {a->v_textures, tex_bytes},            {a->v_densify, sizeof(float) * 2 * E},
+        {a->v_packed, a->v_packed ? sizeof(float) * (size_t)tg::bwd_slots(*a) * E : 0},
+        {a->v_means2d, F * 2 * E}, {a->v_ray_transforms, F * 9 * E},
+        {a->v_colors, F * D * E},  {a->v_opacities, F * E},
+        {a->v_normals, F * 3 * E}, {a->v_means2d_abs, a->v_means2d_abs ? F * 2 * E : 0},
+        {a->v_textures, tex_bytes}, {a->v_densify, F * 2 * E},
         {a->v_tex_coarse, a->f.mip_levels > 0 && a->v_textures
                               ? sizeof(float) * 4 * (size_t)(((int64_t(1) << (2 * a->f.mip_levels)) - 1) / 3) *
                                     (size_t)a->f.n_contrib

@@ -1,23 +1,25 @@
 // Textured / plain 2DGS compositor, adjoint, for sm_100a.
 //
-// One CTA per (camera, tile) work item, one thread per pixel (four for 32x32
-// tiles), back-to-front in batches of `batch_depth` staged splats over the
-// splats that can still matter to the tile (batches beyond every pixel's last
-// contributor are skipped).  Transmittance is recovered from the stored final
-// T and last-contributor index by division, as the reference does
-// (rasterize_to_pixels_textured_gaussians_2dgs_bwd.cu:160, :456-457); nothing
-// per splat is stored by the forward.
+// One CTA per (camera, tile) work item (a quarter of a 32x32 tile), one thread per pixel, back-to-front in batches
+// of `batch_depth` staged splats.  Transmittance is recovered from the stored final T by division, as the
+// reference does (rasterize_to_pixels_textured_gaussians_2dgs_bwd.cu:160, :456-457).
 //
-// Reductions, B200-first:
-//  * per-splat gradients (colour, normal, ray transform, means2d, opacity,
-//    |means2d|) are reduced across the warp by a reduce-scatter butterfly --
-//    31 shuffles leave lane k holding the warp total of value k -- instead of
-//    one 5-level shuffle tree per value; lanes then add into a per-batch
-//    shared-memory accumulator, and the CTA flushes each splat's values with
-//    one global atomic per value (8x fewer global atomics than per-warp);
+// What is evaluated: the forward leaves one bit per (pixel, listed splat), set where the pair was composited
+// (tg_raster_fwd_args.contrib_masks), and the adjoint visits exactly those pairs.  As in the forward each 4x2 pixel
+// group walks its own list -- the union of its eight pixels' bits -- so the four groups of a warp work on four
+// splats at once: 0.34 warp evaluations per listed splat on the 1M-splat mixture, against 1.13 with a warp per
+// 8x4 block and its box test.  Without the bits (NULL) the groups' lists come from group_mask again and every
+// pair is tested.
+//
+// Reductions:
+//  * per-splat gradients (colour, ray transform, means2d, opacity; with an upstream gradient for normals, distortion
+//    or median depth, or |means2d| asked for, also those) are summed over a group's eight lanes by a reduce-scatter
+//    (14 shuffles for 16 values, 21 for 24) that leaves consecutive values in consecutive lanes, which add them to
+//    the entry's row of a packed [E, slots] buffer -- 64 contiguous bytes, two per lane.  A splat meets 1.1 groups
+//    per tile that lists it, so collecting a tile's sums in shared memory first would not save adds; the rows are
+//    spread to the separate gradient arrays by one pass over the entries afterwards;
 //  * per-texel gradients are RGBA float4 vector atomics, one per bilinear tap
-//    (4 per pixel-splat pair instead of the reference's up to 4*(D+1) scalar
-//    atomics).
+//    (4 per pixel-splat pair instead of the reference's up to 4*(D+1) scalar atomics).
 //
 // Adjoint forms: TG_ADJ_REFERENCE follows ..._bwd.cu:438-627; TG_ADJ_BWD2 adds
 // the reference's texture-UV term (..._bwd2.cu:612-676, du/ds = (R-1)/range);
@@ -26,133 +28,109 @@
 
 namespace tg {
 
-// reduce-scatter: on return vals[0] of lane l holds the warp sum of value l.
-__device__ __forceinline__ void warp_reduce_scatter32(float (&vals)[32], unsigned mask) {
+// Slots of an entry's row of gradient sums.  kGeo: with the upstream gradients of normals, distortion and median
+// depth, and |means2d|.
+template <int D, bool kGeo>
+struct GradSlots {
+    static constexpr int kRgb = 0;
+    static constexpr int kM = D;
+    static constexpr int kXY = D + 9;
+    static constexpr int kOpac = D + 11;
+    static constexpr int kNrm = D + 12;
+    static constexpr int kAbs = D + 15;
+    static constexpr int kUsed = kGeo ? D + 17 : D + 12;
+    static constexpr int kCount = kUsed <= 16 ? 16 : 24;
+};
+
+// Sum over each 8 lanes of every value; lane l keeps the NS / 8 sums from slot_base<NS>(l) on, in v[0 ..].
+template <int NS>
+__device__ __forceinline__ void reduce_scatter8(float (&v)[NS]) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) {
+    for (int s = 4, n = NS / 2; s >= 1; s >>= 1, n >>= 1) {
         const bool upper = (lane & s) != 0;
-        const bool have = ((mask >> (lane ^ s)) & 1u) != 0;
 #pragma unroll
-        for (int i = 0; i < s; ++i) {
-            const float send = upper ? vals[i] : vals[i + s];
-            const float keep = upper ? vals[i + s] : vals[i];
-            const float recv = __shfl_xor_sync(mask, send, s);
-            vals[i] = keep + (have ? recv : 0.f);
+        for (int i = 0; i < n; ++i) {
+            const float send = upper ? v[i] : v[i + n];
+            const float keep = upper ? v[i + n] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, s);
         }
     }
 }
+template <int NS>
+__device__ __forceinline__ int slot_base(int lane) {
+    return ((lane & 4) ? NS / 2 : 0) + ((lane & 2) ? NS / 4 : 0) + ((lane & 1) ? NS / 8 : 0);
+}
 
-template <int D>
-struct GradSlots {
-    static constexpr int kRgb = 0;
-    static constexpr int kNrm = D;
-    static constexpr int kM = D + 3;
-    static constexpr int kXY = D + 12;
-    static constexpr int kOpac = D + 14;
-    static constexpr int kAbs = D + 15;
-    static constexpr int kCount = D + 17;
-};
-
-// Resident CTAs per SM the register allocation targets.
+// Resident CTAs of 256 threads per SM the register allocation targets.
 #ifndef TG_BWD_MIN_CTAS
-#define TG_BWD_MIN_CTAS 2
+#define TG_BWD_MIN_CTAS 3
 #endif
-// Register budget: TG_BWD_MIN_CTAS resident CTAs for one pixel per thread,
-// one CTA of 256 threads for the four-pixel (32x32 tile) form.  The
-// anisotropic_bilinear adjoint targets 3 CTAs (80 registers allocated): with its clips
+// The anisotropic_bilinear adjoint targets 3 CTAs (80 registers allocated): with its clips
 // branch-free and its cell boundary sum out of line it spills ~1 KB there but
 // runs 3.9 % faster than at 128, which was already 28 % faster than the
 // unconstrained 245; 64 registers lose 17 % (1M splats, 4 views, measured).
 #ifndef TG_BWD_MIN_CTAS_ANISO
 #define TG_BWD_MIN_CTAS_ANISO 3
 #endif
-template <int PPT, class Filt>
+template <class Filt, bool kGeo>
 struct BwdBounds {
-    static constexpr int kMinCtas = PPT == 1 ? (Filt::kAniso ? TG_BWD_MIN_CTAS_ANISO : TG_BWD_MIN_CTAS) : 1;
+    static constexpr int kMinCtas = Filt::kAniso ? TG_BWD_MIN_CTAS_ANISO : (kGeo || Filt::kUV) ? 2 : TG_BWD_MIN_CTAS;
 };
 
-// Per-pixel state of the back-to-front sweep.
-template <int D>
+// Per-pixel state of the back-to-front sweep.  Everything behind the current splat enters its alpha's gradient
+// through one number: rest = T_final (v_alpha - v_c . background) - sum over the splats behind of
+// weight * (their colour . v_c + normal . v_n + distortion term).
+template <int D, bool kGeo>
 struct PixelAdj {
-    int64_t pix;
     float px, py;
-    bool inside;
-    float T_final, T, v_a, v_dist, v_med, bg_dot;
-    float v_c[D], buf[D];
-    float v_n[3], buf_n[3];
-    int32_t bin_final, median_idx;
-    float acc_d_buf, acc_d, acc_w_buf, acc_w, dist_buf;
-    int32_t local;     // pixel index within the tile
-    int32_t ck_batch;  // forward batch whose end transmittance T was last restarted from (-1: none)
-    int32_t rec;       // anisotropic_bilinear: the forward's record of the next footprint integral (counting down)
-};
-
-// The forward's transmittance checkpoints of one tile (tg_raster_fwd_args.t_checkpoints): base is the tile's
-// first row, rows of `stride` pixels, forward batches of bs splats from range_start rs.  base NULL: none.
-struct TileCkpt {
-    const float* base;
-    int64_t stride;
-    int32_t rs, bs;
+    float T, rest, v_c[D];
+    int32_t ck_batch;  // batch whose end transmittance T was last restarted from (-1: none)
+    // kGeo only
+    float v_n[3], v_dist, v_med, acc_d_buf, acc_d, acc_w_buf, acc_w;
+    int32_t median_idx;
 };
 
 // Adds one (pixel, splat) pair's gradient contributions to the lane's per-splat
-// sums `vals` (slots of GradSlots<D>), issues the pair's texel-gradient atomics,
+// sums `vals` (slots of GradSlots), issues the pair's texel-gradient atomics,
 // and advances the pixel's back-to-front state.  Follows
 // rasterize_to_pixels_textured_gaussians_2dgs_bwd.cu:438-627 (+ bwd2.cu:612-676).
-template <int D, class Tex, class Filt = FiltBilinear>
+template <int D, class Tex, class Filt, bool kGeo, int NS>
 __device__ __forceinline__ void accumulate_pair(const tg_raster_bwd_args& a, const PairOf<Filt>& e,
-                                                PixelAdj<D>& P, const float4 xyo, const float4 nn, const float* cp,
-                                                int32_t idx, float* vt, float uv_scale, float (&vals)[32],
-                                                const TileCkpt& ck, float* vct = nullptr, int mip_clen = 0,
+                                                PixelAdj<D, kGeo>& P, const float opac, const float4 nn,
+                                                const float (&cp)[D], int32_t idx, float* vt, float uv_scale,
+                                                float (&vals)[NS], float* vct = nullptr, int mip_clen = 0,
                                                 float4* aniso_g = nullptr) {
     // aniso_g (anisotropic_bilinear): receives the texel-gradient factor of the pair (divided by the area), which
     // the warp scatters over the footprint together
     constexpr bool kTextured = Tex::kFormat != TG_TEX_NONE;
-    using GS = GradSlots<D>;
+    using GS = GradSlots<D, kGeo>;
     const tg_raster_fwd_args& f = a.f;
-    const float opac = xyo.z;
-    if (idx == P.median_idx) vals[GS::kRgb + D - 1] += P.v_med;
-    if (ck.base != nullptr) {
-        // first pair of a new forward batch (back to front): T restarts from the forward's exact value at the
-        // batch's end -- no splat after this one in the batch contributed to this pixel, or it would have
-        // been met first
-        const int32_t fb = (idx - ck.rs) / ck.bs;
-        if (fb != P.ck_batch) {
-            P.ck_batch = fb;
-            P.T = ck.base[(int64_t)fb * ck.stride + P.local];
-        }
-    }
     const float ra = 1.f / (1.f - e.alpha);
     P.T *= ra;
     const float T = P.T;
     const float fac = e.alpha * T;
-    float texc[D];
+    float q = 0.f;  // d L / d weight of this splat
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-        vals[GS::kRgb + k] += fac * P.v_c[k];
-        texc[k] = kTextured ? tex_color_adj(e, k) : 0.f;
+        vals[GS::kRgb + k] = fac * P.v_c[k];
+        q += ((kTextured ? tex_color_adj(e, k) : 0.f) + cp[k]) * P.v_c[k];
     }
-    float v_alpha = 0.f;
-#pragma unroll
-    for (int k = 0; k < D; ++k) v_alpha += ((texc[k] + cp[k]) * T - P.buf[k] * ra) * P.v_c[k];
-    vals[GS::kNrm + 0] += fac * P.v_n[0];
-    vals[GS::kNrm + 1] += fac * P.v_n[1];
-    vals[GS::kNrm + 2] += fac * P.v_n[2];
-    v_alpha += (nn.x * T - P.buf_n[0] * ra) * P.v_n[0];
-    v_alpha += (nn.y * T - P.buf_n[1] * ra) * P.v_n[1];
-    v_alpha += (nn.z * T - P.buf_n[2] * ra) * P.v_n[2];
-    v_alpha += P.T_final * ra * P.v_a;
-    if (f.backgrounds) v_alpha += -P.T_final * ra * P.bg_dot;
-    {
+    if constexpr (kGeo) {
+        if (idx == P.median_idx) vals[GS::kRgb + D - 1] += P.v_med;
+        vals[GS::kNrm + 0] = fac * P.v_n[0];
+        vals[GS::kNrm + 1] = fac * P.v_n[1];
+        vals[GS::kNrm + 2] = fac * P.v_n[2];
+        q += nn.x * P.v_n[0] + nn.y * P.v_n[1] + nn.z * P.v_n[2];
         const float depth = cp[D - 1];
         const float dl_dw = 2.f * (2.f * (depth * P.acc_w_buf - P.acc_d_buf) + (P.acc_d - depth * P.acc_w));
-        v_alpha += (dl_dw * T - P.dist_buf * ra) * P.v_dist;
+        q += dl_dw * P.v_dist;
         P.acc_d_buf -= fac * depth;
         P.acc_w_buf -= fac;
-        P.dist_buf += dl_dw * fac;
         vals[GS::kRgb + D - 1] += 2.f * fac * (2.f - 2.f * T - P.acc_w + fac) * P.v_dist;
     }
+    const float v_alpha = q * T + P.rest * ra;
+    P.rest -= fac * q;
     // d L / d s, from the Gaussian kernel (3D branch) and, for the UV-aware adjoints, from the
     // texture lookup; both go back through s = zeta.xy / zeta.z and zeta = h_u x h_v once
     float vsx = 0.f, vsy = 0.f;
@@ -167,12 +145,14 @@ __device__ __forceinline__ void accumulate_pair(const tg_raster_bwd_args& a, con
         } else {
             const float vx = v_G * (dG * kFilterInvSquare * e.dx);
             const float vy = v_G * (dG * kFilterInvSquare * e.dy);
-            vals[GS::kXY] += vx;
-            vals[GS::kXY + 1] += vy;
-            vals[GS::kAbs] += fabsf(vx);
-            vals[GS::kAbs + 1] += fabsf(vy);
+            vals[GS::kXY] = vx;
+            vals[GS::kXY + 1] = vy;
+            if constexpr (kGeo) {
+                vals[GS::kAbs] = fabsf(vx);
+                vals[GS::kAbs + 1] = fabsf(vy);
+            }
         }
-        vals[GS::kOpac] += kTextured ? e.vis * v_alpha * e.asf : e.vis * v_alpha;
+        vals[GS::kOpac] = kTextured ? e.vis * v_alpha * e.asf : e.vis * v_alpha;
         tex_a_grad = e.vis * opac * v_alpha;
     }
     if constexpr (Filt::kAniso) {
@@ -232,248 +212,306 @@ __device__ __forceinline__ void accumulate_pair(const tg_raster_bwd_args& a, con
         const float a_ = vsx * iz, b_ = vsy * iz;
         const f3 vz = mk3(a_, b_, -(a_ * e.sx + b_ * e.sy));
         const f3 vhu = cross(e.hv, vz), vhv = cross(vz, e.hu);
-        vals[GS::kM + 0] -= vhu.x; vals[GS::kM + 1] -= vhu.y; vals[GS::kM + 2] -= vhu.z;
-        vals[GS::kM + 3] -= vhv.x; vals[GS::kM + 4] -= vhv.y; vals[GS::kM + 5] -= vhv.z;
-        vals[GS::kM + 6] += P.px * vhu.x + P.py * vhv.x;
-        vals[GS::kM + 7] += P.px * vhu.y + P.py * vhv.y;
-        vals[GS::kM + 8] += P.px * vhu.z + P.py * vhv.z;
+        vals[GS::kM + 0] = -vhu.x; vals[GS::kM + 1] = -vhu.y; vals[GS::kM + 2] = -vhu.z;
+        vals[GS::kM + 3] = -vhv.x; vals[GS::kM + 4] = -vhv.y; vals[GS::kM + 5] = -vhv.z;
+        vals[GS::kM + 6] = P.px * vhu.x + P.py * vhv.x;
+        vals[GS::kM + 7] = P.px * vhu.y + P.py * vhv.y;
+        vals[GS::kM + 8] = P.px * vhu.z + P.py * vhv.z;
     }
-#pragma unroll
-    for (int k = 0; k < D; ++k) P.buf[k] += (texc[k] + cp[k]) * fac;
-    P.buf_n[0] += nn.x * fac;
-    P.buf_n[1] += nn.y * fac;
-    P.buf_n[2] += nn.z * fac;
 }
 
-// One work item (tile) of the adjoint; every early return is uniform over the CTA.
-template <int D, class Tex, int PPT, class Filt = FiltBilinear>
+// Adds one sum straight to its gradient array (a caller without the packed rows).
+template <int D, bool kGeo>
+__device__ __forceinline__ void scatter_slot(const tg_raster_bwd_args& a, int64_t g, int slot, float v) {
+    using GS = GradSlots<D, kGeo>;
+    if (v == 0.f || slot >= GS::kUsed) return;
+    float* dst;
+    if (slot < GS::kM) dst = a.v_colors + g * D + slot;
+    else if (slot < GS::kXY) dst = a.v_ray_transforms + g * 9 + (slot - GS::kM);
+    else if (slot < GS::kOpac) dst = a.v_means2d + g * 2 + (slot - GS::kXY);
+    else if (slot == GS::kOpac) dst = a.v_opacities + g;
+    else if (slot < GS::kAbs) dst = a.v_normals + g * 3 + (slot - GS::kNrm);
+    else dst = a.v_means2d_abs ? a.v_means2d_abs + g * 2 + (slot - GS::kAbs) : nullptr;
+    if (dst) atomicAdd(dst, v);
+}
+
+// Staged splats and the lists of a batch.
+template <int D, class Tex, bool kGeo>
+struct BwdSmem {
+    static constexpr bool kScale = Tex::kFormat == TG_TEX_FP8_E4M3;
+    float4 *m0, *m1, *m2, *col, *nrm;
+    int *row, *entry;
+    float *col5, *scale;
+    uint32_t *words;   // [groups][n_words]
+    uint32_t *pixels;  // [n_words][threads]: the pixels' own bits
+    float4* extra;     // anisotropic_bilinear: the boundary integration's per-warp areas
+    __device__ __forceinline__ BwdSmem(float4* base, int bs, int side) {
+        m0 = base; m1 = m0 + bs; m2 = m1 + bs; col = m2 + bs; nrm = col + bs;
+        row = reinterpret_cast<int*>(nrm + (kGeo ? bs : 0));
+        entry = row + bs;
+        scale = reinterpret_cast<float*>(entry + bs);
+        col5 = scale + (kScale ? bs : 0);
+        words = reinterpret_cast<uint32_t*>(col5 + (D == 5 ? bs : 0));
+        pixels = words + (side * side / kGroupLanes) * (bs / 32);
+        extra = reinterpret_cast<float4*>(pixels + side * side * (bs / 32));
+    }
+    static size_t bytes(int bs, int side) {
+        return (size_t)bs * ((kGeo ? 5 : 4) * sizeof(float4) + 8 + (kScale ? 4 : 0) + (D == 5 ? 4 : 0)) +
+               (size_t)(side * side / kGroupLanes + side * side) * (bs / 32) * 4;
+    }
+};
+
+// One work item of the adjoint; every early return is uniform over the CTA.
+template <int D, class Tex, class Filt, bool kGeo>
 __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const float uv_scale, const int bs,
                                          const int64_t item) {
-    using GS = GradSlots<D>;
-    constexpr int NV = GS::kCount;
+    using GS = GradSlots<D, kGeo>;
+    constexpr int NS = GS::kCount;
+    constexpr unsigned kFull = 0xffffffffu;
+    constexpr bool kTextured = Tex::kFormat != TG_TEX_NONE;
     const tg_raster_fwd_args& f = a.f;
     extern __shared__ float4 smem4[];
-    const int nt = blockDim.x;  // tile_size^2 / PPT threads; bs = splats staged per batch
-    float4* s_box = smem4;  // per-splat cull box (see cull_box)
-    float4* s_xyo = s_box + bs;
-    float4* s_m0 = s_xyo + bs;
-    float4* s_m1 = s_m0 + bs;
-    float4* s_m2 = s_m1 + bs;
-    float4* s_nrm = s_m2 + bs;
-    float* s_col = reinterpret_cast<float*>(s_nrm + bs);
-    int* s_row = reinterpret_cast<int*>(s_col + bs * D);
-    int* s_g = s_row + bs;
-    float* s_grad = reinterpret_cast<float*>(s_g + bs);  // [bs][NV]
-    // anisotropic_bilinear: the boundary integration's per-warp area (16-byte aligned: bs is a multiple of 32)
-    float4* s_aniso = Filt::kAniso ? reinterpret_cast<float4*>(s_grad + bs * NV) + (threadIdx.x >> 5) * kAnisoWarpF4
-                                   : nullptr;
     __shared__ int s_max_bin;
+    const int nt = blockDim.x;  // one thread per pixel of the square
+    const int ts = f.tile_size, side = square_side(ts), subs = squares_per_tile(ts);
+    const BwdSmem<D, Tex, kGeo> S(smem4, bs, side);
+    float4* s_aniso = Filt::kAniso ? S.extra + (threadIdx.x >> 5) * kAnisoWarpF4 : nullptr;
 
-    const unsigned wmask = __activemask();
-    const TileWork tc = tile_work(f, item);
+    const TileWork tc = tile_work(f, subs == 1 ? item : item / subs);
     if (!tc.valid) return;  // uniform over the CTA
     const int tr = threadIdx.x, lane = tr & 31;
     if (f.masks != nullptr && !f.masks[tc.t]) return;
-
-    const int ts = f.tile_size;
+    const int sub = subs == 1 ? 0 : (int)(item % subs);
+    const int X0 = tc.tx * ts + (sub & 1) * side, Y0 = tc.ty * ts + (sub >> 1) * side;
+    const PixelSlot ps = pixel_slot(tr, side);
+    const int j = X0 + ps.x, i = Y0 + ps.y;
+    const int64_t pix = pixel_index(tc, i, j);
+    const bool inside = pix >= 0;
     const int32_t range_start = tc.range_start;
     const int32_t range_end = tc.range_end;
-
-    // pixel-centre rectangle covered by this warp (for the warp-level cull)
-    float wx0 = INFINITY, wx1 = -INFINITY, wy0 = INFINITY, wy1 = -INFINITY;
-#pragma unroll
-    for (int q = 0; q < PPT; ++q) {
-        const int local = tr + q * nt;
-        const float cx = (float)(tc.tx * ts + local % ts) + 0.5f, cy = (float)(tc.ty * ts + local / ts) + 0.5f;
-        wx0 = fminf(wx0, cx); wx1 = fmaxf(wx1, cx); wy0 = fminf(wy0, cy); wy1 = fmaxf(wy1, cy);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        wx0 = fminf(wx0, __shfl_xor_sync(wmask, wx0, o)); wx1 = fmaxf(wx1, __shfl_xor_sync(wmask, wx1, o));
-        wy0 = fminf(wy0, __shfl_xor_sync(wmask, wy0, o)); wy1 = fmaxf(wy1, __shfl_xor_sync(wmask, wy1, o));
-    }
-    for (int k = tr; k < bs * NV; k += nt) s_grad[k] = 0.f;
     if (tr == 0) s_max_bin = -1;
 
-    PixelAdj<D> P[PPT];
-    int32_t thread_bin = -1;
+    PixelAdj<D, kGeo> P;
+    P.px = (float)j + 0.5f;
+    P.py = (float)i + 0.5f;
+    P.T = 1.f;
+    P.rest = 0.f;
+    P.ck_batch = -1;
+    int32_t bin_final = -1;
+    int32_t rec = -1;  // anisotropic_bilinear: the forward's record of the next footprint integral (counting down)
 #pragma unroll
-    for (int q = 0; q < PPT; ++q) {
-        PixelAdj<D>& p = P[q];
-        const int local = tr + q * nt;
-        const int i = tc.ty * ts + local / ts;
-        const int j = tc.tx * ts + local % ts;
-        p.pix = pixel_index(tc, i, j);
-        p.inside = p.pix >= 0;
-        p.local = local;
-        p.ck_batch = -1;
-        p.rec = -1;
-        p.px = (float)j + 0.5f;
-        p.py = (float)i + 0.5f;
-        p.T_final = 1.f; p.v_a = p.v_dist = p.v_med = p.bg_dot = 0.f;
-        p.bin_final = -1; p.median_idx = -1;
-        p.acc_d_buf = p.acc_d = p.acc_w_buf = p.acc_w = p.dist_buf = 0.f;
-        p.v_n[0] = p.v_n[1] = p.v_n[2] = 0.f;
-        p.buf_n[0] = p.buf_n[1] = p.buf_n[2] = 0.f;
-#pragma unroll
-        for (int k = 0; k < D; ++k) { p.v_c[k] = 0.f; p.buf[k] = 0.f; }
-        if (p.inside) {
-            const int64_t px_ = p.pix;
-            const float alpha_out = a.render_alphas[px_];
-            p.T_final = 1.f - alpha_out;
-            p.bin_final = a.last_ids[px_];
-            p.median_idx = a.median_ids[px_];
-            if (Filt::kAniso && f.aniso_records != nullptr) p.rec = f.aniso_record_count[px_] - 1;
-#pragma unroll
-            for (int k = 0; k < D; ++k) p.v_c[k] = a.v_render_colors[px_ * D + k];
-            p.v_a = a.v_render_alphas[px_];
-            p.v_n[0] = a.v_render_normals[px_ * 3];
-            p.v_n[1] = a.v_render_normals[px_ * 3 + 1];
-            p.v_n[2] = a.v_render_normals[px_ * 3 + 2];
-            p.v_dist = a.v_render_distort[px_];
-            p.v_med = a.v_render_median[px_];
-            p.acc_d_buf = a.render_colors[px_ * D + D - 1];
-            p.acc_d = p.acc_d_buf;
-            p.acc_w_buf = alpha_out;
-            p.acc_w = alpha_out;
-            if (f.backgrounds) {
-#pragma unroll
-                for (int k = 0; k < D; ++k) p.bg_dot += f.backgrounds[tc.c * D + k] * p.v_c[k];
-            }
-        }
-        p.T = p.T_final;
-        thread_bin = max(thread_bin, p.bin_final);
+    for (int k = 0; k < D; ++k) P.v_c[k] = 0.f;
+    if constexpr (kGeo) {
+        P.v_n[0] = P.v_n[1] = P.v_n[2] = P.v_dist = P.v_med = 0.f;
+        P.acc_d_buf = P.acc_d = P.acc_w_buf = P.acc_w = 0.f;
+        P.median_idx = -1;
     }
-    // last contributor over the warp (uniform) and over the CTA
-    const int32_t warp_bin_final = __reduce_max_sync(wmask, thread_bin);
+    if (inside) {
+        const float alpha_out = a.render_alphas[pix];
+        P.T = 1.f - alpha_out;
+        bin_final = a.last_ids[pix];
+        float v_a = a.v_render_alphas ? a.v_render_alphas[pix] : 0.f;
+        if (a.v_render_colors) {
+#pragma unroll
+            for (int k = 0; k < D; ++k) P.v_c[k] = a.v_render_colors[pix * D + k];
+        }
+        if (f.backgrounds) {
+            float bg_dot = 0.f;
+#pragma unroll
+            for (int k = 0; k < D; ++k) bg_dot += f.backgrounds[tc.c * D + k] * P.v_c[k];
+            v_a -= bg_dot;
+        }
+        P.rest = P.T * v_a;
+        if constexpr (kGeo) {
+            P.median_idx = a.median_ids[pix];
+            if (a.v_render_normals) {
+                P.v_n[0] = a.v_render_normals[pix * 3];
+                P.v_n[1] = a.v_render_normals[pix * 3 + 1];
+                P.v_n[2] = a.v_render_normals[pix * 3 + 2];
+            }
+            if (a.v_render_distort) P.v_dist = a.v_render_distort[pix];
+            if (a.v_render_median) P.v_med = a.v_render_median[pix];
+            P.acc_d_buf = P.acc_d = a.render_colors[pix * D + D - 1];
+            P.acc_w_buf = P.acc_w = alpha_out;
+        }
+        if (Filt::kAniso && f.aniso_records != nullptr && f.contrib_masks != nullptr)
+            rec = f.aniso_record_count[pix] - 1;
+    }
+    // last contributor over the CTA
+    const int32_t warp_bin_final = __reduce_max_sync(kFull, bin_final);
     __syncthreads();
-    if (lane == __ffs(wmask) - 1) atomicMax(&s_max_bin, warp_bin_final);
+    if (lane == 0) atomicMax(&s_max_bin, warp_bin_final);
     __syncthreads();
-    const int32_t block_max_bin = s_max_bin;
+    const int32_t max_bin = min(s_max_bin, range_end - 1);
     const int64_t tex_stride = (int64_t)f.tex_ry * f.tex_rx;
     const int mip_clen = Filt::kMip ? ((1 << (2 * f.mip_levels)) - 1) / 3 : 0;
-    const int tile_px = nt * PPT;
-    const TileCkpt ck{f.t_checkpoints != nullptr
-                          ? f.t_checkpoints + ((int64_t)tc.t + range_start / bs) * (int64_t)tile_px : nullptr,
-                      (int64_t)tile_px, range_start, bs};
+    const int n_words = bs >> 5;
+    const bool have_bits = f.contrib_masks != nullptr;
+    const uint32_t* bits_base = have_bits ? f.contrib_masks + ((int64_t)tc.t + (range_start >> 5)) * (int64_t)(ts * ts) +
+                                                sub * nt + tr
+                                          : nullptr;
+    const uint32_t* words = S.words + (size_t)(Filt::kAniso ? (tr >> 5) * 4 : tr >> 3) * n_words;
+    auto list_word = [&](int w) -> uint32_t {
+        if constexpr (Filt::kAniso) return words[w] | words[w + n_words] | words[w + 2 * n_words] | words[w + 3 * n_words];
+        else return words[w];
+    };
 
-    for (int32_t batch_end = range_end - 1; batch_end >= range_start; batch_end -= bs) {
-        if (batch_end - (bs - 1) > block_max_bin) continue;  // every splat here is past all last contributors
-        const int32_t batch_size = min(bs, batch_end + 1 - range_start);
-        __syncthreads();  // previous batch fully flushed before restaging
-        for (int slot = tr; slot < bs; slot += nt) {
-            const int32_t idx_load = batch_end - slot;
-            if (idx_load >= range_start) {
-                const int32_t g = f.flatten_ids[idx_load];
+    for (int b = max_bin < range_start ? -1 : (max_bin - range_start) / bs; b >= 0; --b) {
+        const int32_t batch_start = range_start + b * bs;
+        __syncthreads();  // previous batch done before restaging
+        const int last_word = (max_bin - batch_start) >> 5;  // the forward went at least this far
+        for (int slot = tr; slot < bs; slot += nt) {  // (whole warps: bs and nt are multiples of 32)
+            const int32_t idx = batch_start + slot;
+            uint32_t reach = 0u;
+            if (idx <= max_bin) {
+                const int32_t g = f.flatten_ids[idx];
                 const float2 xy = reinterpret_cast<const float2*>(f.means2d)[g];
                 const int32_t row = f.gaussian_ids ? (int32_t)f.gaussian_ids[g] : g % f.N;
-                const float scale = (Tex::kFormat == TG_TEX_FP8_E4M3) ? f.tex_scales[row] : 1.f;
-                s_xyo[slot] = make_float4(xy.x, xy.y, f.opacities[g], scale);
+                const float op = f.opacities[g];
                 const float* m = f.ray_transforms + 9 * (int64_t)g;
-                s_m0[slot] = make_float4(m[0], m[1], m[2], 0.f);
-                s_m1[slot] = make_float4(m[3], m[4], m[5], 0.f);
-                s_m2[slot] = make_float4(m[6], m[7], m[8], 0.f);
-                s_box[slot] = cull_box(s_xyo[slot], s_m0[slot], s_m1[slot], s_m2[slot], Tex::kFormat != TG_TEX_NONE,
-                                       f.range_x, f.range_y, f.g_weight, !Filt::kAniso);
-                const float* n = f.normals + 3 * (int64_t)g;
-                s_nrm[slot] = make_float4(n[0], n[1], n[2], 0.f);
-#pragma unroll
-                for (int k = 0; k < D; ++k) s_col[slot * D + k] = f.colors[(int64_t)g * D + k];
-                s_row[slot] = row;
-                s_g[slot] = g;
-            }
-        }
-        __syncthreads();
-        for (int t = max(0, batch_end - warp_bin_final); t < batch_size; ++t) {
-            const int32_t idx = batch_end - t;
-            const float4 box = s_box[t];
-            if (box.z < wx0 || box.x > wx1 || box.w < wy0 || box.y > wy1) continue;  // no pixel of this warp can be valid
-            const float4 xyo = s_xyo[t], m0 = s_m0[t], m1 = s_m1[t], m2 = s_m2[t];
-            const int row = s_row[t];
-            const int64_t tex_base = (int64_t)row * tex_stride;
-            const float4 nn = s_nrm[t];
-            const float* cp = s_col + t * D;
-            float* vt = a.v_textures != nullptr ? a.v_textures + 4 * tex_base : nullptr;
-            float* vct = Filt::kMip && a.v_tex_coarse != nullptr ? a.v_tex_coarse + 4 * (int64_t)row * mip_clen
-                                                                 : nullptr;
-            float vals[32];
-#pragma unroll
-            for (int k = 0; k < 32; ++k) vals[k] = 0.f;
-            bool any = false;
-#pragma unroll
-            for (int q = 0; q < PPT; ++q) {
-                if constexpr (Filt::kAniso) {  // every lane takes part: the warp integrates footprints together
-                    const bool act = P[q].inside && idx <= P[q].bin_final && in_box(box, P[q].px, P[q].py);
-                    // the forward's integral of this pair's footprint, if it has one (it keeps the first
-                    // aniso_record_cap of each pixel's, in order; this walks them back to front)
-                    const float4* rec = act && P[q].rec >= 0 && P[q].rec < f.aniso_record_cap
-                                            ? reinterpret_cast<const float4*>(f.aniso_records) +
-                                                  P[q].pix * f.aniso_record_cap + P[q].rec
-                                            : nullptr;
-                    PairOf<Filt> e;
-                    eval_aniso_coop<Tex, true>(e, act, P[q].px, P[q].py, xyo, m0, m1, m2, f.textures, tex_base, f.tex_rx,
-                                         f.tex_ry, f.range_x, f.range_y, f.g_weight, wmask,
-                                         f.aniso_prefix ? reinterpret_cast<const float4*>(f.aniso_prefix) + tex_base
-                                                        : nullptr,
-                                         s_aniso, rec);
-                    if (e.tex_valid) --P[q].rec;  // this pair's footprint was integrated (or read): one record
-                    const bool use = act && e.valid;
-                    float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (use) {
-                        any = true;
-                        accumulate_pair<D, Tex, Filt>(a, e, P[q], xyo, nn, cp, idx, vt, uv_scale, vals, ck, vct,
-                                                      mip_clen, &g4);
-                    }
-                    aniso_coop_scatter<true>(e.F, g4,
-                                       use && e.tex_valid && vt != nullptr &&
-                                           (g4.x != 0.f || g4.y != 0.f || g4.z != 0.f || g4.w != 0.f),
-                                       vt, f.tex_rx, wmask,
-                                       a.v_aniso_prefix != nullptr ? a.v_aniso_prefix + 4 * tex_base : nullptr,
-                                       f.tex_ry, s_aniso);
-                    continue;
+                const float4 m0 = make_float4(m[0], m[1], m[2], xy.x), m1 = make_float4(m[3], m[4], m[5], xy.y),
+                             m2 = make_float4(m[6], m[7], m[8], op);
+                S.m0[slot] = m0;
+                S.m1[slot] = m1;
+                S.m2[slot] = m2;
+                const float* c = f.colors + (int64_t)g * D;
+                S.col[slot] = make_float4(c[0], D > 1 ? c[D > 1 ? 1 : 0] : 0.f, D > 2 ? c[D > 2 ? 2 : 0] : 0.f,
+                                          D > 3 ? c[D > 3 ? 3 : 0] : 0.f);
+                if constexpr (D == 5) S.col5[slot] = c[4];
+                if constexpr (kGeo) {
+                    const float* n = f.normals + 3 * (int64_t)g;
+                    S.nrm[slot] = make_float4(n[0], n[1], n[2], 0.f);
                 }
-                if (!(P[q].inside && idx <= P[q].bin_final) || !in_box(box, P[q].px, P[q].py)) continue;
-                PairOf<Filt> e;
-                eval_pair<Tex, Filt>(e, P[q].px, P[q].py, xyo, m0, m1, m2, f.textures, tex_base, f.tex_rx,
-                                     f.tex_ry, f.range_x, f.range_y, f.g_weight,
-                                     MipSrc{f.tex_coarse, (int64_t)row * mip_clen, mip_clen, f.mip_levels});
-                if (!e.valid) continue;
-                any = true;
-                accumulate_pair<D, Tex, Filt>(a, e, P[q], xyo, nn, cp, idx, vt, uv_scale, vals, ck, vct, mip_clen);
+                if constexpr (BwdSmem<D, Tex, kGeo>::kScale) S.scale[slot] = f.tex_scales[row];
+                S.row[slot] = row;
+                S.entry[slot] = g;
+                if (!have_bits)
+                    reach = group_mask(make_float4(xy.x, xy.y, op, 1.f), m0, m1, m2, kTextured, f.range_x, f.range_y,
+                                       f.g_weight, !Filt::kAniso, X0, Y0, side);
             }
-            if (!__any_sync(wmask, any)) continue;
-            warp_reduce_scatter32(vals, wmask);
-            if (lane < NV && vals[0] != 0.f) atomicAdd(s_grad + t * NV + lane, vals[0]);
+            if (!have_bits) store_group_words(reach, S.words, n_words, slot >> 5, side);
+        }
+        for (int w = 0; w < n_words; ++w) {
+            uint32_t own = inside ? kFull : 0u;
+            if (have_bits) {
+                own = w <= last_word ? bits_base[(int64_t)(b * n_words + w) * (ts * ts)] : 0u;
+                uint32_t u = own | __shfl_xor_sync(kFull, own, 4);
+                u |= __shfl_xor_sync(kFull, u, 2);
+                u |= __shfl_xor_sync(kFull, u, 1);
+                if ((lane & 7) == 0) S.words[(tr >> 3) * n_words + w] = u;
+            }
+            S.pixels[w * nt + tr] = own;
         }
         __syncthreads();
-        // flush this batch's per-splat sums: one global atomic per (splat, value)
-        for (int k = tr; k < batch_size * NV; k += nt) {
-            const float v = s_grad[k];
-            if (v == 0.f) continue;
-            s_grad[k] = 0.f;
-            const int t = k / NV, slot = k - t * NV;
-            const int64_t g = s_g[t];
-            float* dst;
-            if (slot < GS::kNrm) dst = a.v_colors + g * D + slot;
-            else if (slot < GS::kM) dst = a.v_normals + g * 3 + (slot - GS::kNrm);
-            else if (slot < GS::kXY) dst = a.v_ray_transforms + g * 9 + (slot - GS::kM);
-            else if (slot < GS::kOpac) dst = a.v_means2d + g * 2 + (slot - GS::kXY);
-            else if (slot == GS::kOpac) dst = a.v_opacities + g;
-            else dst = a.v_means2d_abs ? a.v_means2d_abs + g * 2 + (slot - GS::kAbs) : nullptr;
-            if (dst) atomicAdd(dst, v);
+        int w = n_words - 1;
+        uint32_t bits = list_word(w), own = S.pixels[w * nt + tr];
+        for (;;) {
+            while (bits == 0u && w > 0) {
+                bits = list_word(--w);
+                own = S.pixels[w * nt + tr];
+            }
+            if (!__any_sync(kFull, bits != 0u)) break;
+            const bool listed = bits != 0u;  // (a group whose list is used up idles until its warp's others are done)
+            const int bit = listed ? 31 - __clz(bits) : 0;
+            bits &= ~(1u << bit);
+            const int t = w * 32 + bit;
+            const int32_t idx = batch_start + t;
+            const bool act = listed && ((own >> bit) & 1u) != 0u && idx <= bin_final;
+            float vals[NS];
+#pragma unroll
+            for (int k = 0; k < NS; ++k) vals[k] = 0.f;
+            if (Filt::kAniso || act) {
+                const float4 m0 = S.m0[t], m1 = S.m1[t], m2 = S.m2[t];
+                const float4 xyo = make_float4(m0.w, m1.w, m2.w, BwdSmem<D, Tex, kGeo>::kScale ? S.scale[t] : 1.f);
+                const int row = S.row[t];
+                const int64_t tex_base = (int64_t)row * tex_stride;
+                float* vt = a.v_textures != nullptr ? a.v_textures + 4 * tex_base : nullptr;
+                float* vct = Filt::kMip && a.v_tex_coarse != nullptr ? a.v_tex_coarse + 4 * (int64_t)row * mip_clen
+                                                                     : nullptr;
+                PairOf<Filt> e;
+                if constexpr (Filt::kAniso) {  // every lane takes part: the warp integrates footprints together
+                    // the forward's integral of this pair's footprint, if it has one (it keeps the first
+                    // aniso_record_cap contributors of each pixel, in order; this walks them back to front)
+                    const float4* r = act && rec >= 0 && rec < f.aniso_record_cap
+                                          ? reinterpret_cast<const float4*>(f.aniso_records) +
+                                                pix * f.aniso_record_cap + rec
+                                          : nullptr;
+                    eval_aniso_coop<Tex, true>(e, act, P.px, P.py, xyo, m0, m1, m2, f.textures, tex_base, f.tex_rx,
+                                               f.tex_ry, f.range_x, f.range_y, f.g_weight, kFull,
+                                               f.aniso_prefix ? reinterpret_cast<const float4*>(f.aniso_prefix) + tex_base
+                                                              : nullptr,
+                                               s_aniso, r);
+                    if (act) --rec;
+                } else {
+                    eval_pair<Tex, Filt>(e, P.px, P.py, xyo, m0, m1, m2, f.textures, tex_base, f.tex_rx, f.tex_ry,
+                                         f.range_x, f.range_y, f.g_weight,
+                                         MipSrc{f.tex_coarse, (int64_t)row * mip_clen, mip_clen, f.mip_levels});
+                }
+                float4 g4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                const bool use = act && e.valid;
+                if (use) {
+                    if (f.t_checkpoints != nullptr && b != P.ck_batch) {
+                        // first pair of a new forward batch (back to front): T restarts from the forward's exact
+                        // value at the batch's end -- no splat after this one in the batch contributed to this
+                        // pixel, or it would have been met first
+                        P.ck_batch = b;
+                        P.T = f.t_checkpoints[((int64_t)tc.t + range_start / bs + b) * (int64_t)(ts * ts) +
+                                              (i - tc.ty * ts) * ts + (j - tc.tx * ts)];
+                    }
+                    const float4 c4 = S.col[t];
+                    float cp[D];
+#pragma unroll
+                    for (int k = 0; k < D; ++k) cp[k] = k < 4 ? f4get(c4, k) : S.col5[t];
+                    const float4 nn = kGeo ? S.nrm[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    accumulate_pair<D, Tex, Filt, kGeo, NS>(a, e, P, xyo.z, nn, cp, idx, vt, uv_scale, vals, vct,
+                                                            mip_clen, &g4);
+                }
+                if constexpr (Filt::kAniso)
+                    aniso_coop_scatter<true>(e.F, g4,
+                                             use && e.tex_valid && vt != nullptr &&
+                                                 (g4.x != 0.f || g4.y != 0.f || g4.z != 0.f || g4.w != 0.f),
+                                             vt, f.tex_rx, kFull,
+                                             a.v_aniso_prefix != nullptr ? a.v_aniso_prefix + 4 * tex_base : nullptr,
+                                             f.tex_ry, s_aniso);
+            }
+            reduce_scatter8<NS>(vals);
+            if constexpr (Filt::kAniso) {  // the four groups hold the same splat
+#pragma unroll
+                for (int k = 0; k < NS / 8; ++k) {
+                    vals[k] += __shfl_xor_sync(kFull, vals[k], 8);
+                    vals[k] += __shfl_xor_sync(kFull, vals[k], 16);
+                }
+                if (lane >= 8) continue;
+            }
+            const int64_t g = S.entry[t];
+            const int slot = slot_base<NS>(lane);
+            if (a.v_packed != nullptr) {
+                float* dst = a.v_packed + g * NS + slot;
+                if constexpr (NS == 16) {
+                    if (vals[0] != 0.f || vals[1] != 0.f)
+                        atomicAdd(reinterpret_cast<float2*>(dst), make_float2(vals[0], vals[1]));
+                } else {
+#pragma unroll
+                    for (int k = 0; k < NS / 8; ++k)
+                        if (vals[k] != 0.f) atomicAdd(dst + k, vals[k]);
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < NS / 8; ++k) scatter_slot<D, kGeo>(a, g, slot + k, vals[k]);
+            }
         }
     }
 }
 
 // CTA per work item, or (work_queue != NULL) a persistent grid whose CTAs take
 // items from the queue counter until none is left.
-template <int D, class Tex, int PPT, bool kPersistent, class Filt = FiltBilinear>
-__global__ void __launch_bounds__(256, BwdBounds<PPT, Filt>::kMinCtas) raster_bwd_kernel(const tg_raster_bwd_args a,
-                                                                                   const float uv_scale,
-                                                                                   const int bs,
-                                                                                   const int64_t n_items) {
+template <int D, class Tex, bool kPersistent, class Filt, bool kGeo>
+__global__ void __launch_bounds__(256, BwdBounds<Filt, kGeo>::kMinCtas) raster_bwd_kernel(const tg_raster_bwd_args a,
+                                                                                          const float uv_scale,
+                                                                                          const int bs,
+                                                                                          const int64_t n_items) {
     if constexpr (!kPersistent) {
-        bwd_tile<D, Tex, PPT, Filt>(a, uv_scale, bs, blockIdx.x);
+        bwd_tile<D, Tex, Filt, kGeo>(a, uv_scale, bs, blockIdx.x);
         return;
     }
     else {
@@ -484,7 +522,7 @@ __global__ void __launch_bounds__(256, BwdBounds<PPT, Filt>::kMinCtas) raster_bw
             const int64_t item = s_item;
             __syncthreads();  // s_item read by all before it is rewritten
             if (item >= n_items) return;
-            bwd_tile<D, Tex, PPT, Filt>(a, uv_scale, bs, item);
+            bwd_tile<D, Tex, Filt, kGeo>(a, uv_scale, bs, item);
         }
     }
 }
@@ -499,91 +537,115 @@ __global__ void densify_grad_kernel(const float* __restrict__ v_M, const float* 
     v_densify[2 * e + 1] = v_M[9 * e + 5] * depth;
 }
 
-size_t bwd_smem_bytes(int D, int bs) {
-    return (size_t)bs * (6 * sizeof(float4) + D * sizeof(float) + 2 * sizeof(int) + (D + 17) * sizeof(float));
-}
-
-// The mipmapped2 / anisotropic_bilinear kernels exist for FP32 / BF16 storage and 3 or 4 channels only.
-template <int D, class Tex, class Filt>
-constexpr bool filter_instance() {
-    return (D == 3 || D == 4) && (Tex::kFormat == TG_TEX_F32 || Tex::kFormat == TG_TEX_BF16);
-}
-template <int D, class Tex, class Filt>
-const void* filter_bwd_fn() {
-    if constexpr (filter_instance<D, Tex, Filt>()) return (const void*)raster_bwd_kernel<D, Tex, 1, false, Filt>;
-    else return nullptr;
-}
-template <int D, class Tex, class Filt>
-void launch_filter_bwd(dim3 g, dim3 b, size_t smem, cudaStream_t s, const tg_raster_bwd_args& a, float uv_scale, int bs,
-                       int64_t blocks) {
-    if constexpr (filter_instance<D, Tex, Filt>())
-        raster_bwd_kernel<D, Tex, 1, false, Filt><<<g, b, smem, s>>>(a, uv_scale, bs, blocks);
-}
-
-// The bilinear adjoint instances: 32x32 tiles (four pixels per thread) or not, persistent or not.
-template <int D, class Tex, class F>
-const void* bilinear_bwd_fn(bool four, bool pers) {
-    if constexpr (F::kUV && Tex::kFormat == TG_TEX_NONE) return nullptr;  // (never asked for)
-    else
-        return four ? (pers ? (const void*)raster_bwd_kernel<D, Tex, 4, true, F>
-                            : (const void*)raster_bwd_kernel<D, Tex, 4, false, F>)
-                    : (pers ? (const void*)raster_bwd_kernel<D, Tex, 1, true, F>
-                            : (const void*)raster_bwd_kernel<D, Tex, 1, false, F>);
-}
-template <int D, class Tex, class F>
-void launch_bilinear_bwd(bool four, bool pers, dim3 g, dim3 b, size_t smem, cudaStream_t s,
-                         const tg_raster_bwd_args& a, float uv_scale, int bs, int64_t blocks) {
-    if constexpr (!(F::kUV && Tex::kFormat == TG_TEX_NONE)) {
-        if (four && pers) raster_bwd_kernel<D, Tex, 4, true, F><<<g, b, smem, s>>>(a, uv_scale, bs, blocks);
-        else if (four) raster_bwd_kernel<D, Tex, 4, false, F><<<g, b, smem, s>>>(a, uv_scale, bs, blocks);
-        else if (pers) raster_bwd_kernel<D, Tex, 1, true, F><<<g, b, smem, s>>>(a, uv_scale, bs, blocks);
-        else raster_bwd_kernel<D, Tex, 1, false, F><<<g, b, smem, s>>>(a, uv_scale, bs, blocks);
+// Spreads the entries' packed rows over the gradient arrays (every element is written, so none is cleared first)
+// and forms v_densify.  128 rows per CTA go through shared memory, so that both the reads and the writes of the
+// odd-sized arrays are coalesced; the pass moves its bytes once (HBM-bound).
+template <int D, bool kGeo>
+__global__ void __launch_bounds__(128) unpack_grads_kernel(const tg_raster_bwd_args a) {
+    using GS = GradSlots<D, kGeo>;
+    constexpr int NS = GS::kCount, kRows = 128, kPitch = NS + 1;
+    __shared__ float s[kRows * kPitch];
+    const int64_t e0 = (int64_t)blockIdx.x * kRows;
+    const int n = (int)min((int64_t)kRows, a.n_elems - e0);
+    const float4* src = reinterpret_cast<const float4*>(a.v_packed + e0 * NS);
+    for (int k = threadIdx.x; k < n * (NS / 4); k += kRows) {
+        const float4 v = src[k];
+        float* d = s + (k / (NS / 4)) * kPitch + (k % (NS / 4)) * 4;
+        d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
     }
+    __syncthreads();
+    auto spread = [&](float* dst, int width, int off) {
+        for (int k = threadIdx.x; k < n * width; k += kRows) dst[e0 * width + k] = s[(k / width) * kPitch + off + k % width];
+    };
+    spread(a.v_colors, D, GS::kRgb);
+    spread(a.v_ray_transforms, 9, GS::kM);
+    spread(a.v_means2d, 2, GS::kXY);
+    spread(a.v_opacities, 1, GS::kOpac);
+    if constexpr (kGeo) {
+        spread(a.v_normals, 3, GS::kNrm);
+        if (a.v_means2d_abs) spread(a.v_means2d_abs, 2, GS::kAbs);
+    } else {
+        for (int k = threadIdx.x; k < n * 3; k += kRows) a.v_normals[e0 * 3 + k] = 0.f;
+    }
+    if ((int)threadIdx.x < n) {
+        const int64_t e = e0 + threadIdx.x;
+        const float depth = a.f.ray_transforms[9 * e + 8];
+        const float* r = s + threadIdx.x * kPitch + GS::kM;
+        reinterpret_cast<float2*>(a.v_densify)[e] = make_float2(r[2] * depth, r[5] * depth);
+    }
+}
+
+// Whether the call needs the sums of the geometric upstream gradients (else the smaller rows do).
+bool bwd_geo(const tg_raster_bwd_args& a) {
+    return a.v_render_normals != nullptr || a.v_render_distort != nullptr || a.v_render_median != nullptr ||
+           a.v_means2d_abs != nullptr || a.adjoint != TG_ADJ_REFERENCE || !(a.f.D == 3 || a.f.D == 4);
+}
+// Floats per entry of v_packed that a call uses (include/tg2dgs.h: callers provide the larger size).
+int bwd_slots(const tg_raster_bwd_args& a) { return bwd_geo(a) ? 24 : 16; }
+
+template <int D, class Tex, bool kPersistent, class Filt, bool kGeo>
+cudaError_t launch_bwd_kernel(const tg_raster_bwd_args& a, float uv_scale, cudaStream_t s) {
+    const tg_raster_fwd_args& f = a.f;
+    const int side = square_side(f.tile_size), threads = side * side;
+    const int bs = f.batch_depth > 0 ? f.batch_depth : f.tile_size * f.tile_size;
+    const size_t smem = BwdSmem<D, Tex, kGeo>::bytes(bs, side) +
+                        (Filt::kAniso ? (size_t)(threads / 32) * kAnisoWarpF4 * 16 : 0);
+    const int64_t tiles = f.views ? f.n_tiles : (int64_t)f.C * f.tile_width * f.tile_height;
+    const int64_t items = tiles * squares_per_tile(f.tile_size);
+    if (items > 0x7fffffff) return cudaErrorInvalidValue;
+    const auto fn = raster_bwd_kernel<D, Tex, kPersistent, Filt, kGeo>;
+    cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return err;
+    if (items > 0 && f.n_isects > 0) {
+        int64_t grid = items;
+        if (kPersistent) {
+            if ((err = cudaMemsetAsync(f.work_queue, 0, sizeof(uint32_t), s)) != cudaSuccess) return err;
+            if ((err = persistent_grid((const void*)fn, threads, smem, items, grid)) != cudaSuccess) return err;
+        }
+        fn<<<(unsigned)grid, threads, smem, s>>>(a, uv_scale, bs, items);
+        note_launches(1);
+        if ((err = cudaGetLastError()) != cudaSuccess) return err;
+    }
+    if (a.n_elems > 0) {
+        if (a.v_packed != nullptr)
+            unpack_grads_kernel<D, kGeo><<<(unsigned)((a.n_elems + 127) / 128), 128, 0, s>>>(a);
+        else
+            densify_grad_kernel<<<(unsigned)((a.n_elems + 255) / 256), 256, 0, s>>>(a.v_ray_transforms,
+                                                                                   f.ray_transforms, a.n_elems,
+                                                                                   a.v_densify);
+        note_launches(1);
+    }
+    return cudaGetLastError();
+}
+
+template <int D, class Tex, class Filt, bool kGeo>
+cudaError_t launch_bwd_bilinear(const tg_raster_bwd_args& a, float uv_scale, cudaStream_t s) {
+    return a.f.work_queue != nullptr ? launch_bwd_kernel<D, Tex, true, Filt, kGeo>(a, uv_scale, s)
+                                     : launch_bwd_kernel<D, Tex, false, Filt, kGeo>(a, uv_scale, s);
 }
 
 template <int D, class Tex>
 cudaError_t launch_bwd_t(const tg_raster_bwd_args& a, cudaStream_t s) {
-    const tg_raster_fwd_args& f = a.f;
-    const int tile_px = f.tile_size * f.tile_size;
-    const int bs = f.batch_depth > 0 ? f.batch_depth : tile_px;
-    size_t smem = bwd_smem_bytes(D, bs);
-    const int64_t blocks = f.views ? f.n_tiles : (int64_t)f.C * f.tile_width * f.tile_height;
-    const float uv_scale = a.adjoint == TG_ADJ_BWD2 ? 1.f : (a.adjoint == TG_ADJ_EXACT ? 0.5f : 0.f);
-    // mipmapped2 / anisotropic_bilinear: one pixel per thread, one CTA per tile
-    const bool mip = f.mip_levels > 0, aniso = f.filter == TG_FILTER_ANISO_BILINEAR;
-    if (aniso) smem += (size_t)(tile_px / 32) * kAnisoWarpF4 * 16;  // the boundary integration's per-warp area
-    if ((mip || aniso) && !filter_instance<D, Tex, FiltMip2>()) return cudaErrorInvalidValue;
-    const bool four = tile_px > 256;  // 32x32 tiles: four pixels per thread, 256 threads
-    const bool pers = f.work_queue != nullptr;
-    // the bwd2 / exact adjoints (uv_scale != 0) take the instances that carry the UV term
-    const bool uv = Tex::kFormat != TG_TEX_NONE && uv_scale != 0.f;
-    const void* fn = mip ? filter_bwd_fn<D, Tex, FiltMip2>()
-                   : aniso ? filter_bwd_fn<D, Tex, FiltAniso>()
-                   : uv ? bilinear_bwd_fn<D, Tex, FiltBilinearUV>(four, pers)
-                        : bilinear_bwd_fn<D, Tex, FiltBilinear>(four, pers);
-    const int threads = four ? tile_px / 4 : tile_px;
-    cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return err;
-    if (blocks > 0 && f.n_isects > 0) {
-        int64_t grid = blocks;
-        if (pers) {
-            if ((err = cudaMemsetAsync(f.work_queue, 0, sizeof(uint32_t), s)) != cudaSuccess) return err;
-            if ((err = persistent_grid(fn, threads, smem, blocks, grid)) != cudaSuccess) return err;
+    constexpr bool kTextured = Tex::kFormat != TG_TEX_NONE;
+    constexpr bool kSmallRows = D == 3 || D == 4;  // channel counts with instances for the smaller rows
+    const bool geo = bwd_geo(a);
+    const bool mip = a.f.mip_levels > 0, aniso = a.f.filter == TG_FILTER_ANISO_BILINEAR;
+    if (mip || aniso) {  // FP32 / BF16 storage and 3 or 4 channels only; one CTA per tile
+        if constexpr (kSmallRows && (Tex::kFormat == TG_TEX_F32 || Tex::kFormat == TG_TEX_BF16)) {
+            if (mip)
+                return geo ? launch_bwd_kernel<D, Tex, false, FiltMip2, true>(a, 0.f, s)
+                           : launch_bwd_kernel<D, Tex, false, FiltMip2, false>(a, 0.f, s);
+            return geo ? launch_bwd_kernel<D, Tex, false, FiltAniso, true>(a, 0.f, s)
+                       : launch_bwd_kernel<D, Tex, false, FiltAniso, false>(a, 0.f, s);
         }
-        const dim3 g((unsigned)grid), b((unsigned)threads);
-        if (mip) launch_filter_bwd<D, Tex, FiltMip2>(g, b, smem, s, a, uv_scale, bs, blocks);
-        else if (aniso) launch_filter_bwd<D, Tex, FiltAniso>(g, b, smem, s, a, uv_scale, bs, blocks);
-        else if (uv) launch_bilinear_bwd<D, Tex, FiltBilinearUV>(four, pers, g, b, smem, s, a, uv_scale, bs, blocks);
-        else launch_bilinear_bwd<D, Tex, FiltBilinear>(four, pers, g, b, smem, s, a, uv_scale, bs, blocks);
-        note_launches(1);
+        return cudaErrorInvalidValue;
     }
-    if ((err = cudaGetLastError()) != cudaSuccess) return err;
-    if (a.n_elems > 0)
-        densify_grad_kernel<<<(unsigned)((a.n_elems + 255) / 256), 256, 0, s>>>(a.v_ray_transforms,
-                                                                               f.ray_transforms, a.n_elems,
-                                                                               a.v_densify);
-    if (a.n_elems > 0) note_launches(1);
-    return cudaGetLastError();
+    if constexpr (kTextured)  // the bwd2 / exact adjoints take the instances that carry the UV term
+        if (a.adjoint != TG_ADJ_REFERENCE)
+            return launch_bwd_bilinear<D, Tex, FiltBilinearUV, true>(a, a.adjoint == TG_ADJ_BWD2 ? 1.f : 0.5f, s);
+    if constexpr (kSmallRows)
+        if (!geo) return launch_bwd_bilinear<D, Tex, FiltBilinear, false>(a, 0.f, s);
+    return launch_bwd_bilinear<D, Tex, FiltBilinear, true>(a, 0.f, s);
 }
 
 template <class Tex>

@@ -678,7 +678,7 @@ __device__ __forceinline__ void eval_pair(PairOf<Filt>& e, float px, float py, c
         e.g3 = e.sx * e.sx + e.sy * e.sy;
         e.dx = xyo.x - px;
         e.dy = xyo.y - py;
-        e.g2 = kFilterInvSquare * (e.dx * e.dx + e.dy * e.dy);
+        e.g2 = kFilterInvSquare * __fmaf_rn(e.dx, e.dx, e.dy * e.dy);  // (one rounding order in every instance)
         const float sigma = 0.5f * fminf(e.g3, e.g2);
         e.kern = __expf(-sigma);
         e.vis = 0.998f - g_weight + g_weight * e.kern;
@@ -761,7 +761,7 @@ __device__ __forceinline__ void eval_pair(PairOf<Filt>& e, float px, float py, c
     e.g3 = e.sx * e.sx + e.sy * e.sy;
     e.dx = xyo.x - px;
     e.dy = xyo.y - py;
-    e.g2 = kFilterInvSquare * (e.dx * e.dx + e.dy * e.dy);
+    e.g2 = kFilterInvSquare * __fmaf_rn(e.dx, e.dx, e.dy * e.dy);  // (one rounding order in every instance)
     const float sigma = 0.5f * fminf(e.g3, e.g2);
     e.kern = __expf(-sigma);
     if (kTextured) {

@@ -116,8 +116,7 @@ __device__ __forceinline__ void fwd_tile(const tg_raster_fwd_args& a, const int 
 
     float T = 1.f, pix_out[D], nrm_out[3] = {0.f, 0.f, 0.f}, distort = 0.f, accum_vis_depth = 0.f, median_depth = 0.f;
     int32_t cur_idx = 0, median_idx = 0;
-    // anisotropic_bilinear records: footprint integrals computed so far, and those up to the last contributor
-    int32_t rec_n = 0, rec_last = 0;
+    int32_t rec_n = 0;  // anisotropic_bilinear: contributors whose footprint integral was recorded (or counted)
     const bool records = Filt::kAniso && a.aniso_records != nullptr;
 #pragma unroll
     for (int k = 0; k < D; ++k) pix_out[k] = 0.f;
@@ -165,13 +164,23 @@ __device__ __forceinline__ void fwd_tile(const tg_raster_fwd_args& a, const int 
         }
         __syncthreads();
         int w = 0;
-        uint32_t bits = list_word(0);
+        uint32_t bits = list_word(0), own = 0u;  // own: this pixel's contributors among word w's splats
+        // the contributors' bits of this batch's words, for the adjoint
+        uint32_t* bits_out = a.contrib_masks != nullptr
+                                 ? a.contrib_masks + ((int64_t)tc.t + (range_start >> 5) + b * n_words) *
+                                                         (int64_t)(ts * ts) + sub * nt + tr
+                                 : nullptr;
+        const int live_words = min(n_words, (range_end - batch_start + 31) >> 5);
         for (;;) {
             const unsigned live = __ballot_sync(kFull, !done);
             const bool group_live = Filt::kAniso ? live != 0u : ((live >> (lane & 24)) & 0xffu) != 0u;
             if (!group_live) bits = 0u;
             else
-                while (bits == 0u && w + 1 < n_words) bits = list_word(++w);
+                while (bits == 0u && w + 1 < n_words) {
+                    if (bits_out != nullptr && w < live_words) bits_out[(int64_t)w * (ts * ts)] = own;
+                    own = 0u;
+                    bits = list_word(++w);
+                }
             if (!__any_sync(kFull, bits != 0u)) break;
             const bool act = bits != 0u && !done;
             const int t = w * 32 + (bits != 0u ? __ffs(bits) - 1 : 0);
@@ -190,11 +199,6 @@ __device__ __forceinline__ void fwd_tile(const tg_raster_fwd_args& a, const int 
                                          a.aniso_prefix ? reinterpret_cast<const float4*>(a.aniso_prefix) + tex_base
                                                         : nullptr,
                                          s_aniso);
-                    if (act && records && e.tex_valid) {  // every integral, in order, whether or not the pair is kept
-                        if (rec_n < a.aniso_record_cap)
-                            reinterpret_cast<float4*>(a.aniso_records)[pix * a.aniso_record_cap + rec_n] = e.tsum;
-                        ++rec_n;
-                    }
                 } else {
                     eval_pair<Tex, Filt>(e, px, py, xyo, m0, m1, m2, a.textures, tex_base, a.tex_rx, a.tex_ry, a.range_x,
                                          a.range_y, a.g_weight,
@@ -225,7 +229,14 @@ __device__ __forceinline__ void fwd_tile(const tg_raster_fwd_args& a, const int 
                             median_idx = batch_start + t;
                         }
                         cur_idx = batch_start + t;
-                        rec_last = rec_n;
+                        if constexpr (Filt::kAniso)
+                            if (records) {
+                                if (rec_n < a.aniso_record_cap)
+                                    reinterpret_cast<float4*>(a.aniso_records)[pix * a.aniso_record_cap + rec_n] =
+                                        e.tsum;
+                                ++rec_n;
+                            }
+                        own |= 1u << (t & 31);
                         T = next_T;
                         // counted in the top four bits: eight lanes' alphas (each < 1) fit below them
                         if (e.alpha > a.contrib_threshold) stat = __float2uint_rn(e.alpha * 16777216.f) | (1u << 28);
@@ -250,6 +261,8 @@ __device__ __forceinline__ void fwd_tile(const tg_raster_fwd_args& a, const int 
                 }
             }
         }
+        if (bits_out != nullptr)
+            for (; w < live_words; ++w, own = 0u) bits_out[(int64_t)w * (ts * ts)] = own;
         if (a.t_checkpoints != nullptr)  // every pixel's transmittance at the end of this batch
             a.t_checkpoints[((int64_t)tc.t + range_start / bs + b) * (int64_t)(ts * ts) +
                             (i - tc.ty * ts) * ts + (j - tc.tx * ts)] = T;
@@ -268,7 +281,7 @@ __device__ __forceinline__ void fwd_tile(const tg_raster_fwd_args& a, const int 
     a.out_distort[pix] = distort;
     a.out_median[pix] = median_depth;
     a.median_ids[pix] = median_idx;
-    if (records) a.aniso_record_count[pix] = rec_last;
+    if (records) a.aniso_record_count[pix] = rec_n;
 }
 
 // CTA per work item, or (work_queue != NULL) a persistent grid whose CTAs take

@@ -719,6 +719,9 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
         a.contrib_sum, a.contrib_count = B.ptr(contrib_sum), B.ptr(contrib_count)
         ckpt = _checkpoint_buffer(layout, isect_offsets, flatten_ids, tile_size, C, dev)
         a.t_checkpoints = B.ptr(ckpt)
+        masks_buf = _contrib_masks(layout, isect_offsets, flatten_ids, tile_size, C, dev) if any(
+            ctx.needs_input_grad) else None
+        a.contrib_masks = B.ptr(masks_buf)
         st = B.stream_of(means2d)
         prefix = _aniso_prefix(tex_store, tex_scales, st) if filter_code == B.TG_FILTER_ANISO_BILINEAR else None
         a.aniso_prefix = B.ptr(prefix)
@@ -742,7 +745,9 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
         ctx.t_checkpoints = ckpt
         ctx.aniso_prefix = prefix
         ctx.aniso_records = (records, counts)
+        ctx.contrib_masks = masks_buf
         ctx.mark_non_differentiable(contrib_sum, contrib_count)
+        ctx.set_materialize_grads(False)  # an output the loss does not use passes no gradient (NULL) to the adjoint
         return render_colors, render_alphas, render_normals, render_distort, render_median, contrib_sum, contrib_count
 
     @staticmethod
@@ -756,18 +761,13 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
         dev = means2d.device
         D = colors.shape[-1]
 
-        def g(t, shape):
-            return torch.zeros(shape, dtype=torch.float32, device=dev) if t is None else t.float().contiguous()
-
-        v_rc = g(v_render_colors, pshape + (D,))
-        v_ra = g(v_render_alphas, pshape + (1,))
-        v_rn = g(v_render_normals, pshape + (3,))
-        v_rd = g(v_render_distort, pshape + (1,))
-        v_rm = g(v_render_median, pshape + (1,))
+        v_rc, v_ra, v_rn, v_rd, v_rm = (None if t is None else t.float().contiguous() for t in (
+            v_render_colors, v_render_alphas, v_render_normals, v_render_distort, v_render_median))
         f = _fwd_args(means2d, ray_transforms, colors, opacities, normals, tex_store, tex_scales, range_x, range_y,
                       backgrounds, m, width, height, tile_size, isect_offsets, flatten_ids, gaussian_ids, n_contrib,
                       0.0, g_weight, C, N, ctx.layout, ctx.n_isects_dev, *ctx.mip)
         f.t_checkpoints = B.ptr(ctx.t_checkpoints)
+        f.contrib_masks = B.ptr(ctx.contrib_masks)
         f.aniso_prefix = B.ptr(ctx.aniso_prefix)
         if ctx.aniso_records[0] is not None:
             f.aniso_records, f.aniso_record_count = B.ptr(ctx.aniso_records[0]), B.ptr(ctx.aniso_records[1])
@@ -791,6 +791,8 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
         a.v_tex_coarse = B.ptr(v_coarse)
         v_prefix = torch.empty_like(ctx.aniso_prefix) if ctx.aniso_prefix is not None and want_tex else None
         a.v_aniso_prefix = B.ptr(v_prefix)
+        packed_rows = torch.empty((means2d.numel() // 2, 24), dtype=torch.float32, device=dev)
+        a.v_packed = B.ptr(packed_rows)
         st = B.stream_of(means2d)
         B.call("tg_rasterize_bwd", st, B.lib().tg_rasterize_bwd, ctypes.byref(a), st)
         if v_coarse is not None:
@@ -800,7 +802,9 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
             means2d.absgrad = v_means2d_abs
         v_backgrounds = None
         if bg_grad_index_ok and backgrounds is not None and ctx.needs_input_grad[7]:
-            if len(pshape) == 3:
+            if v_rc is None:
+                v_backgrounds = torch.zeros_like(backgrounds)
+            elif len(pshape) == 3:
                 v_backgrounds = (v_rc * (1.0 - render_alphas).float()).sum(dim=(1, 2))
             else:
                 vt = ctx.layout["view_table"]
@@ -839,6 +843,21 @@ def _checkpoint_buffer(layout, isect_offsets, flatten_ids, tile_size, C, device)
     bs = layout.get("batch_depth") or tile_size * tile_size
     return torch.empty((n_tiles + flatten_ids.numel() // bs + 1, tile_size * tile_size), dtype=torch.float32,
                        device=device)
+
+
+# Device memory for the contributors' bits a differentiated forward keeps (one bit per pixel and listed splat of its
+# tile); a call that would need more does without, and its adjoint tests every pair again.
+CONTRIB_MASK_BYTES = 8 << 30
+
+
+def _contrib_masks(layout, isect_offsets, flatten_ids, tile_size, C, device):
+    """The contrib_masks buffer of tg_raster_fwd_args: [n_tiles + n_isects / 32 + 1, tile_size^2] int32, or None."""
+    vt = None if layout is None else layout.get("view_table")
+    n_tiles = vt.n_tiles if vt is not None else C * isect_offsets.shape[1] * isect_offsets.shape[2]
+    rows = n_tiles + flatten_ids.numel() // 32 + 1
+    if rows * tile_size * tile_size * 4 > CONTRIB_MASK_BYTES:
+        return None
+    return torch.empty((rows, tile_size * tile_size), dtype=torch.int32, device=device)
 
 
 def _check_common(means2d, ray_transforms, colors, opacities, isect_offsets, tile_size, image_width, image_height,
