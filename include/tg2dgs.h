@@ -487,6 +487,16 @@ typedef struct {
 } tg_raster_bwd_args;
 TG_API int tg_rasterize_bwd(const tg_raster_bwd_args* a, tg_stream_t stream);
 
+/* ------------------------------------------------------------------ normal images
+ * Replaces the renderer's einsum of the inverse view matrices with the normal
+ * image (the end of rasterization_2dgs, textured_gaussians/rendering.py:1009-1338): out[p] = A_c in[p] for the
+ * pixels p of view c, A_c the upper-left 3x3 block of viewmats[c]^-1
+ * ([C,4,4] row-major; C <= 65535), or its transpose (the adjoint).  in / out:
+ * [n_pixels,3], view c's pixels at c * view_pixels, or, with `views`, at its
+ * pix_base (view_pixels is then the largest view's count). */
+TG_API int tg_rotate_normals(const float* viewmats, int32_t C, const tg_view* views, int64_t view_pixels,
+                             int64_t n_pixels, int32_t transpose, const float* in, float* out, tg_stream_t stream);
+
 /* ------------------------------------------------------------------ spherical harmonics
  * Replaces compute_sh_fwd_tensor / compute_sh_bwd_tensor
  * (textured_gaussians/cuda/csrc/compute_sh_fwd.cu, compute_sh_bwd.cu).

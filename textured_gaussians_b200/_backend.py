@@ -134,6 +134,7 @@ def lib() -> ctypes.CDLL:
                 ("tg_generate_mipmap", [P, P, I64, I32, P]),
                 ("tg_generate_mipmap_bwd", [P, P, I64, I32, P]),
                 ("tg_aniso_prefix", [P, I32, P, I64, I32, I32, P, P]),
+                ("tg_rotate_normals", [P, I32, P, I64, I64, I32, P, P, P]),
                 ("tg_sh_bwd", [I64, I64, I32, I32, P, P, P, P, P, P, P]),
             ]:
                 fn = getattr(L, name)

@@ -37,6 +37,7 @@ from .cuda._wrapper import (
     isect_offset_encode_views,
     isect_tiles,
     n_isects_of,
+    normals_to_world,
     rasterize_to_pixels_2dgs,
     rasterize_to_pixels_textured_gaussians,
     spherical_harmonics,
@@ -168,7 +169,7 @@ def rasterization_textured_gaussians_batch(
         means.contiguous(), quats.contiguous(), scales.contiguous(), viewmats.contiguous(), Ks.contiguous(), 0, 0,
         eps2d, near_plane, far_plane, radius_clip, False, mode, (vt.views, ranges, max_range), *sh)
     camera_ids, gaussian_ids, radii, means2d, depths, ray_transforms, normals = proj[:7]
-    opac = opacities[gaussian_ids]
+    opac = opacities.index_select(0, gaussian_ids)
     if fuse:
         cols = proj[-1]
     elif sh_degree is not None:
@@ -177,7 +178,7 @@ def rasterization_textured_gaussians_batch(
         cols = spherical_harmonics(sh_degree, dirs, colors[gaussian_ids], masks=radii > 0)
         cols = torch.clamp_min(cols + 0.5, 0.0)
     else:
-        cols = colors[gaussian_ids]
+        cols = colors.index_select(0, gaussian_ids)
     if render_mode in ("RGB+D", "RGB+ED"):
         cols = torch.cat((cols, depths[..., None]), dim=-1)
     elif render_mode in ("D", "ED"):
@@ -208,13 +209,12 @@ def rasterization_textured_gaussians_batch(
     if render_mode in ("ED", "RGB+ED"):
         flat_colors = torch.cat([flat_colors[..., :-1], flat_colors[..., -1:] / flat_alphas.clamp(min=1e-10)], dim=-1)
 
-    camtoworlds = _inverse(viewmats)
     colors_v, alphas_v = vt.split(flat_colors), vt.split(flat_alphas)
     median_v = vt.split(flat_median)
-    normals_v = [torch.einsum("ij,hwj->hwi", camtoworlds[c, :3, :3], n)
-                 for c, n in enumerate(vt.split(flat_normals))]
+    normals_v = vt.split(normals_to_world(flat_normals, viewmats, vt))
     normals_from_depth = None
     if render_mode in ("RGB+ED", "RGB+D"):
+        camtoworlds = _inverse(viewmats)
         normals_from_depth = []
         for c in range(C):
             d = colors_v[c][..., -1:] if depth_mode == "expected" else median_v[c]

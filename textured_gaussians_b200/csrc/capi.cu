@@ -51,6 +51,8 @@ cudaError_t launch_aniso_prefix(const void* textures, int tex_format, const floa
                                 int rx, float* prefix, cudaStream_t s);
 cudaError_t launch_aniso_prefix_fold(const float* v_prefix, int64_t G, int ry, int rx, float* v_textures,
                                      cudaStream_t s);
+cudaError_t launch_rotate_normals(const float* viewmats, int C, const tg_view* views, int64_t view_pixels,
+                                  int64_t n_pixels, int transpose, const float* in, float* out, cudaStream_t s);
 int fail_with(int code, const char* msg);
 }  // namespace tg
 
@@ -485,6 +487,15 @@ int tg_rasterize_bwd(const tg_raster_bwd_args* a, tg_stream_t stream) {
         e = tg::launch_aniso_prefix_fold(a->v_aniso_prefix, a->f.n_contrib, a->f.tex_ry, a->f.tex_rx, a->v_textures,
                                          stream);
     return cuda_status(e, "tg_rasterize_bwd");
+}
+
+int tg_rotate_normals(const float* viewmats, int32_t C, const tg_view* views, int64_t view_pixels, int64_t n_pixels,
+                      int32_t transpose, const float* in, float* out, tg_stream_t stream) {
+    TG_REQUIRE(C >= 0 && C <= 65535 && view_pixels >= 0 && n_pixels >= 0, TG_ERR_INVALID_ARG, "bad sizes");
+    if (C == 0 || view_pixels == 0 || n_pixels == 0) return TG_OK;
+    TG_REQUIRE(viewmats && in && out, TG_ERR_INVALID_ARG, "null pointer");
+    return cuda_status(tg::launch_rotate_normals(viewmats, C, views, view_pixels, n_pixels, transpose, in, out, stream),
+                       "tg_rotate_normals");
 }
 
 int tg_sh_fwd(int64_t n, int64_t coeff_rows, int32_t degree, int32_t K, const float* dirs, const float* coeffs,

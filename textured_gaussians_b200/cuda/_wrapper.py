@@ -1050,6 +1050,43 @@ def rasterize_to_pixels_2dgs(
     return (render_colors,) + tuple(out[1:])
 
 
+# --------------------------------------------------------------------------- normal images
+class _RotateNormals(torch.autograd.Function):
+    """World-space normal images: the upper-left block of each view matrix's inverse applied to its pixels."""
+
+    @staticmethod
+    def forward(ctx, normals, viewmats, views, view_pixels, transpose):
+        ctx.save_for_backward(viewmats)
+        ctx.cfg = (views, view_pixels, 1 - transpose)
+        x = normals.contiguous()
+        out = torch.empty_like(x)
+        st = B.stream_of(x)
+        B.call("tg_rotate_normals", st, B.lib().tg_rotate_normals, B.ptr(viewmats), viewmats.shape[0], B.ptr(views),
+               int(view_pixels), x.numel() // 3, transpose, B.ptr(x), B.ptr(out), st)
+        return out
+
+    @staticmethod
+    def backward(ctx, v_out):
+        return _RotateNormals.apply(v_out, *ctx.saved_tensors, *ctx.cfg), None, None, None, None
+
+
+def normals_to_world(normals: Tensor, viewmats: Tensor, view_table=None) -> Tensor:
+    """Camera-space normal images [C,H,W,3] (or flat [n_pixels,3] with ``view_table``) in world space.
+
+    View matrices that need a gradient, or other than FP32, take the torch expression (one matrix product per
+    view), as does a call on more views than the kernel's grid holds."""
+    if viewmats.requires_grad or viewmats.dtype != torch.float32 or normals.dtype != torch.float32 or \
+            viewmats.shape[0] > 65535 or viewmats.dim() != 3:
+        inv = torch.linalg.inv_ex(viewmats)[0][..., :3, :3]
+        if view_table is None:
+            return torch.einsum("...ij,...hwj->...hwi", inv, normals)
+        return torch.cat([torch.einsum("ij,pj->pi", inv[c], normals[b:b + n])
+                          for c, (b, n) in enumerate(zip(view_table.pix_base, view_table.pix_count))])
+    if view_table is None:
+        return _RotateNormals.apply(normals, viewmats.contiguous(), None, normals.shape[1] * normals.shape[2], 0)
+    return _RotateNormals.apply(normals, viewmats.contiguous(), view_table.views, max(view_table.pix_count), 0)
+
+
 # --------------------------------------------------------------------------- gradient consumers
 _SHADOW_FORMAT = {None: B.TG_TEX_NONE, torch.bfloat16: B.TG_TEX_BF16, torch.float16: B.TG_TEX_F16}
 

@@ -5,7 +5,7 @@ textured_gaussians/rendering.py:1009-1338 and :1342-1685 of the reference:
 projection -> tile intersection (+ sort) -> offsets -> SH colours -> compositor
 -> expected-depth normalisation / depth normals -> normals to world space.
 Every stage runs this package's sm_100a kernels; the glue between them
-(repeat of opacities, camera centres, clamps, ED division, normal rotation)
+(repeat of opacities, camera centres, clamps, ED division)
 is torch on the same device.
 
 ``packed=True`` runs the packed layout end to end (visible (camera, Gaussian)
@@ -40,6 +40,7 @@ from .cuda._wrapper import (
     isect_offset_encode,
     isect_tiles,
     n_isects_of,
+    normals_to_world,
     tile_order_heaviest_first,
     rasterize_to_pixels_2dgs,
     rasterize_to_pixels_textured_gaussians,
@@ -87,7 +88,7 @@ def _prepare(means, quats, scales, opacities, colors, viewmats, Ks, width, heigh
         sh_degree=sh_degree if fuse else None)
     if packed:
         camera_ids, gaussian_ids, radii, means2d, depths, ray_transforms, normals = proj[:7]
-        opacities = opacities[gaussian_ids]
+        opacities = opacities.index_select(0, gaussian_ids)  # (its adjoint adds with atomics instead of sorting the ids)
     else:
         radii, means2d, depths, ray_transforms, normals = proj[:5]
         opacities = opacities.repeat(C, 1)
@@ -115,7 +116,7 @@ def _prepare(means, quats, scales, opacities, colors, viewmats, Ks, width, heigh
             colors = spherical_harmonics_shared(sh_degree, dirs, colors, masks=radii > 0)  # [C, N, 3]
         colors = torch.clamp_min(colors + 0.5, 0.0)
     elif colors.dim() == 2:
-        colors = colors[gaussian_ids] if packed else colors.expand(C, *([-1] * colors.dim()))
+        colors = colors.index_select(0, gaussian_ids) if packed else colors.expand(C, *([-1] * colors.dim()))
     elif packed:
         colors = colors[camera_ids, gaussian_ids, :]
 
@@ -161,7 +162,7 @@ def _finish(p, render_colors, render_alphas, render_normals, render_distort, ren
         "render_distort": render_distort,
         "gradient_2dgs": p["densify"],
     }
-    render_normals = torch.einsum("...ij,...hwj->...hwi", _inverse(viewmats)[..., :3, :3], render_normals)
+    render_normals = normals_to_world(render_normals, viewmats)
     return (render_colors, render_alphas, render_normals, render_normals_from_depth, render_distort, render_median,
             gs_contrib_sum, gs_contrib_count, meta)
 
