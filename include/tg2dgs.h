@@ -265,6 +265,34 @@ TG_API size_t tg_scan_workspace_bytes(int64_t n_elems);
 TG_API int tg_isect_count(const tg_isect_args* a, tg_stream_t stream);
 TG_API int tg_isect_emit(const tg_isect_args* a, tg_stream_t stream);
 
+/* Sorted intersection lists, in two calls with the host's read of *n_isects
+ * between them, as for tg_isect_count / tg_isect_emit + tg_sort_pairs and with
+ * the same results (tiles_per_gauss, and isect_ids / flatten_ids sorted
+ * stably by the 32 + tile_bits + camera_bits low key bits): the entries are
+ * sorted by depth, and the intersections, written in that order, by camera and
+ * tile alone.
+ * tg_isect_sorted_count: tiles_per_gauss, *n_isects and the entries' order
+ * (left in order_ws); needs depths, not cum_tiles or scan_workspace.
+ * tg_isect_sorted_lists: isect_ids and flatten_ids [n], n = *n_isects; in
+ * capacity mode (overflow != NULL) n = capacity and the tail as described at
+ * `capacity`.  order_ws: what tg_isect_sorted_count filled, of
+ * tg_isect_sorted_order_bytes(n_elems) bytes; list_ws:
+ * tg_isect_sorted_lists_bytes(n, tile_bits + camera_bits) bytes, both 16-byte
+ * aligned.  n_elems and n below 2^30. */
+TG_API size_t tg_isect_sorted_order_bytes(int64_t n_elems);
+TG_API int tg_isect_sorted_count(const tg_isect_args* a, void* order_ws, size_t order_bytes, tg_stream_t stream);
+TG_API size_t tg_isect_sorted_lists_bytes(int64_t n, int32_t key_bits);
+TG_API int tg_isect_sorted_lists(const tg_isect_args* a, void* order_ws, int64_t n, void* list_ws, size_t list_bytes,
+                                 tg_stream_t stream);
+
+/* Work order for the compositor (tg_raster_fwd_args.tile_order): the tiles by
+ * descending list length, ties by index.  offsets [n_tiles] as from
+ * tg_isect_offset_encode; n_isects (or, if not NULL, *n_isects_dev, at most
+ * n_isects) ends the last tile's list.  ws: tg_tile_order_workspace_bytes. */
+TG_API size_t tg_tile_order_workspace_bytes(int64_t n_tiles);
+TG_API int tg_tile_order(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, const int64_t* n_isects_dev,
+                         int32_t* order, void* ws, size_t ws_bytes, tg_stream_t stream);
+
 /* Stable LSD onesweep radix sort of (int64 key, int32 value) pairs on key bits
  * [0, end_bit), ping-ponging between (keys, vals) and (keys_alt, vals_alt).
  * Replaces cub::DeviceRadixSort::SortPairs as called at
@@ -294,7 +322,7 @@ TG_API int tg_sort_lookback_selftest(int64_t* keys, int32_t* vals, int64_t* keys
  * that owns all GPU memory, a real-time loop that must not call cudaMalloc, a
  * host without a caching allocator).  No counterpart in the reference.  The
  * caller passes only keys, values and their ping-pong buffers; the scratch the
- * sort needs lives in a static device array of this library (8 MiB + 16 KiB
+ * sort needs lives in a static device array of this library (8 MiB + 8.5 KiB
  * held on every GPU that loads it, until exit), so n is limited to
  * TG_SORT_NOALLOC_MAX_PAIRS -- larger n is rejected with TG_ERR_INVALID_ARG.
  * Calls share that array: those that overlap on one GPU race and must be

@@ -121,6 +121,9 @@ def lib() -> ctypes.CDLL:
                 ("tg_project_packed_bwd", [ctypes.POINTER(ProjectPackedBwdArgs), P]),
                 ("tg_isect_count", [ctypes.POINTER(IsectArgs), P]),
                 ("tg_isect_emit", [ctypes.POINTER(IsectArgs), P]),
+                ("tg_isect_sorted_count", [ctypes.POINTER(IsectArgs), P, ctypes.c_size_t, P]),
+                ("tg_isect_sorted_lists", [ctypes.POINTER(IsectArgs), P, I64, P, ctypes.c_size_t, P]),
+                ("tg_tile_order", [P, I64, I64, P, P, P, ctypes.c_size_t, P]),
                 ("tg_sort_pairs", [P, P, P, P, I64, I32, P, ctypes.c_size_t, ctypes.POINTER(I32), P]),
                 ("tg_sort_status", [P, I64, I32, P]),
                 ("tg_sort_lookback_selftest", [P, P, P, P, P, ctypes.c_size_t, P]),
@@ -142,10 +145,14 @@ def lib() -> ctypes.CDLL:
                 fn.restype = ctypes.c_int
             L.tg_kernel_launch_count.restype = ctypes.c_uint64
             L.tg_kernel_launch_count.argtypes = []
-            for name in ("tg_scan_workspace_bytes", "tg_sort_workspace_bytes", "tg_project_packed_workspace_bytes"):
+            for name in ("tg_scan_workspace_bytes", "tg_sort_workspace_bytes", "tg_project_packed_workspace_bytes",
+                         "tg_isect_sorted_order_bytes", "tg_isect_sorted_lists_bytes", "tg_tile_order_workspace_bytes"):
                 getattr(L, name).restype = ctypes.c_size_t
             L.tg_project_packed_workspace_bytes.argtypes = [I32, I32]
             L.tg_scan_workspace_bytes.argtypes = [I64]
+            L.tg_isect_sorted_order_bytes.argtypes = [I64]
+            L.tg_isect_sorted_lists_bytes.argtypes = [I64, I32]
+            L.tg_tile_order_workspace_bytes.argtypes = [I64]
             L.tg_sort_workspace_bytes.argtypes = [I64, I32]
             _lib = L
     return _lib

@@ -22,6 +22,14 @@ cudaError_t launch_project_packed_bwd(const tg_project_packed_bwd_args& a, cudaS
 size_t scan_workspace_bytes(int64_t n_elems);
 cudaError_t launch_isect_count(const tg_isect_args& a, cudaStream_t s);
 cudaError_t launch_isect_emit(const tg_isect_args& a, int tile_n_bits, int end_bit, cudaStream_t s);
+size_t isect_order_workspace_bytes(int64_t E);
+cudaError_t launch_isect_order(const tg_isect_args& a, void* workspace, cudaStream_t s);
+size_t isect_lists_workspace_bytes(int64_t n, int key_bits);
+cudaError_t launch_isect_lists(const tg_isect_args& a, void* order_ws, int64_t n, int tile_bits, int key_bits, void* ws,
+                               cudaStream_t s);
+size_t tile_order_workspace_bytes(int64_t n_tiles);
+cudaError_t launch_tile_order(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, const int64_t* n_dev,
+                              int32_t* order, void* ws, cudaStream_t s);
 uint32_t* sort_error_flag(void* workspace, int64_t n, int end_bit);
 int sort_lookback_selftest(int64_t* keys, int32_t* vals, int64_t* keys_alt, int32_t* vals_alt, void* workspace,
                            size_t ws_bytes, cudaStream_t s, cudaError_t& cerr);
@@ -336,6 +344,65 @@ int tg_isect_emit(const tg_isect_args* a, tg_stream_t stream) {
     const int tb = bit_width((int64_t)a->tile_width * a->tile_height);
     const int cb = bit_width(a->n_cameras);
     return cuda_status(tg::launch_isect_emit(*a, tb, 32 + tb + cb, stream), "tg_isect_emit");
+}
+
+size_t tg_isect_sorted_order_bytes(int64_t n_elems) { return tg::isect_order_workspace_bytes(std::max<int64_t>(n_elems, 0)); }
+
+size_t tg_isect_sorted_lists_bytes(int64_t n, int32_t key_bits) {
+    return tg::isect_lists_workspace_bytes(std::max<int64_t>(n, 0), std::min(std::max(key_bits, 1), 32));
+}
+
+int tg_isect_sorted_count(const tg_isect_args* a, void* order_ws, size_t order_bytes, tg_stream_t stream) {
+    TG_REQUIRE(a != nullptr, TG_ERR_INVALID_ARG, "null args");
+    TG_REQUIRE(a->n_elems >= 0 && a->n_elems < (int64_t(1) << 30), TG_ERR_INVALID_ARG, "n_elems out of range");
+    TG_REQUIRE(a->tile_size > 0 && a->tile_width > 0 && a->tile_height > 0 && a->n_cameras > 0, TG_ERR_INVALID_ARG,
+               "bad tile grid");
+    TG_REQUIRE(bit_width((int64_t)a->tile_width * a->tile_height) + bit_width(a->n_cameras) <= 32, TG_ERR_INVALID_ARG,
+               "camera and tile ids need more than 32 bits");
+    TG_REQUIRE(a->n_isects, TG_ERR_INVALID_ARG, "null n_isects");
+    if (a->n_elems > 0) {
+        TG_REQUIRE(a->means2d && a->radii && a->depths && a->tiles_per_gauss && aligned(a->means2d, 8),
+                   TG_ERR_INVALID_ARG, "null or misaligned pointer");
+        TG_REQUIRE(a->camera_ids != nullptr || a->N > 0, TG_ERR_INVALID_ARG, "dense layout needs N > 0");
+        TG_REQUIRE(order_ws && aligned(order_ws, 16) && order_bytes >= tg::isect_order_workspace_bytes(a->n_elems),
+                   TG_ERR_WORKSPACE, "order workspace missing, misaligned or smaller than %zu bytes",
+                   tg::isect_order_workspace_bytes(a->n_elems));
+    }
+    return cuda_status(tg::launch_isect_order(*a, order_ws, stream), "tg_isect_sorted_count");
+}
+
+int tg_isect_sorted_lists(const tg_isect_args* a, void* order_ws, int64_t n, void* list_ws, size_t list_bytes,
+                          tg_stream_t stream) {
+    TG_REQUIRE(a != nullptr, TG_ERR_INVALID_ARG, "null args");
+    TG_REQUIRE(n >= 0 && n < (int64_t(1) << 30) && a->n_elems >= 0 && a->n_elems < (int64_t(1) << 30),
+               TG_ERR_INVALID_ARG, "sort supports up to 2^30 pairs");
+    TG_REQUIRE(!a->overflow || (a->capacity == n && a->n_isects), TG_ERR_INVALID_ARG,
+               "capacity mode needs n = capacity and n_isects");
+    if (n == 0) return TG_OK;
+    const int tb = bit_width((int64_t)a->tile_width * a->tile_height), cb = bit_width(a->n_cameras);
+    TG_REQUIRE(a->tile_width > 0 && a->tile_height > 0 && a->n_cameras > 0 && tb + cb <= 32, TG_ERR_INVALID_ARG,
+               "bad tile grid");
+    TG_REQUIRE(a->isect_ids && a->flatten_ids, TG_ERR_INVALID_ARG, "null pointer");
+    if (a->n_elems > 0)
+        TG_REQUIRE(a->means2d && a->radii && a->depths && order_ws && (a->camera_ids || a->N > 0), TG_ERR_INVALID_ARG,
+                   "null pointer");
+    TG_REQUIRE(list_ws && aligned(list_ws, 16) && list_bytes >= tg::isect_lists_workspace_bytes(n, tb + cb),
+               TG_ERR_WORKSPACE, "list workspace missing, misaligned or smaller than %zu bytes",
+               tg::isect_lists_workspace_bytes(n, tb + cb));
+    return cuda_status(tg::launch_isect_lists(*a, order_ws, n, tb, tb + cb, list_ws, stream), "tg_isect_sorted_lists");
+}
+
+size_t tg_tile_order_workspace_bytes(int64_t n_tiles) { return tg::tile_order_workspace_bytes(std::max<int64_t>(n_tiles, 0)); }
+
+int tg_tile_order(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, const int64_t* n_isects_dev,
+                  int32_t* order, void* ws, size_t ws_bytes, tg_stream_t stream) {
+    TG_REQUIRE(n_tiles >= 0 && n_tiles < (int64_t(1) << 30) && n_isects >= 0, TG_ERR_INVALID_ARG, "bad sizes");
+    if (n_tiles == 0) return TG_OK;
+    TG_REQUIRE(offsets && order && ws && aligned(ws, 16), TG_ERR_INVALID_ARG, "null or misaligned pointer");
+    TG_REQUIRE(ws_bytes >= tg::tile_order_workspace_bytes(n_tiles), TG_ERR_WORKSPACE, "workspace smaller than %zu bytes",
+               tg::tile_order_workspace_bytes(n_tiles));
+    return cuda_status(tg::launch_tile_order(offsets, n_tiles, n_isects, n_isects_dev, order, ws, stream),
+                       "tg_tile_order");
 }
 
 int tg_sort_lookback_selftest(int64_t* keys, int32_t* vals, int64_t* keys_alt, int32_t* vals_alt, void* workspace,

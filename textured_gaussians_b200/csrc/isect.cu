@@ -10,11 +10,20 @@
 // The sort is a hand-written LSD onesweep radix sort (8-bit digits): one
 // read of the keys builds the digit histograms of every pass, then each pass
 // is a single kernel whose CTAs take 4096-key tiles in launch order, rank the
-// keys with warp match-any, publish their digit counts and resolve their
-// global digit offsets by decoupled look-back over earlier tiles.  Every
-// look-back wait is bounded; a wait that gives up raises a workspace error
-// flag that the host turns into TG_ERR_TIMEOUT.
+// keys with warp ballots, publish their digit counts and resolve their
+// global digit offsets by decoupled look-back over earlier tiles (sort.cuh).
+// Every look-back wait is bounded; a wait that gives up raises a workspace
+// error flag that the host turns into TG_ERR_TIMEOUT.
+//
+// Sorted intersection lists (the renderer's path) do not sort the 64-bit keys.
+// An entry's intersections share its depth, so the entries are sorted by depth
+// once, their intersections written in that order, and only the (camera, tile)
+// half of the keys is left to sort -- stably, which gives the same order as
+// sorting the whole keys, ties included.  Against seven passes of 24 bytes a pair
+// over the intersections (1M splats x four 1600x1200 views, 30M of them, 4M
+// entries) that is four passes of 16 bytes an entry and three of 16-20 bytes a pair.
 #include "scan.cuh"
+#include "sort.cuh"
 
 namespace tg {
 
@@ -190,21 +199,10 @@ __global__ void __launch_bounds__(256) offset_encode_views_kernel(const int64_t*
 }
 
 // ------------------------------------------------------------------ onesweep radix sort
-constexpr int kSortThreads = 256;
-constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 16;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys per CTA
-constexpr int kRadix = 256;
 constexpr int kMaxPasses = 8;
-constexpr uint32_t kFlagAgg = 1u << 30;
-constexpr uint32_t kFlagInc = 2u << 30;
-constexpr uint32_t kFlagMask = 3u << 30;
-constexpr uint32_t kValueMask = kFlagAgg - 1u;
-constexpr uint32_t kSpinLimit = 1u << 22;  // ~0.3 s of polling with 64 ns sleeps
 
 struct SortWorkspace {
     uint32_t* hist;          // [kMaxPasses][256] digit counts
-    uint32_t* digit_offsets; // [kMaxPasses][256] exclusive scans
     uint32_t* tile_counter;  // [kMaxPasses]
     uint32_t* error;         // [1]
     uint32_t* status;        // [passes][n_tiles][256]
@@ -218,7 +216,6 @@ inline SortWorkspace carve_sort_workspace(void* base, int64_t n, int passes) {
     char* p = static_cast<char*>(base);
     size_t off = 0;
     w.hist = reinterpret_cast<uint32_t*>(p + off); off += align256(sizeof(uint32_t) * kMaxPasses * kRadix);
-    w.digit_offsets = reinterpret_cast<uint32_t*>(p + off); off += align256(sizeof(uint32_t) * kMaxPasses * kRadix);
     w.tile_counter = reinterpret_cast<uint32_t*>(p + off); off += align256(sizeof(uint32_t) * kMaxPasses);
     w.error = reinterpret_cast<uint32_t*>(p + off); off += align256(sizeof(uint32_t));
     w.status = reinterpret_cast<uint32_t*>(p + off); off += align256(sizeof(uint32_t) * (size_t)passes * n_tiles * kRadix);
@@ -241,152 +238,24 @@ __global__ void __launch_bounds__(kSortThreads) sort_histogram_kernel(const uint
         if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
 }
 
-__global__ void __launch_bounds__(kRadix) sort_digit_offsets_kernel(const uint32_t* hist, uint32_t* offsets) {
-    // one CTA per pass, one thread per digit
-    __shared__ uint32_t s[kRadix];
-    const int p = blockIdx.x, d = threadIdx.x;
-    s[d] = hist[p * kRadix + d];
-    __syncthreads();
-    // Hillis-Steele inclusive scan over 256 digits
-    for (int o = 1; o < kRadix; o <<= 1) {
-        const uint32_t v = d >= o ? s[d - o] : 0u;
-        __syncthreads();
-        s[d] += v;
-        __syncthreads();
-    }
-    offsets[p * kRadix + d] = s[d] - hist[p * kRadix + d];
-}
-
-__device__ __forceinline__ uint32_t ld_volatile(const uint32_t* p) { return *reinterpret_cast<const volatile uint32_t*>(p); }
-__device__ __forceinline__ void st_volatile(uint32_t* p, uint32_t v) { *reinterpret_cast<volatile uint32_t*>(p) = v; }
-
-__global__ void __launch_bounds__(kSortThreads) sort_pass_kernel(const uint64_t* __restrict__ keys_in,
+template <class Key>
+__global__ void __launch_bounds__(kSortThreads, 3) sort_pass_kernel(const Key* __restrict__ keys_in,
                                                                  const uint32_t* __restrict__ vals_in,
-                                                                 uint64_t* __restrict__ keys_out,
+                                                                 Key* __restrict__ keys_out,
                                                                  uint32_t* __restrict__ vals_out, int64_t n, int shift,
-                                                                 uint32_t digit_mask, const uint32_t* digit_offsets,
-                                                                 uint32_t* status, uint32_t* tile_counter,
-                                                                 uint32_t* error) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    uint64_t* s_keys = reinterpret_cast<uint64_t*>(smem_raw);
-    uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_keys + kSortTile);
-    uint32_t* s_whist = s_vals + kSortTile;             // [warps][256]
-    uint32_t* s_tile_start = s_whist + kSortWarps * kRadix;  // [256]
-    uint32_t* s_gbase = s_tile_start + kRadix;          // [256]
-    __shared__ uint32_t s_tile;
-    __shared__ uint32_t s_scan[kSortWarps];
-
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
-    for (int i = tid; i < kSortWarps * kRadix; i += kSortThreads) s_whist[i] = 0;
-    __syncthreads();
-    const uint32_t tile = s_tile;
-    const int64_t base = (int64_t)tile * kSortTile;
-
-    uint64_t k[kSortItems];
-    uint32_t v[kSortItems];
-    uint32_t dg[kSortItems];
-    uint32_t rk[kSortItems];
-    const int64_t wbase = base + (int64_t)warp * (kSortItems * 32);
-#pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-        const int64_t pos = wbase + i * 32 + lane;
-        const bool ok = pos < n;
-        k[i] = ok ? keys_in[pos] : 0ull;
-        v[i] = ok ? vals_in[pos] : 0u;
-        dg[i] = ok ? (uint32_t)((k[i] >> shift) & digit_mask) : (uint32_t)kRadix;  // kRadix marks padding
-    }
-    const unsigned lt = lanemask_lt();
-    uint32_t* wh = s_whist + warp * kRadix;
-#pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-        const unsigned peers = __match_any_sync(0xffffffffu, dg[i]);
-        const int leader = __ffs(peers) - 1;
-        uint32_t b = 0;
-        if (lane == leader && dg[i] < (uint32_t)kRadix) {
-            b = wh[dg[i]];
-            wh[dg[i]] = b + __popc(peers);
-        }
-        b = __shfl_sync(peers, b, leader);
-        rk[i] = b + __popc(peers & lt);
-    }
-    __syncthreads();
-
-    // per digit (thread = digit): exclusive scan over warps, tile total
-    const int d = tid;
-    uint32_t count = 0;
-#pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) {
-        const uint32_t c = s_whist[w * kRadix + d];
-        s_whist[w * kRadix + d] = count;
-        count += c;
-    }
-    uint32_t* st = status + (size_t)tile * kRadix;
-    if (tile == 0) {
-        st_volatile(st + d, kFlagInc | count);
-    } else {
-        st_volatile(st + d, kFlagAgg | count);
-    }
-    uint32_t prefix = 0;
-    if (tile > 0) {
-        int64_t j = (int64_t)tile - 1;
-        while (j >= 0) {
-            const uint32_t* src = status + (size_t)j * kRadix + d;
-            uint32_t s = ld_volatile(src);
-            uint32_t iter = 0;
-            while ((s & kFlagMask) == 0u) {
-                if (++iter > kSpinLimit) break;
-                __nanosleep(64);
-                s = ld_volatile(src);
-            }
-            if ((s & kFlagMask) == 0u) {  // gave up: record and stop waiting
-                atomicExch(error, 1u);
-                break;
-            }
-            prefix += s & kValueMask;
-            if (s & kFlagInc) break;
-            --j;
-        }
-        st_volatile(st + d, kFlagInc | (prefix + count));
-    }
-    s_gbase[d] = digit_offsets[d] + prefix;
-
-    // exclusive scan of the tile's digit counts -> start of each digit in the tile
-    uint32_t incl = count;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += u;
-    }
-    if (lane == 31) s_scan[warp] = incl;
-    __syncthreads();
-    uint32_t wpre = 0;
-    for (int w = 0; w < warp; ++w) wpre += s_scan[w];
-    s_tile_start[d] = wpre + incl - count;
-    __syncthreads();
-
-#pragma unroll
-    for (int i = 0; i < kSortItems; ++i) {
-        if (dg[i] < (uint32_t)kRadix) {
-            const uint32_t lp = s_tile_start[dg[i]] + wh[dg[i]] + rk[i];
-            s_keys[lp] = k[i];
-            s_vals[lp] = v[i];
-        }
-    }
-    __syncthreads();
-    const int64_t rem = n - base;
-    const int tile_n = rem < kSortTile ? (int)rem : kSortTile;
-    for (int j = tid; j < tile_n; j += kSortThreads) {
-        const uint64_t key = s_keys[j];
-        const uint32_t dd = (uint32_t)((key >> shift) & digit_mask);
-        const uint32_t pos = s_gbase[dd] + ((uint32_t)j - s_tile_start[dd]);
-        keys_out[pos] = key;
-        vals_out[pos] = s_vals[j];
-    }
+                                                                 int bits, const uint32_t* hist, uint32_t* status,
+                                                                 uint32_t* tile_counter, uint32_t* error) {
+    sort_pass<Key>(
+        [&](int64_t i, Key& k, uint32_t& v) {
+            k = keys_in[i];
+            v = vals_in[i];
+        },
+        [&](int64_t i, Key k, uint32_t v) {
+            keys_out[i] = k;
+            vals_out[i] = v;
+        },
+        n, shift, bits, hist, status, tile_counter, error);
 }
-
-constexpr size_t kSortSmem = sizeof(uint64_t) * kSortTile + sizeof(uint32_t) * kSortTile +
-                             sizeof(uint32_t) * (kSortWarps * kRadix + 2 * kRadix);
 
 size_t sort_workspace_bytes(int64_t n, int end_bit) {
     const int passes = (end_bit + 7) / 8;
@@ -408,12 +277,12 @@ int sort_pairs(int64_t* keys, int32_t* vals, int64_t* keys_alt, int32_t* vals_al
     const int hist_blocks = (int)std::min<int64_t>(n_tiles, (int64_t)kNumSMs * 4);
     sort_histogram_kernel<<<hist_blocks, kSortThreads, 0, s>>>(reinterpret_cast<const uint64_t*>(keys), n, passes,
                                                                end_bit, w.hist);
-    sort_digit_offsets_kernel<<<passes, kRadix, 0, s>>>(w.hist, w.digit_offsets);
-    note_launches(2);
+    note_launches(1);
     if ((cerr = cudaGetLastError()) != cudaSuccess) return TG_ERR_CUDA;
     // a per-device function attribute: set on every call (cheap, allowed during stream capture)
-    if ((cerr = cudaFuncSetAttribute(sort_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kSortSmem)) != cudaSuccess)
+    constexpr size_t smem = sort_pass_smem<uint64_t>();
+    if ((cerr = cudaFuncSetAttribute(sort_pass_kernel<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem)) != cudaSuccess)
         return TG_ERR_CUDA;
     uint64_t* kin = reinterpret_cast<uint64_t*>(keys);
     uint32_t* vin = reinterpret_cast<uint32_t*>(vals);
@@ -421,10 +290,8 @@ int sort_pairs(int64_t* keys, int32_t* vals, int64_t* keys_alt, int32_t* vals_al
     uint32_t* vout = reinterpret_cast<uint32_t*>(vals_alt);
     for (int p = 0; p < passes; ++p) {
         const int shift = 8 * p;
-        const int bits = std::min(8, end_bit - shift);
-        const uint32_t dmask = (1u << bits) - 1u;
-        sort_pass_kernel<<<(unsigned)n_tiles, kSortThreads, kSortSmem, s>>>(
-            kin, vin, kout, vout, n, shift, dmask, w.digit_offsets + p * kRadix,
+        sort_pass_kernel<uint64_t><<<(unsigned)n_tiles, kSortThreads, smem, s>>>(
+            kin, vin, kout, vout, n, shift, std::min(8, end_bit - shift), w.hist + p * kRadix,
             w.status + (size_t)p * n_tiles * kRadix, w.tile_counter + p, w.error);
         if ((cerr = cudaGetLastError()) != cudaSuccess) return TG_ERR_CUDA;
         note_launches(1);
@@ -451,15 +318,15 @@ int sort_lookback_selftest(int64_t* keys, int32_t* vals, int64_t* keys_alt, int3
     if ((cerr = cudaMemsetAsync(workspace, 0, w.bytes, s)) != cudaSuccess) return TG_ERR_CUDA;
     set_u32_kernel<<<1, 1, 0, s>>>(w.tile_counter, 1u);  // the single CTA takes tile 1
     sort_histogram_kernel<<<2, kSortThreads, 0, s>>>(reinterpret_cast<const uint64_t*>(keys), n, 1, 8, w.hist);
-    sort_digit_offsets_kernel<<<1, kRadix, 0, s>>>(w.hist, w.digit_offsets);
-    if ((cerr = cudaFuncSetAttribute(sort_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kSortSmem)) != cudaSuccess)
+    constexpr size_t smem = sort_pass_smem<uint64_t>();
+    if ((cerr = cudaFuncSetAttribute(sort_pass_kernel<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)smem)) != cudaSuccess)
         return TG_ERR_CUDA;
-    sort_pass_kernel<<<1, kSortThreads, kSortSmem, s>>>(
+    sort_pass_kernel<uint64_t><<<1, kSortThreads, smem, s>>>(
         reinterpret_cast<const uint64_t*>(keys), reinterpret_cast<const uint32_t*>(vals),
-        reinterpret_cast<uint64_t*>(keys_alt), reinterpret_cast<uint32_t*>(vals_alt), n, 0, 0xffu, w.digit_offsets,
-        w.status, w.tile_counter, w.error);
-    note_launches(4);
+        reinterpret_cast<uint64_t*>(keys_alt), reinterpret_cast<uint32_t*>(vals_alt), n, 0, 8, w.hist, w.status,
+        w.tile_counter, w.error);
+    note_launches(3);
     if ((cerr = cudaGetLastError()) != cudaSuccess) return TG_ERR_CUDA;
     uint32_t h = 0;
     if ((cerr = cudaStreamSynchronize(s)) != cudaSuccess) return TG_ERR_CUDA;
@@ -521,6 +388,522 @@ cudaError_t launch_offset_encode(const int64_t* keys, int64_t n, int C, int tw, 
     offset_encode_kernel<<<(unsigned)((n_ids + 255) / 256), 256, 0, s>>>(keys, n, n_ids, tw * th, tile_n_bits, mask,
                                                                        offsets);
     note_launches(1);
+    return cudaGetLastError();
+}
+
+// ------------------------------------------------------------------ sorted intersection lists
+constexpr int kOrderChunk = 1024;  // depth-ordered entries per emission CTA
+constexpr int kDepthPasses = 4;
+
+// Scratch of the entry stage.
+struct OrderWorkspace {
+    uint32_t* hist;     // [4][256] depth digits  (zeroed, with all up to `status` inclusive)
+    uint32_t* counter;  // [4] tiles taken, then the error flag
+    uint32_t* status;   // [4][tiles][256]
+    uint32_t *keys[2], *ids[2];  // ping-pong; the depth order ends in ids[1]
+    int64_t* chunks;    // [chunks + 1] intersections before each chunk of the depth order
+    size_t zeroed, bytes;
+};
+inline OrderWorkspace carve_order_workspace(void* base, int64_t E) {
+    OrderWorkspace w;
+    char* p = static_cast<char*>(base);
+    size_t off = 0;
+    auto take = [&](size_t n) {
+        char* q = p + off;
+        off += align256(n);
+        return q;
+    };
+    const int64_t tiles = E > kSmallSort ? (E + kSortTile - 1) / kSortTile : 0;  // the small sort needs no status
+    w.hist = reinterpret_cast<uint32_t*>(take(4 * kDepthPasses * kRadix));
+    w.counter = reinterpret_cast<uint32_t*>(take(4 * (kDepthPasses + 1)));
+    w.status = reinterpret_cast<uint32_t*>(take(4 * (size_t)kDepthPasses * tiles * kRadix));
+    w.zeroed = off;
+    for (int i = 0; i < 2; ++i) w.keys[i] = reinterpret_cast<uint32_t*>(take(4 * (size_t)(tiles ? E : 0)));
+    for (int i = 0; i < 2; ++i) w.ids[i] = reinterpret_cast<uint32_t*>(take(4 * (size_t)(tiles || i ? E : 0)));
+    w.chunks = reinterpret_cast<int64_t*>(take(8 * ((E + kOrderChunk - 1) / kOrderChunk + 1)));
+    w.bytes = off;
+    return w;
+}
+size_t isect_order_workspace_bytes(int64_t E) { return carve_order_workspace(nullptr, E).bytes; }
+
+// Adds one to s[d] for every lane with ok, one add per warp where all its digits agree (a depth's exponent digits).
+__device__ __forceinline__ void count_digit(uint32_t* s, uint32_t d, bool ok) {
+    const unsigned m = __ballot_sync(0xffffffffu, ok);
+    if (m == 0u) return;
+    const uint32_t d0 = __shfl_sync(0xffffffffu, d, __ffs(m) - 1);
+    if (__all_sync(0xffffffffu, !ok || d == d0)) {
+        if ((threadIdx.x & 31) == 0) atomicAdd(s + d0, (uint32_t)__popc(m));
+    } else if (ok) {
+        atomicAdd(s + d, 1u);
+    }
+}
+
+// Tile counts of the entries, and the digit counts of their depths.
+__global__ void __launch_bounds__(256) order_count_kernel(tg_isect_args a, uint32_t* hist) {
+    __shared__ uint32_t s_hist[kDepthPasses * kRadix];
+    if (hist != nullptr) {
+        for (int i = threadIdx.x; i < kDepthPasses * kRadix; i += 256) s_hist[i] = 0;
+        __syncthreads();
+    }
+    const int64_t first = (int64_t)blockIdx.x * kOrderChunk;
+#pragma unroll 1
+    for (int i = 0; i < kOrderChunk; i += 256) {
+        const int64_t e = first + i + threadIdx.x;
+        const bool in = e < a.n_elems;
+        if (in) {
+            int32_t cnt = 0;
+            const int32_t r = a.radii[e];
+            uint32_t tw, th;
+            if (r > 0 && camera_grid(a, e, tw, th)) {
+                const float2 m = reinterpret_cast<const float2*>(a.means2d)[e];
+                uint32_t x0, y0, x1, y1;
+                tile_box(m.x, m.y, r, a.tile_size, tw, th, x0, y0, x1, y1);
+                cnt = (int32_t)((y1 - y0) * (x1 - x0));
+            }
+            a.tiles_per_gauss[e] = cnt;
+        }
+        if (hist != nullptr) {
+            const uint32_t k = in ? __float_as_uint(a.depths[e]) : 0u;
+#pragma unroll
+            for (int p = 0; p < kDepthPasses; ++p) count_digit(s_hist + p * kRadix, (k >> (8 * p)) & 0xffu, in);
+        }
+    }
+    if (hist == nullptr) return;
+    __syncthreads();
+    for (int i = threadIdx.x; i < kDepthPasses * kRadix; i += 256)
+        if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
+}
+
+// Pass p of the entries' depth sort; the first reads the depths themselves.
+__global__ void __launch_bounds__(kSortThreads, 4) order_pass_kernel(const float* __restrict__ depths,
+                                                                  const uint32_t* __restrict__ keys_in,
+                                                                  const uint32_t* __restrict__ ids_in,
+                                                                  uint32_t* __restrict__ keys_out,
+                                                                  uint32_t* __restrict__ ids_out, int64_t n, int pass,
+                                                                  const uint32_t* hist, uint32_t* status,
+                                                                  uint32_t* counter, uint32_t* error) {
+    sort_pass<uint32_t>(
+        [&](int64_t i, uint32_t& k, uint32_t& v) {
+            k = pass == 0 ? __float_as_uint(depths[i]) : keys_in[i];
+            v = pass == 0 ? (uint32_t)i : ids_in[i];
+        },
+        [&](int64_t i, uint32_t k, uint32_t v) {
+            if (pass != kDepthPasses - 1) keys_out[i] = k;  // (only the order is kept of the last)
+            ids_out[i] = v;
+        },
+        n, 8 * pass, 8, hist, status, counter, error);
+}
+
+// The whole entry order by one CTA, for n <= kSmallSort.
+__global__ void __launch_bounds__(kSmallThreads) order_small_kernel(const float* __restrict__ depths, int n,
+                                                                    uint32_t* __restrict__ ids) {
+    uint32_t *s_keys, *s_idx;
+    sort_small([&](int i) { return __float_as_uint(depths[i]); }, n, 32, s_keys, s_idx);
+    for (int i = threadIdx.x; i < n; i += kSmallThreads) ids[i] = s_idx[i];
+}
+
+// Intersections of each chunk of the depth order.
+__global__ void __launch_bounds__(256) order_sums_kernel(const uint32_t* __restrict__ ids,
+                                                         const int32_t* __restrict__ counts, int64_t n,
+                                                         int64_t* chunks) {
+    __shared__ int64_t s_warp[kScanThreads / 32];
+    int64_t local = 0;
+#pragma unroll
+    for (int i = 0; i < kOrderChunk; i += 256) {
+        const int64_t k = (int64_t)blockIdx.x * kOrderChunk + i + threadIdx.x;
+        if (k < n) local += counts[ids[k]];
+    }
+    int64_t total;
+    block_excl_scan(local, s_warp, total);
+    if (threadIdx.x == 0) chunks[blockIdx.x] = total;
+}
+
+// Exclusive scan of the chunk sums by one CTA of 1024 threads, four sums each; the total goes to chunks[n_chunks]
+// and *n_total.
+__global__ void __launch_bounds__(1024) order_scan_kernel(int64_t* chunks, int64_t n_chunks, int64_t* n_total) {
+    __shared__ int64_t s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t carry = 0;
+    for (int64_t b = 0; b < n_chunks; b += 4096) {
+        const int64_t i0 = b + threadIdx.x * 4;
+        int64_t v[4], sum = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            v[k] = i0 + k < n_chunks ? chunks[i0 + k] : 0;
+            sum += v[k];
+        }
+        int64_t incl = warp_incl_scan(sum);
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        if (warp == 0) s_warp[lane] = warp_incl_scan(s_warp[lane]);
+        __syncthreads();
+        int64_t run = carry + incl - sum + (warp > 0 ? s_warp[warp - 1] : 0);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (i0 + k < n_chunks) chunks[i0 + k] = run;
+            run += v[k];
+        }
+        carry += s_warp[31];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        chunks[n_chunks] = carry;
+        *n_total = carry;
+    }
+}
+
+cudaError_t launch_isect_order(const tg_isect_args& a, void* workspace, cudaStream_t s) {
+    const int64_t E = a.n_elems;
+    if (E == 0) return cudaMemsetAsync(a.n_isects, 0, sizeof(int64_t), s);
+    const OrderWorkspace w = carve_order_workspace(workspace, E);
+    const int64_t chunks = (E + kOrderChunk - 1) / kOrderChunk;
+    const bool small = E <= kSmallSort;
+    cudaError_t e = cudaSuccess;
+    if (!small && (e = cudaMemsetAsync(workspace, 0, w.zeroed, s)) != cudaSuccess) return e;
+    order_count_kernel<<<(unsigned)chunks, 256, 0, s>>>(a, small ? nullptr : w.hist);
+    if (small) {
+        if ((e = cudaFuncSetAttribute(order_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kSmallSmem)) != cudaSuccess)
+            return e;
+        order_small_kernel<<<1, kSmallThreads, kSmallSmem, s>>>(a.depths, (int)E, w.ids[1]);
+        note_launches(2);
+    } else {
+        constexpr size_t smem = sort_pass_smem<uint32_t>();
+        if ((e = cudaFuncSetAttribute(order_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+            cudaSuccess)
+            return e;
+        const int64_t tiles = (E + kSortTile - 1) / kSortTile;
+        for (int p = 0; p < kDepthPasses; ++p)
+            order_pass_kernel<<<(unsigned)tiles, kSortThreads, smem, s>>>(
+                a.depths, w.keys[(p + 1) & 1], w.ids[(p + 1) & 1], w.keys[p & 1], w.ids[p & 1], E, p,
+                w.hist + p * kRadix, w.status + (size_t)p * tiles * kRadix, w.counter + p, w.counter + kDepthPasses);
+        note_launches(1 + kDepthPasses);
+    }
+    order_sums_kernel<<<(unsigned)chunks, 256, 0, s>>>(w.ids[1], a.tiles_per_gauss, E, w.chunks);
+    order_scan_kernel<<<1, 1024, 0, s>>>(w.chunks, chunks, a.n_isects);
+    note_launches(2);
+    return cudaGetLastError();
+}
+
+// Scratch of the list stage: pairs of (camera | tile) key and entry.
+struct ListWorkspace {
+    uint32_t* hist;     // [4][256]  (zeroed, with all up to `status` inclusive)
+    uint32_t* counter;  // [4] tiles taken, then the error flag
+    uint32_t* status;   // [passes][tiles][256]
+    uint32_t *keys[2], *ids[2];
+    size_t zeroed, bytes;
+};
+inline ListWorkspace carve_list_workspace(void* base, int64_t n, int passes) {
+    ListWorkspace w;
+    char* p = static_cast<char*>(base);
+    size_t off = 0;
+    auto take = [&](size_t k) {
+        char* q = p + off;
+        off += align256(k);
+        return q;
+    };
+    const int64_t tiles = (n + kSortTile - 1) / kSortTile;
+    w.hist = reinterpret_cast<uint32_t*>(take(4 * 4 * kRadix));
+    w.counter = reinterpret_cast<uint32_t*>(take(4 * 5));
+    w.status = reinterpret_cast<uint32_t*>(take(4 * (size_t)passes * tiles * kRadix));
+    w.zeroed = off;
+    for (int i = 0; i < 2; ++i) w.keys[i] = reinterpret_cast<uint32_t*>(take(4 * (size_t)n));
+    for (int i = 0; i < 2; ++i) w.ids[i] = reinterpret_cast<uint32_t*>(take(4 * (size_t)n));
+    w.bytes = off;
+    return w;
+}
+// Passes over `key_bits` bits, each of the same number of bits (fewer digits: longer runs to write).
+inline int list_passes(int key_bits) { return (key_bits + 7) / 8; }
+inline int list_pass_bits(int key_bits) { return (key_bits + list_passes(key_bits) - 1) / list_passes(key_bits); }
+size_t isect_lists_workspace_bytes(int64_t n, int key_bits) {
+    return carve_list_workspace(nullptr, n, list_passes(key_bits)).bytes;
+}
+
+// Writes the intersections in depth order and counts their keys' digits.  A CTA expands 1024 entries: their tile
+// boxes go to shared memory, and each thread fills four consecutive list places at a time (one search for the
+// first, then stepping), so that the writes are whole vectors whatever the entries' sizes.
+__global__ void __launch_bounds__(256) isect_expand_kernel(tg_isect_args a, const uint32_t* __restrict__ order,
+                                                           const int64_t* __restrict__ chunks, int64_t limit,
+                                                           int tile_bits, int passes, int pass_bits,
+                                                           uint32_t* __restrict__ keys, uint32_t* __restrict__ ids,
+                                                           uint32_t* hist) {
+    __shared__ uint32_t s_hist[4 * kRadix];
+    __shared__ uint32_t s_off[kOrderChunk + 1];  // places before each entry
+    __shared__ uint32_t s_id[kOrderChunk], s_first[kOrderChunk], s_width[kOrderChunk], s_row[kOrderChunk],
+        s_high[kOrderChunk];  // s_high: the key's camera bits, or all ones (a negative depth's sign extension)
+    __shared__ uint32_t s_warp[8];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < 4 * kRadix; i += 256) s_hist[i] = 0;
+    const int64_t first = (int64_t)blockIdx.x * kOrderChunk;
+    uint32_t cnt[4], sum = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {  // thread t owns entries 4t .. 4t+3 of the chunk
+        const int64_t k = first + tid * 4 + i;
+        const int slot = tid * 4 + i;
+        cnt[i] = 0;
+        if (k < a.n_elems) {
+            const uint32_t e = order[k];
+            const int32_t r = a.radii[e];
+            uint32_t tw, th;
+            if (r > 0 && camera_grid(a, e, tw, th)) {
+                const float2 m = reinterpret_cast<const float2*>(a.means2d)[e];
+                uint32_t x0, y0, x1, y1;
+                tile_box(m.x, m.y, r, a.tile_size, tw, th, x0, y0, x1, y1);
+                cnt[i] = (y1 - y0) * (x1 - x0);
+                const int64_t cid = a.camera_ids ? a.camera_ids[e] : (int64_t)e / a.N;
+                s_id[slot] = e;
+                s_first[slot] = y0 * tw + x0;
+                s_width[slot] = x1 - x0;
+                s_row[slot] = tw;
+                s_high[slot] = (__float_as_uint(a.depths[e]) >> 31) ? 0xffffffffu : (uint32_t)(cid << tile_bits);
+            }
+        }
+        sum += cnt[i];
+    }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t run = incl - sum;
+    for (int w = 0; w < warp; ++w) run += s_warp[w];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        s_off[tid * 4 + i] = run;
+        run += cnt[i];
+    }
+    if (tid == 255) s_off[kOrderChunk] = run;
+    __syncthreads();
+    const int64_t base = chunks[blockIdx.x];
+    const int64_t end = min(base + (int64_t)s_off[kOrderChunk], limit);
+    const uint32_t digit_mask = (1u << pass_bits) - 1u;
+    for (int64_t p4 = (base >> 2) + tid; p4 * 4 < end; p4 += 256) {  // four places from 4 * p4 on
+        const int64_t lo = max(p4 * 4, base), hi = min(p4 * 4 + 4, end);
+        uint32_t rel = (uint32_t)(lo - base);
+        int slot = 0;  // last entry whose places start at or before rel
+#pragma unroll
+        for (int step = kOrderChunk / 2; step > 0; step >>= 1)
+            if (s_off[slot + step] <= rel) slot += step;
+        uint32_t k = rel - s_off[slot];
+        uint32_t y = k / s_width[slot], x = k - y * s_width[slot];
+        uint32_t key[4], id[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int64_t pos = p4 * 4 + q;
+            if (pos < lo || pos >= hi) continue;
+            key[q] = s_high[slot] | (s_first[slot] + y * s_row[slot] + x);
+            id[q] = s_id[slot];
+            for (int p = 0; p < passes; ++p)
+                atomicAdd(&s_hist[p * kRadix + ((key[q] >> (p * pass_bits)) & digit_mask)], 1u);
+            ++rel;
+            if (++x == s_width[slot]) {
+                x = 0;
+                ++y;
+            }
+            if (pos + 1 < hi && rel == s_off[slot + 1]) {
+                do ++slot; while (slot + 1 < kOrderChunk && s_off[slot + 1] == rel);  // (entries without places)
+                x = y = 0;
+            }
+        }
+        if (hi - lo == 4) {
+            reinterpret_cast<uint4*>(keys)[p4] = make_uint4(key[0], key[1], key[2], key[3]);
+            reinterpret_cast<uint4*>(ids)[p4] = make_uint4(id[0], id[1], id[2], id[3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int64_t pos = p4 * 4 + q;
+                if (pos >= lo && pos < hi) {
+                    keys[pos] = key[q];
+                    ids[pos] = id[q];
+                }
+            }
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < passes * kRadix; i += 256)
+        if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
+    if (a.overflow && tid == 0 && base + (int64_t)s_off[kOrderChunk] > limit) atomicOr(a.overflow, 1u);
+}
+
+// Capacity mode: the places past the valid count get the largest key (they sort last) and no entry.
+__global__ void __launch_bounds__(256) isect_expand_pad_kernel(const int64_t* n_dev, int64_t capacity, uint32_t pad_key,
+                                                               int passes, int pass_bits, uint32_t* keys, uint32_t* ids,
+                                                               uint32_t* hist) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n = min(max(*n_dev, (int64_t)0), capacity);
+    if (i == 0 && n < capacity)
+        for (int p = 0; p < passes; ++p)
+            atomicAdd(&hist[p * kRadix + ((pad_key >> (p * pass_bits)) & ((1u << pass_bits) - 1u))],
+                      (uint32_t)(capacity - n));
+    if (i < n || i >= capacity) return;
+    keys[i] = pad_key;
+    ids[i] = 0xffffffffu;
+}
+
+// One pass over the (camera, tile) keys; the last writes the 64-bit keys and the entries.
+template <bool kLast>
+__global__ void __launch_bounds__(kSortThreads, 4) list_pass_kernel(const uint32_t* __restrict__ keys_in,
+                                                                 const uint32_t* __restrict__ ids_in,
+                                                                 uint32_t* __restrict__ keys_out,
+                                                                 uint32_t* __restrict__ ids_out,
+                                                                 const float* __restrict__ depths,
+                                                                 int64_t* __restrict__ isect_ids,
+                                                                 int32_t* __restrict__ flatten_ids, int64_t n,
+                                                                 int shift, int bits, const uint32_t* hist,
+                                                                 uint32_t* status, uint32_t* counter, uint32_t* error) {
+    sort_pass<uint32_t>(
+        [&](int64_t i, uint32_t& k, uint32_t& v) {
+            k = keys_in[i];
+            v = ids_in[i];
+        },
+        [&](int64_t i, uint32_t k, uint32_t v) {
+            if constexpr (kLast) {
+                const bool pad = v == 0xffffffffu;
+                const uint32_t low = pad ? 0xffffffffu : __float_as_uint(__ldg(depths + v));
+                isect_ids[i] = (int64_t)(((uint64_t)k << 32) | low);
+                flatten_ids[i] = pad ? 0 : (int32_t)v;
+            } else {
+                keys_out[i] = k;
+                ids_out[i] = v;
+            }
+        },
+        n, shift, bits, hist, status, counter, error);
+}
+
+cudaError_t launch_isect_lists(const tg_isect_args& a, void* order_ws, int64_t n, int tile_bits, int key_bits, void* ws,
+                               cudaStream_t s) {
+    const int64_t E = a.n_elems;
+    if (n == 0) return cudaSuccess;
+    const int passes = list_passes(key_bits), pass_bits = list_pass_bits(key_bits);
+    const OrderWorkspace o = carve_order_workspace(order_ws, E);
+    const ListWorkspace w = carve_list_workspace(ws, n, passes);
+    cudaError_t e = cudaMemsetAsync(ws, 0, w.zeroed, s);
+    if (e != cudaSuccess) return e;
+    if (E > 0) {
+        isect_expand_kernel<<<(unsigned)((E + kOrderChunk - 1) / kOrderChunk), 256, 0, s>>>(
+            a, o.ids[1], o.chunks, n, tile_bits, passes, pass_bits, w.keys[0], w.ids[0], w.hist);
+        note_launches(1);
+    }
+    if (a.overflow) {
+        const uint32_t pad = key_bits >= 32 ? 0xffffffffu : (1u << key_bits) - 1u;
+        isect_expand_pad_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a.n_isects, n, pad, passes, pass_bits,
+                                                                           w.keys[0], w.ids[0], w.hist);
+        note_launches(1);
+    }
+    constexpr size_t smem = sort_pass_smem<uint32_t>();
+    if ((e = cudaFuncSetAttribute(list_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+            cudaSuccess ||
+        (e = cudaFuncSetAttribute(list_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+            cudaSuccess)
+        return e;
+    const int64_t tiles = (n + kSortTile - 1) / kSortTile;
+    for (int p = 0; p < passes; ++p) {
+        const int shift = p * pass_bits, bits = std::min(pass_bits, key_bits - shift);
+        const auto fn = p == passes - 1 ? list_pass_kernel<true> : list_pass_kernel<false>;
+        fn<<<(unsigned)tiles, kSortThreads, smem, s>>>(w.keys[p & 1], w.ids[p & 1], w.keys[(p + 1) & 1],
+                                                       w.ids[(p + 1) & 1], a.depths, a.isect_ids, a.flatten_ids, n,
+                                                       shift, bits, w.hist + p * kRadix,
+                                                       w.status + (size_t)p * tiles * kRadix, w.counter + p,
+                                                       w.counter + 4);
+    }
+    note_launches(passes);
+    return cudaGetLastError();
+}
+
+// ------------------------------------------------------------------ tile order
+// Tiles by descending list length (stable): keys bound - length, bound >= every length.
+__device__ __forceinline__ uint32_t tile_key(const int32_t* __restrict__ offsets, int64_t t, int64_t n_tiles,
+                                             int64_t n_isects, const int64_t* n_dev, uint32_t bound) {
+    const int64_t end = t + 1 < n_tiles ? (int64_t)offsets[t + 1] : (n_dev ? *n_dev : n_isects);
+    const int64_t c = end - (int64_t)offsets[t];
+    return bound - (uint32_t)min(max(c, (int64_t)0), (int64_t)bound);
+}
+
+__global__ void __launch_bounds__(kSmallThreads) tile_order_small_kernel(const int32_t* offsets, int n_tiles,
+                                                                         int64_t n_isects, const int64_t* n_dev,
+                                                                         uint32_t bound, int end_bit, int32_t* order) {
+    uint32_t *s_keys, *s_idx;
+    sort_small([&](int i) { return tile_key(offsets, i, n_tiles, n_isects, n_dev, bound); }, n_tiles, end_bit, s_keys,
+               s_idx);
+    for (int i = threadIdx.x; i < n_tiles; i += kSmallThreads) order[i] = (int32_t)s_idx[i];
+}
+
+__global__ void __launch_bounds__(256) tile_order_count_kernel(const int32_t* offsets, int64_t n_tiles,
+                                                               int64_t n_isects, const int64_t* n_dev, uint32_t bound,
+                                                               int passes, uint32_t* hist) {
+    __shared__ uint32_t s_hist[4 * kRadix];
+    for (int i = threadIdx.x; i < 4 * kRadix; i += 256) s_hist[i] = 0;
+    __syncthreads();
+    const int64_t stride = (int64_t)gridDim.x * 256;
+    for (int64_t b = (int64_t)blockIdx.x * 256; b < n_tiles; b += stride) {  // uniform over the CTA
+        const int64_t t = b + threadIdx.x;
+        const bool in = t < n_tiles;
+        const uint32_t k = in ? tile_key(offsets, t, n_tiles, n_isects, n_dev, bound) : 0u;
+        for (int p = 0; p < passes; ++p) count_digit(s_hist + p * kRadix, (k >> (8 * p)) & 0xffu, in);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < passes * kRadix; i += 256)
+        if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
+}
+
+__global__ void __launch_bounds__(kSortThreads, 4) tile_order_pass_kernel(
+    const int32_t* __restrict__ offsets, int64_t n_isects, const int64_t* n_dev, uint32_t bound,
+    const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ ids_in, uint32_t* __restrict__ keys_out,
+    uint32_t* __restrict__ ids_out, int64_t n, int pass, int bits, const uint32_t* hist, uint32_t* status,
+    uint32_t* counter, uint32_t* error) {
+    sort_pass<uint32_t>(
+        [&](int64_t i, uint32_t& k, uint32_t& v) {
+            k = pass == 0 ? tile_key(offsets, i, n, n_isects, n_dev, bound) : keys_in[i];
+            v = pass == 0 ? (uint32_t)i : ids_in[i];
+        },
+        [&](int64_t i, uint32_t k, uint32_t v) {
+            keys_out[i] = k;
+            ids_out[i] = v;
+        },
+        n, 8 * pass, bits, hist, status, counter, error);
+}
+
+// Above kSmallSort tiles: the list stage's scratch serves (its pairs are of the same kind).
+size_t tile_order_workspace_bytes(int64_t n_tiles) {
+    return n_tiles <= kSmallSort ? 256 : carve_list_workspace(nullptr, n_tiles, 4).bytes;
+}
+
+cudaError_t launch_tile_order(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, const int64_t* n_dev,
+                              int32_t* order, void* ws, cudaStream_t s) {
+    if (n_tiles == 0) return cudaSuccess;
+    const uint32_t bound = (uint32_t)std::min<int64_t>(std::max<int64_t>(n_isects, 1), 0x7fffffff);
+    int end_bit = 0;
+    for (uint32_t b = bound; b; b >>= 1) ++end_bit;
+    cudaError_t e;
+    if (n_tiles <= kSmallSort) {
+        if ((e = cudaFuncSetAttribute(tile_order_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kSmallSmem)) != cudaSuccess)
+            return e;
+        tile_order_small_kernel<<<1, kSmallThreads, kSmallSmem, s>>>(offsets, (int)n_tiles, n_isects, n_dev, bound,
+                                                                     end_bit, order);
+        note_launches(1);
+        return cudaGetLastError();
+    }
+    const int passes = (end_bit + 7) / 8;
+    const ListWorkspace w = carve_list_workspace(ws, n_tiles, 4);
+    if ((e = cudaMemsetAsync(ws, 0, w.zeroed, s)) != cudaSuccess) return e;
+    const int64_t tiles = (n_tiles + kSortTile - 1) / kSortTile;
+    tile_order_count_kernel<<<(unsigned)std::min<int64_t>((n_tiles + 1023) / 1024, kNumSMs * 4), 256, 0, s>>>(
+        offsets, n_tiles, n_isects, n_dev, bound, passes, w.hist);
+    constexpr size_t smem = sort_pass_smem<uint32_t>();
+    if ((e = cudaFuncSetAttribute(tile_order_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+        cudaSuccess)
+        return e;
+    for (int p = 0; p < passes; ++p) {
+        uint32_t* out = p == passes - 1 ? reinterpret_cast<uint32_t*>(order) : w.ids[(p + 1) & 1];
+        tile_order_pass_kernel<<<(unsigned)tiles, kSortThreads, smem, s>>>(
+            offsets, n_isects, n_dev, bound, w.keys[p & 1], w.ids[p & 1], w.keys[(p + 1) & 1], out, n_tiles, p,
+            std::min(8, end_bit - 8 * p), w.hist + p * kRadix, w.status + (size_t)p * tiles * kRadix, w.counter + p,
+            w.counter + 4);
+    }
+    note_launches(1 + passes);
     return cudaGetLastError();
 }
 

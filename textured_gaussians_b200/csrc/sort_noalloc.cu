@@ -6,13 +6,13 @@
 // real-time loop that must not call cudaMalloc (which may synchronise the
 // device) or a host without a caching allocator that cannot afford a
 // cudaMalloc/cudaFree pair per call.  For them this entry point keeps the
-// sort's scratch (digit histograms, digit offsets, tile counters, the
+// sort's scratch (digit histograms, tile counters, the
 // look-back status words and the wait-timeout flag) in a file-scope static
 // device array of fixed size, so the caller passes only the keys, values and
 // their ping-pong buffers.
 //
 // Costs and limits:
-//  * every GPU that loads this library holds kNoAllocScratchBytes (8 MiB + 16 KiB)
+//  * every GPU that loads this library holds kNoAllocScratchBytes (8 MiB + 8.5 KiB)
 //    of device memory for this array until the process exits;
 //  * at most kNoAllocMaxPairs (4,194,304) pairs per call; larger sizes are
 //    rejected with TG_ERR_INVALID_ARG before anything is launched;
@@ -51,10 +51,10 @@ namespace {
 constexpr int64_t kNoAllocMaxPairs = int64_t(1) << 22;
 constexpr size_t kAlign = 256;
 constexpr size_t al(size_t x) { return (x + kAlign - 1) & ~(kAlign - 1); }
-// Same layout the sort carves from any workspace: histograms and digit
-// offsets for 8 passes, 8 tile counters, an error flag, then one status word
-// per (pass, 4096-key tile, digit).
-constexpr size_t kNoAllocScratchBytes = al(4 * 8 * 256) + al(4 * 8 * 256) + al(4 * 8) + al(4) +
+// Same layout the sort carves from any workspace: histograms for 8 passes, 8
+// tile counters, an error flag, then one status word per (pass, 4096-key tile,
+// digit).
+constexpr size_t kNoAllocScratchBytes = al(4 * 8 * 256) + al(4 * 8) + al(4) +
                                         al(size_t(4) * 8 * (kNoAllocMaxPairs / 4096) * 256);
 
 static __device__ __align__(256) unsigned char g_sort_scratch[kNoAllocScratchBytes];

@@ -406,39 +406,47 @@ def isect_tiles(
     radii = radii.int().contiguous()
     depths = depths.float().contiguous()
     tiles_per_gauss = torch.empty(radii.shape, dtype=torch.int32, device=dev)
-    cum = torch.empty((max(E, 1),), dtype=torch.int64, device=dev)
     n_dev = torch.empty((1,), dtype=torch.int64, device=dev)
-    ws = torch.empty((B.lib().tg_scan_workspace_bytes(E),), dtype=torch.uint8, device=dev)
+    key_bits = _bit_width(tile_width * tile_height) + _bit_width(C)
+    # sorted lists go by depth order first, then camera and tile; the unsorted ones (and sizes beyond the former's
+    # 2^30 entries) are written in entry order from a prefix sum over the entries
+    by_depth = sort and E < 1 << 30
+    cum = None if by_depth else torch.empty((max(E, 1),), dtype=torch.int64, device=dev)
+    L = B.lib()
+    ws = torch.empty((L.tg_isect_sorted_order_bytes(E) if by_depth else L.tg_scan_workspace_bytes(E),),
+                     dtype=torch.uint8, device=dev)
     a = B.IsectArgs(E, N, B.ptr(cam), B.ptr(means2d), B.ptr(radii), B.ptr(depths), int(tile_size), int(tile_width),
                     int(tile_height), int(C), B.ptr(tiles_per_gauss), B.ptr(cum), B.ptr(n_dev), B.ptr(ws), None, None,
                     None if view_table is None else B.ptr(view_table.views))
     stream = B.stream_of(means2d)
-    B.call("tg_isect_count", stream, B.lib().tg_isect_count, ctypes.byref(a), stream)
-    end_bit = 32 + _bit_width(tile_width * tile_height) + _bit_width(C)
+    if by_depth:
+        B.call("tg_isect_sorted_count", stream, L.tg_isect_sorted_count, ctypes.byref(a), B.ptr(ws), ws.numel(), stream)
+    else:
+        B.call("tg_isect_count", stream, L.tg_isect_count, ctypes.byref(a), stream)
     plan = active_plan()
-    if plan is not None and plan.mode == "capture":
-        # no host read: capacity-sized keys (tail padded to sort last), device count attached to flatten_ids
-        cap = plan.next_capacity()
-        isect_ids = torch.empty((cap,), dtype=torch.int64, device=dev)
-        flatten_ids = torch.empty((cap,), dtype=torch.int32, device=dev)
-        a.isect_ids, a.flatten_ids = B.ptr(isect_ids), B.ptr(flatten_ids)
-        a.capacity, a.overflow = cap, B.ptr(plan.new_flag(dev))
-        B.call("tg_isect_emit", stream, B.lib().tg_isect_emit, ctypes.byref(a), stream)
-        if sort:
-            isect_ids, flatten_ids = sort_pairs(isect_ids, flatten_ids, end_bit)
-        flatten_ids._tg_n_isects = n_dev
-        return tiles_per_gauss, isect_ids, flatten_ids
-    n_isects = int(n_dev.item())  # the one host synchronisation, as in the reference
-    if plan is not None:
-        plan.sizes.append(n_isects)
+    capture = plan is not None and plan.mode == "capture"
+    if capture:  # no host read: capacity-sized keys (tail padded to sort last), device count attached to flatten_ids
+        n_isects = plan.next_capacity()
+        a.capacity, a.overflow = n_isects, B.ptr(plan.new_flag(dev))
+    else:
+        n_isects = int(n_dev.item())  # the one host synchronisation, as in the reference
+        if plan is not None:
+            plan.sizes.append(n_isects)
     isect_ids = torch.empty((n_isects,), dtype=torch.int64, device=dev)
     flatten_ids = torch.empty((n_isects,), dtype=torch.int32, device=dev)
     if n_isects:
-        a.isect_ids = B.ptr(isect_ids)
-        a.flatten_ids = B.ptr(flatten_ids)
-        B.call("tg_isect_emit", stream, B.lib().tg_isect_emit, ctypes.byref(a), stream)
-        if sort:
-            isect_ids, flatten_ids = sort_pairs(isect_ids, flatten_ids, end_bit)
+        a.isect_ids, a.flatten_ids = B.ptr(isect_ids), B.ptr(flatten_ids)
+        if by_depth:
+            wsb = L.tg_isect_sorted_lists_bytes(n_isects, key_bits)
+            list_ws = torch.empty((wsb,), dtype=torch.uint8, device=dev)
+            B.call("tg_isect_sorted_lists", stream, L.tg_isect_sorted_lists, ctypes.byref(a), B.ptr(ws), n_isects,
+                   B.ptr(list_ws), wsb, stream)
+        else:
+            B.call("tg_isect_emit", stream, L.tg_isect_emit, ctypes.byref(a), stream)
+            if sort:
+                isect_ids, flatten_ids = sort_pairs(isect_ids, flatten_ids, 32 + key_bits)
+    if capture:
+        flatten_ids._tg_n_isects = n_dev
     return tiles_per_gauss, isect_ids, flatten_ids
 
 
@@ -498,16 +506,18 @@ def isect_offset_encode_views(isect_ids: Tensor, view_table) -> Tensor:
 def tile_order_heaviest_first(isect_offsets: Tensor, n_isects: int) -> Tensor:
     """Permutation of the flat tiles by descending intersection count (stable),
     so the longest tiles start first and the tail of the launch is short."""
-    flat = isect_offsets.reshape(-1).to(torch.int64)
+    flat = isect_offsets.reshape(-1).to(torch.int32).contiguous()
     n = flat.numel()
+    order = torch.empty((n,), dtype=torch.int32, device=flat.device)
     if isinstance(n_isects, Tensor):  # device count (graph capture)
-        tail = n_isects.reshape(1).to(torch.int64)
+        n_dev, bound = n_isects.reshape(1).to(torch.int64), (1 << 31) - 1
     else:
-        tail = torch.full((1,), int(n_isects), dtype=torch.int64, device=flat.device)
-    counts = torch.diff(flat, append=tail)
-    keys = ((1 << 31) - 1) - counts.clamp(0, (1 << 31) - 1)
-    vals = torch.arange(n, dtype=torch.int32, device=flat.device)
-    _, order = sort_pairs(keys.contiguous(), vals, 31)
+        n_dev, bound = None, int(n_isects)
+    L = B.lib()
+    wsb = L.tg_tile_order_workspace_bytes(n)
+    ws = torch.empty((wsb,), dtype=torch.uint8, device=flat.device)
+    st = B.stream_of(flat)
+    B.call("tg_tile_order", st, L.tg_tile_order, B.ptr(flat), n, bound, B.ptr(n_dev), B.ptr(order), B.ptr(ws), wsb, st)
     return order
 
 
