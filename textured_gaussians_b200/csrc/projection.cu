@@ -183,13 +183,14 @@ __device__ __forceinline__ f3 camera_centre(const float* __restrict__ vm) {
 
 // Fused SH colour of Gaussian n seen from camera c: max(SH + 0.5, 0) for a
 // visible entry, 0.5 (the value the unfused path gives a masked entry) otherwise.
+// row: the Gaussian's coefficients.
+template <int NB>
 __device__ __forceinline__ f3 fused_sh_color(const float* __restrict__ means, const float* __restrict__ viewmats,
-                                             int degree, int K, const float* __restrict__ coeffs, int c, int64_t n,
-                                             bool visible) {
+                                             const float* row, int c, int64_t n, bool visible) {
     if (!visible) return mk3(0.5f, 0.5f, 0.5f);
     const f3 o = camera_centre(viewmats + 16 * c);
     const f3 d = mk3(means[3 * n] - o.x, means[3 * n + 1] - o.y, means[3 * n + 2] - o.z);
-    const f3 col = sh_color(degree, d, coeffs + n * K * 3);
+    const f3 col = sh_color<NB>(d, row);
     return mk3(fmaxf(col.x + 0.5f, 0.f), fmaxf(col.y + 0.5f, 0.f), fmaxf(col.z + 0.5f, 0.f));
 }
 
@@ -206,39 +207,95 @@ __device__ __forceinline__ void store3(float* dst, int64_t i, f3 v) {
 // centre being a constant).
 template <int NB>
 __device__ __forceinline__ f3 fused_sh_vjp(const float* __restrict__ means, const float* __restrict__ viewmats,
-                                           int K, const float* __restrict__ coeffs, int c, int64_t n, f3 g,
-                                           float* acc) {
+                                           const float* crow, int c, int64_t n, f3 g, float* acc) {
     constexpr int degree = NB == 1 ? 0 : NB == 4 ? 1 : NB == 9 ? 2 : NB == 16 ? 3 : 4;
     const f3 o = camera_centre(viewmats + 16 * c);
     const f3 d = mk3(means[3 * n] - o.x, means[3 * n + 1] - o.y, means[3 * n + 2] - o.z);
-    const float* crow = coeffs + n * K * 3;
-    const f3 col = sh_color(degree, d, crow);
+    const f3 col = sh_color<NB>(d, crow);
     g.x = col.x + 0.5f >= 0.f ? g.x : 0.f;
     g.y = col.y + 0.5f >= 0.f ? g.y : 0.f;
     g.z = col.z + 0.5f >= 0.f ? g.z : 0.f;
     return sh_color_vjp<NB>(degree, d, crow, g, acc);
 }
 
-__global__ void __launch_bounds__(256) project_fwd_kernel(tg_project_fwd_args a) {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t total = (int64_t)a.C * a.N;
-    if (idx >= total) return;
-    const int c = (int)(idx / a.N);
-    const int64_t n = idx - (int64_t)c * a.N;
-    Projected o;
-    const bool vis = project_one(a.means, a.quats, a.scales, a.viewmats, a.Ks, a.width, a.height, a.near_plane,
-                                 a.far_plane, a.radius_clip, c, n, o);
-    if (!vis) {
-        o.radius = 0;
-        o.m2d = make_float2(0.f, 0.f);
-        o.depth = 0.f;
-#pragma unroll
-        for (int k = 0; k < 9; ++k) o.M[k] = 0.f;
-        o.nrm = mk3(0, 0, 0);
+// ------------------------------------------------------------------ warp staging
+// Rows of 9 and 3 floats per entry written one thread per row, and SH rows of up to 300 bytes read so, touch a
+// sector per lane and instruction (1M splats, 4 cameras, SH degree 3: forward 525 us at 0.9 TB/s; 196 us staged).
+// So a warp moves the rows of its 32 entries, contiguous in memory, through shared memory with whole-line accesses;
+// the odd row lengths keep the row-wise side free of bank conflicts.
+// Warps per CTA: four, two where degree 4's rows would pass 48 KB of shared memory.
+template <int NB>
+constexpr int kProjWarps = NB == 25 ? 2 : 4;
+
+// Copies n floats from a warp's shared memory to global memory, in vectors where the address allows.
+__device__ __forceinline__ void warp_store(float* __restrict__ g, const float* s, int n) {
+    const int lane = threadIdx.x & 31;
+    if ((n & 3) == 0 && (reinterpret_cast<uintptr_t>(g) & 15) == 0) {
+        for (int i = lane; i < n / 4; i += 32) reinterpret_cast<float4*>(g)[i] = reinterpret_cast<const float4*>(s)[i];
+    } else {
+        for (int i = lane; i < n; i += 32) g[i] = s[i];
     }
-    store_projected(o, idx, a.radii, a.means2d, a.depths, a.ray_transforms, a.normals);
-    if (a.sh_coeffs)
-        store3(a.colors, idx, fused_sh_color(a.means, a.viewmats, a.sh_degree, a.sh_K, a.sh_coeffs, c, n, vis));
+}
+// The SH rows of `cnt` Gaussians from n0 on (3 NB of their 3 K floats), at an odd pitch.
+template <int NB>
+struct ShRows {
+    static constexpr int kRow = 3 * NB, kPitch = kRow | 1;
+    static constexpr int kFloats = NB > 0 ? ((32 * kPitch + 3) & ~3) : 0;
+    __device__ __forceinline__ static void load(float* s, const float* __restrict__ coeffs, int64_t n0, int cnt, int K) {
+        const float* g = coeffs + n0 * K * 3;
+        for (int i = threadIdx.x & 31; i < cnt * kRow; i += 32) {
+            const int r = i / kRow;
+            s[r * kPitch + (i - r * kRow)] = g[(int64_t)r * K * 3 + (i - r * kRow)];
+        }
+    }
+};
+
+// NB: SH bases of the fused SH colours ((degree+1)^2; 0 = none).  Each warp projects 32 Gaussians into cameras
+// blockIdx.y, blockIdx.y + gridDim.y, ...
+template <int NB>
+__global__ void __launch_bounds__(32 * kProjWarps<NB>, 6) project_fwd_kernel(tg_project_fwd_args a) {
+    constexpr int kOut = 32 * 9 + 32 * 3 + (NB > 0 ? 32 * 3 : 0);
+    __shared__ float4 s_all[kProjWarps<NB> * (kOut + ShRows<NB>::kFloats) / 4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float* s_m = reinterpret_cast<float*>(s_all) + warp * (kOut + ShRows<NB>::kFloats);
+    float *s_n = s_m + 32 * 9, *s_c = s_n + 32 * 3, *s_sh = s_m + kOut;
+    const int64_t n0 = ((int64_t)blockIdx.x * kProjWarps<NB> + warp) * 32, n = n0 + lane;
+    const int cnt = (int)min((int64_t)32, a.N - n0);
+    if (cnt <= 0) return;  // (whole warps; only warp-level synchronisation below)
+    if constexpr (NB > 0) {
+        ShRows<NB>::load(s_sh, a.sh_coeffs, n0, cnt, a.sh_K);
+        __syncwarp();
+    }
+    for (int c = blockIdx.y; c < a.C; c += gridDim.y) {
+        const int64_t i0 = (int64_t)c * a.N + n0;
+        if (lane < cnt) {
+            Projected o;
+            const bool vis = project_one(a.means, a.quats, a.scales, a.viewmats, a.Ks, a.width, a.height, a.near_plane,
+                                         a.far_plane, a.radius_clip, c, n, o);
+            if (!vis) {
+                o.radius = 0;
+                o.m2d = make_float2(0.f, 0.f);
+                o.depth = 0.f;
+#pragma unroll
+                for (int k = 0; k < 9; ++k) o.M[k] = 0.f;
+                o.nrm = mk3(0, 0, 0);
+            }
+            a.radii[i0 + lane] = o.radius;
+            reinterpret_cast<float2*>(a.means2d)[i0 + lane] = o.m2d;
+            a.depths[i0 + lane] = o.depth;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) s_m[lane * 9 + k] = o.M[k];
+            store3(s_n, lane, o.nrm);
+            if constexpr (NB > 0)
+                store3(s_c, lane,
+                       fused_sh_color<NB>(a.means, a.viewmats, s_sh + lane * ShRows<NB>::kPitch, c, n, vis));
+        }
+        __syncwarp();
+        warp_store(a.ray_transforms + 9 * i0, s_m, 9 * cnt);
+        warp_store(a.normals + 3 * i0, s_n, 3 * cnt);
+        if constexpr (NB > 0) warp_store(a.colors + 3 * i0, s_c, 3 * cnt);
+        __syncwarp();  // read before the next camera's rows replace them
+    }
 }
 
 // ------------------------------------------------------------------ packed forward
@@ -300,6 +357,7 @@ __global__ void packed_indptr_kernel(const int64_t* chunk_offsets, const int64_t
 // Pass 2: recompute, rank the visible entries of each 256-entry slice with a
 // warp ballot plus a CTA prefix over warps, and write them at chunk offset +
 // rank, so entries keep (camera, Gaussian) order.
+template <int NB>
 __global__ void __launch_bounds__(kPackThreads) project_packed_emit_kernel(tg_project_packed_args a,
                                                                           const int64_t* chunk_offsets) {
     __shared__ int32_t s_warp[kPackThreads / 32];
@@ -334,9 +392,9 @@ __global__ void __launch_bounds__(kPackThreads) project_packed_emit_kernel(tg_pr
                 a.camera_ids[pos] = c;
                 a.gaussian_ids[pos] = n;
                 store_projected(o, pos, a.radii, a.means2d, a.depths, a.ray_transforms, a.normals);
-                if (a.sh_coeffs)
+                if constexpr (NB > 0)
                     store3(a.colors, pos,
-                           fused_sh_color(a.means, a.viewmats, a.sh_degree, a.sh_K, a.sh_coeffs, c, n, true));
+                           fused_sh_color<NB>(a.means, a.viewmats, a.sh_coeffs + n * a.sh_K * 3, c, n, true));
             } else if (a.overflow) {
                 atomicOr(a.overflow, 1u);
             }
@@ -455,53 +513,72 @@ __device__ __forceinline__ EntryGrad project_entry_vjp(const float* __restrict__
 }
 
 // NB: SH bases of the fused SH adjoint ((degree+1)^2; 0 = no fused SH), which
-// sizes the per-thread coefficient-gradient accumulator.
+// sizes the per-thread coefficient-gradient accumulator.  The upstream rows are read one thread per row: each
+// thread has all of a camera's loads in flight at once and their sectors meet again in L1 (staged through shared
+// memory like the forward's stores, load then compute, degree 0 took 312 us instead of 125 for 1M splats, 4 cameras).
+// The SH rows, 192 bytes at degree 3, are staged: 802 -> 389 us.  Resident CTAs: the register allocation that goes with
+// eight (degrees 0 and 1) and four (2 and 3) measured best of 5-8 and 2-5.
 template <int NB>
-__global__ void __launch_bounds__(256) project_bwd_kernel(tg_project_bwd_args a) {
+__global__ void __launch_bounds__(32 * kProjWarps<NB>, NB <= 4 ? 8 : NB <= 16 ? 4 : 1) project_bwd_kernel(tg_project_bwd_args a) {
     constexpr bool kSH = NB > 0;
-    const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= a.N) return;
+    constexpr bool kStage = NB > 1;  // (degree 0's rows are as short as the others)
+    __shared__ float s_all[kStage ? kProjWarps<NB> * ShRows<NB>::kFloats : 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float* s_sh = s_all + warp * ShRows<NB>::kFloats;
+    const int64_t n0 = ((int64_t)blockIdx.x * kProjWarps<NB> + warp) * 32, n = n0 + lane;
+    const int cnt = (int)min((int64_t)32, a.N - n0);
+    if (cnt <= 0) return;  // (whole warps; only warp-level synchronisation below)
     float acc[kSH ? 3 * NB : 1];  // SH coefficient gradient, summed over cameras in registers
-    if constexpr (kSH) {
 #pragma unroll
-        for (int k = 0; k < 3 * NB; ++k) acc[k] = 0.f;
+    for (int k = 0; k < (kSH ? 3 * NB : 1); ++k) acc[k] = 0.f;
+    if constexpr (kStage) {
+        ShRows<NB>::load(s_sh, a.sh_coeffs, n0, cnt, a.sh_K);
+        __syncwarp();
     }
-    const f3 p = mk3(a.means[3 * n], a.means[3 * n + 1], a.means[3 * n + 2]);
-    const float4 q = __ldg(reinterpret_cast<const float4*>(a.quats) + n);
-    const float s0 = a.scales[3 * n], s1 = a.scales[3 * n + 1];
-    const m3 Rq = quat_rot(q.x, q.y, q.z, q.w);
-    f3 v_mean = mk3(0, 0, 0);
-    float4 v_quat = make_float4(0, 0, 0, 0);
-    float v_s0 = 0.f, v_s1 = 0.f;
-    for (int c = 0; c < a.C; ++c) {
-        const int64_t idx = (int64_t)c * a.N + n;
-        if (a.radii[idx] <= 0) continue;
-        const EntryGrad g = project_entry_vjp(
-            a.viewmats, a.Ks, c, p, q, s0, s1, Rq, a.ray_transforms + 9 * idx, a.v_ray_transforms + 9 * idx,
-            a.v_depths[idx], a.v_means2d[2 * idx], a.v_means2d[2 * idx + 1],
-            mk3(a.v_normals[3 * idx], a.v_normals[3 * idx + 1], a.v_normals[3 * idx + 2]), a.mode);
-        v_quat.x += g.v_quat.x; v_quat.y += g.v_quat.y; v_quat.z += g.v_quat.z; v_quat.w += g.v_quat.w;
-        v_s0 += g.v_s0;
-        v_s1 += g.v_s1;
-        v_mean = v_mean + g.v_mean;
-        if constexpr (kSH) {
-            const f3 gc = mk3(a.v_colors[3 * idx], a.v_colors[3 * idx + 1], a.v_colors[3 * idx + 2]);
-            v_mean = v_mean + fused_sh_vjp<NB>(a.means, a.viewmats, a.sh_K, a.sh_coeffs, c, n, gc, acc);
+    if (lane < cnt) {
+        const float* crow = kStage ? s_sh + lane * ShRows<NB>::kPitch : a.sh_coeffs + n * a.sh_K * 3;
+        const f3 p = mk3(a.means[3 * n], a.means[3 * n + 1], a.means[3 * n + 2]);
+        const float4 q = __ldg(reinterpret_cast<const float4*>(a.quats) + n);
+        const float s0 = a.scales[3 * n], s1 = a.scales[3 * n + 1];
+        const m3 Rq = quat_rot(q.x, q.y, q.z, q.w);
+        f3 v_mean = mk3(0, 0, 0);
+        float4 v_quat = make_float4(0, 0, 0, 0);
+        float v_s0 = 0.f, v_s1 = 0.f;
+        for (int c = 0; c < a.C; ++c) {
+            const int64_t idx = (int64_t)c * a.N + n;
+            if (a.radii[idx] <= 0) continue;
+            const EntryGrad g = project_entry_vjp(
+                a.viewmats, a.Ks, c, p, q, s0, s1, Rq, a.ray_transforms + 9 * idx, a.v_ray_transforms + 9 * idx,
+                a.v_depths[idx], a.v_means2d[2 * idx], a.v_means2d[2 * idx + 1],
+                mk3(a.v_normals[3 * idx], a.v_normals[3 * idx + 1], a.v_normals[3 * idx + 2]), a.mode);
+            v_quat.x += g.v_quat.x; v_quat.y += g.v_quat.y; v_quat.z += g.v_quat.z; v_quat.w += g.v_quat.w;
+            v_s0 += g.v_s0;
+            v_s1 += g.v_s1;
+            v_mean = v_mean + g.v_mean;
+            if constexpr (kSH) {
+                const f3 gc = mk3(a.v_colors[3 * idx], a.v_colors[3 * idx + 1], a.v_colors[3 * idx + 2]);
+                v_mean = v_mean + fused_sh_vjp<NB>(a.means, a.viewmats, crow, c, n, gc, acc);
+            }
+        }
+        store3(a.v_means, n, v_mean);
+        reinterpret_cast<float4*>(a.v_quats)[n] = v_quat;
+        store3(a.v_scales, n, mk3(v_s0, v_s1, 0.f));
+        if constexpr (kStage) {
+#pragma unroll
+            for (int k = 0; k < 3 * NB; ++k) s_sh[lane * ShRows<NB>::kPitch + k] = acc[k];  // (the lane's own row)
+        } else if constexpr (kSH) {
+            float* vc = a.v_sh_coeffs + n * a.sh_K * 3;
+            for (int k = 0; k < 3 * a.sh_K; ++k) vc[k] = k < 3 ? acc[k % 3] : 0.f;
         }
     }
-    if constexpr (kSH) {
-        float* vc = a.v_sh_coeffs + n * a.sh_K * 3;
-#pragma unroll
-        for (int k = 0; k < 3 * NB; ++k) vc[k] = acc[k];
-        for (int k = 3 * NB; k < 3 * a.sh_K; ++k) vc[k] = 0.f;
+    if constexpr (kStage) {
+        __syncwarp();
+        const int row = 3 * a.sh_K;
+        for (int i = lane; i < cnt * row; i += 32) {
+            const int r = i / row, k = i - r * row;
+            a.v_sh_coeffs[n0 * row + i] = k < 3 * NB ? s_sh[r * ShRows<NB>::kPitch + k] : 0.f;
+        }
     }
-    a.v_means[3 * n] = v_mean.x;
-    a.v_means[3 * n + 1] = v_mean.y;
-    a.v_means[3 * n + 2] = v_mean.z;
-    reinterpret_cast<float4*>(a.v_quats)[n] = v_quat;
-    a.v_scales[3 * n] = v_s0;
-    a.v_scales[3 * n + 1] = v_s1;
-    a.v_scales[3 * n + 2] = 0.f;
 }
 
 // Packed adjoint: one thread per entry.  Sparse: the entry's gradient is
@@ -522,7 +599,7 @@ __global__ void __launch_bounds__(256) project_packed_bwd_kernel(tg_project_pack
         for (int k = 0; k < 3 * NB; ++k) acc[k] = 0.f;
         const f3 gc = mk3(a.v_colors[3 * i], a.v_colors[3 * i + 1], a.v_colors[3 * i + 2]);
         if (gc.x != 0.f || gc.y != 0.f || gc.z != 0.f) {
-            v_dir = fused_sh_vjp<NB>(a.means, a.viewmats, a.sh_K, a.sh_coeffs, (int)c, n, gc, acc);
+            v_dir = fused_sh_vjp<NB>(a.means, a.viewmats, a.sh_coeffs + n * a.sh_K * 3, (int)c, n, gc, acc);
             float* vc = a.v_sh_coeffs + n * a.sh_K * 3;
 #pragma unroll
             for (int k = 0; k < 3 * NB; ++k)
@@ -556,24 +633,44 @@ __global__ void __launch_bounds__(256) project_packed_bwd_kernel(tg_project_pack
     }
 }
 
+template <int NB>
+void project_fwd(const tg_project_fwd_args& a, cudaStream_t s) {
+    // a CTA takes its Gaussians through every camera (their parameters and SH rows read once), or, where that
+    // leaves fewer than about eight CTAs per SM, through a share of the cameras
+    constexpr int threads = 32 * kProjWarps<NB>;
+    const int64_t bx = ((int64_t)a.N + threads - 1) / threads;
+    const int64_t by = std::min<int64_t>({(int64_t)a.C, (kNumSMs * 8 + bx - 1) / bx, (int64_t)65535});
+    project_fwd_kernel<NB><<<dim3((unsigned)bx, (unsigned)by), threads, 0, s>>>(a);
+}
+template <int NB>
+void project_bwd(const tg_project_bwd_args& a, cudaStream_t s) {
+    constexpr int threads = 32 * kProjWarps<NB>;
+    project_bwd_kernel<NB><<<(unsigned)(((int64_t)a.N + threads - 1) / threads), threads, 0, s>>>(a);
+}
+
 cudaError_t launch_project_fwd(const tg_project_fwd_args& a, cudaStream_t s) {
-    const int64_t total = (int64_t)a.C * a.N;
-    if (total == 0) return cudaSuccess;
-    project_fwd_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(a);
+    if ((int64_t)a.C * a.N == 0) return cudaSuccess;
+    switch (a.sh_coeffs ? a.sh_degree : -1) {
+        case 0: project_fwd<1>(a, s); break;
+        case 1: project_fwd<4>(a, s); break;
+        case 2: project_fwd<9>(a, s); break;
+        case 3: project_fwd<16>(a, s); break;
+        case 4: project_fwd<25>(a, s); break;
+        default: project_fwd<0>(a, s); break;
+    }
     note_launches(1);
     return cudaGetLastError();
 }
 
 cudaError_t launch_project_bwd(const tg_project_bwd_args& a, cudaStream_t s) {
     if (a.N == 0) return cudaSuccess;
-    const unsigned grid = (unsigned)((a.N + 255) / 256);
     switch (a.sh_coeffs ? a.sh_degree : -1) {
-        case 0: project_bwd_kernel<1><<<grid, 256, 0, s>>>(a); break;
-        case 1: project_bwd_kernel<4><<<grid, 256, 0, s>>>(a); break;
-        case 2: project_bwd_kernel<9><<<grid, 256, 0, s>>>(a); break;
-        case 3: project_bwd_kernel<16><<<grid, 256, 0, s>>>(a); break;
-        case 4: project_bwd_kernel<25><<<grid, 256, 0, s>>>(a); break;
-        default: project_bwd_kernel<0><<<grid, 256, 0, s>>>(a); break;
+        case 0: project_bwd<1>(a, s); break;
+        case 1: project_bwd<4>(a, s); break;
+        case 2: project_bwd<9>(a, s); break;
+        case 3: project_bwd<16>(a, s); break;
+        case 4: project_bwd<25>(a, s); break;
+        default: project_bwd<0>(a, s); break;
     }
     note_launches(1);
     return cudaGetLastError();
@@ -614,8 +711,16 @@ cudaError_t launch_project_packed_count(const tg_project_packed_args& a, cudaStr
 cudaError_t launch_project_packed_emit(const tg_project_packed_args& a, cudaStream_t s) {
     const int64_t per_row = packed_chunks_per_row(a);
     if ((int64_t)a.C * per_row == 0 || a.nnz_host == 0) return cudaSuccess;
-    project_packed_emit_kernel<<<dim3((unsigned)per_row, (unsigned)a.C), kPackThreads, 0, s>>>(
-        a, static_cast<const int64_t*>(a.workspace));
+    const dim3 grid((unsigned)per_row, (unsigned)a.C);
+    const int64_t* chunk = static_cast<const int64_t*>(a.workspace);
+    switch (a.sh_coeffs ? a.sh_degree : -1) {
+        case 0: project_packed_emit_kernel<1><<<grid, kPackThreads, 0, s>>>(a, chunk); break;
+        case 1: project_packed_emit_kernel<4><<<grid, kPackThreads, 0, s>>>(a, chunk); break;
+        case 2: project_packed_emit_kernel<9><<<grid, kPackThreads, 0, s>>>(a, chunk); break;
+        case 3: project_packed_emit_kernel<16><<<grid, kPackThreads, 0, s>>>(a, chunk); break;
+        case 4: project_packed_emit_kernel<25><<<grid, kPackThreads, 0, s>>>(a, chunk); break;
+        default: project_packed_emit_kernel<0><<<grid, kPackThreads, 0, s>>>(a, chunk); break;
+    }
     note_launches(1);
     if (a.overflow) {
         packed_tail_kernel<<<(unsigned)((a.nnz_host + 255) / 256), 256, 0, s>>>(a.nnz, a.nnz_host, a.N,

@@ -60,18 +60,21 @@ __device__ __forceinline__ void sh_bases(int degree, S x, S y, S z, S* b) {
 }
 
 // Colour (before the +0.5 / clamp) of direction d (not normalised) under the
-// coefficients c [K][3].
-__device__ __forceinline__ f3 sh_color(int degree, f3 d, const float* __restrict__ c) {
-    float b[25];
-    if (degree >= 1) {
+// coefficients c [K][3], with NB = (degree+1)^2 bases (a compile-time count:
+// with a runtime one the bases live in local memory).
+template <int NB>
+__device__ __forceinline__ f3 sh_color(f3 d, const float* __restrict__ c) {
+    constexpr int degree = NB == 1 ? 0 : NB == 4 ? 1 : NB == 9 ? 2 : NB == 16 ? 3 : 4;
+    float b[NB];
+    if constexpr (degree >= 1) {
         const float inv = rsqrtf(d.x * d.x + d.y * d.y + d.z * d.z);
         sh_bases<float>(degree, d.x * inv, d.y * inv, d.z * inv, b);
     } else {
         b[0] = 0.2820947917738781f;
     }
-    const int nb = (degree + 1) * (degree + 1);
     float r0 = 0.f, r1 = 0.f, r2 = 0.f;
-    for (int k = 0; k < nb; ++k) {
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
         r0 += b[k] * c[3 * k];
         r1 += b[k] * c[3 * k + 1];
         r2 += b[k] * c[3 * k + 2];
