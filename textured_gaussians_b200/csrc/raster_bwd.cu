@@ -350,11 +350,7 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
     const uint32_t* bits_base = have_bits ? f.contrib_masks + ((int64_t)tc.t + (range_start >> 5)) * (int64_t)(ts * ts) +
                                                 sub * nt + tr
                                           : nullptr;
-    const uint32_t* words = S.words + (size_t)(Filt::kAniso ? (tr >> 5) * 4 : tr >> 3) * n_words;
-    auto list_word = [&](int w) -> uint32_t {
-        if constexpr (Filt::kAniso) return words[w] | words[w + n_words] | words[w + 2 * n_words] | words[w + 3 * n_words];
-        else return words[w];
-    };
+    const uint32_t* words = S.words + (size_t)(tr >> 3) * n_words;  // the lane's group's list
 
     for (int b = max_bin < range_start ? -1 : (max_bin - range_start) / bs; b >= 0; --b) {
         const int32_t batch_start = range_start + b * bs;
@@ -404,10 +400,10 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
         }
         __syncthreads();
         int w = n_words - 1;
-        uint32_t bits = list_word(w), own = S.pixels[w * nt + tr];
+        uint32_t bits = words[w], own = S.pixels[w * nt + tr];
         for (;;) {
             while (bits == 0u && w > 0) {
-                bits = list_word(--w);
+                bits = words[--w];
                 own = S.pixels[w * nt + tr];
             }
             if (!__any_sync(kFull, bits != 0u)) break;
@@ -436,11 +432,9 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
                                           ? reinterpret_cast<const float4*>(f.aniso_records) +
                                                 pix * f.aniso_record_cap + rec
                                           : nullptr;
-                    eval_aniso_coop<Tex, true>(e, act, P.px, P.py, xyo, m0, m1, m2, f.textures, tex_base, f.tex_rx,
-                                               f.tex_ry, f.range_x, f.range_y, f.g_weight, kFull,
-                                               f.aniso_prefix ? reinterpret_cast<const float4*>(f.aniso_prefix) + tex_base
-                                                              : nullptr,
-                                               s_aniso, r);
+                    eval_aniso_coop<Tex, true>(e, act, P.px, P.py, xyo, m0, m1, m2, f.textures, row, f.tex_rx, f.tex_ry,
+                                               f.range_x, f.range_y, f.g_weight, kFull,
+                                               reinterpret_cast<const float4*>(f.aniso_prefix), s_aniso, r);
                     if (act) --rec;
                 } else {
                     eval_pair<Tex, Filt>(e, P.px, P.py, xyo, m0, m1, m2, f.textures, tex_base, f.tex_rx, f.tex_ry,
@@ -470,19 +464,9 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
                     aniso_coop_scatter<true>(e.F, g4,
                                              use && e.tex_valid && vt != nullptr &&
                                                  (g4.x != 0.f || g4.y != 0.f || g4.z != 0.f || g4.w != 0.f),
-                                             vt, f.tex_rx, kFull,
-                                             a.v_aniso_prefix != nullptr ? a.v_aniso_prefix + 4 * tex_base : nullptr,
-                                             f.tex_ry, s_aniso);
+                                             a.v_textures, row, f.tex_rx, f.tex_ry, kFull, a.v_aniso_prefix, s_aniso);
             }
             reduce_scatter8<NS>(vals);
-            if constexpr (Filt::kAniso) {  // the four groups hold the same splat
-#pragma unroll
-                for (int k = 0; k < NS / 8; ++k) {
-                    vals[k] += __shfl_xor_sync(kFull, vals[k], 8);
-                    vals[k] += __shfl_xor_sync(kFull, vals[k], 16);
-                }
-                if (lane >= 8) continue;
-            }
             const int64_t g = S.entry[t];
             const int slot = slot_base<NS>(lane);
             if (a.v_packed != nullptr) {

@@ -445,14 +445,16 @@ static __device__ __noinline__ void segment_scatter(float2 a, float2 b, float4 g
 // segment's owner lane (and x0), and one float4 per lane.  Small on purpose: the compositor's shared memory
 // comes out of the L1 that the boundary walk reads the texture through.
 constexpr int kAnisoSegs = 64;
-constexpr int kAnisoWarpF4 = kAnisoSegs + 32 + kAnisoSegs / 4;  // segments, per-lane slots, owners (int)
+constexpr int kAnisoWarpF4 = kAnisoSegs + 32 + kAnisoSegs / 4 + 8;  // segments, per-lane slots, owners, rows (int)
 struct AnisoWarp {
     float4* seg;  // [kAnisoSegs] (a.x, a.y, b.x, b.y)
     float4* lane; // [32]
     int* own;     // [kAnisoSegs] owner lane | x0 << 5
+    int* row;     // [32] texture row of each lane's splat (the warp's groups work on different splats)
 };
 __device__ __forceinline__ AnisoWarp aniso_warp(float4* base) {
-    return AnisoWarp{base, base + kAnisoSegs, reinterpret_cast<int*>(base + kAnisoSegs + 32)};
+    int* own = reinterpret_cast<int*>(base + kAnisoSegs + 32);
+    return AnisoWarp{base, base + kAnisoSegs, own, own + kAnisoSegs};
 }
 
 // The kept boundary segments of a lane's footprint (want: a convex footprint with cells to integrate) and
@@ -505,8 +507,8 @@ __device__ __forceinline__ void aniso_put(const SegList& L, int r0, const AnisoW
 // Every lane's footprint integral (before the division by the area) for the lanes with want set, the warp's
 // boundary segments spread over its lanes and summed per owner in shared memory.  Called by the full warp.
 template <class Tex, bool kShared>
-__device__ __forceinline__ float4 aniso_boundary_sum(const AnisoFoot& F, bool want, const void* textures,
-                                                     int64_t tex_base, const float4* P, int rx, int ry, float scale,
+__device__ __forceinline__ float4 aniso_boundary_sum(const AnisoFoot& F, bool want, const void* textures, int row,
+                                                     const float4* P, int rx, int ry, float scale,
                                                      const AnisoWarp& W, unsigned mask) {
     const int lane = threadIdx.x & 31;
     want = want && F.maxu > F.minu && F.maxv > F.minv;  // no cell (also: rx or ry below 2): nothing to walk
@@ -514,6 +516,7 @@ __device__ __forceinline__ float4 aniso_boundary_sum(const AnisoFoot& F, bool wa
     SegList L;
     aniso_segments(F, want, rx, ry, mask, L);
     W.lane[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+    W.row[lane] = row;
     for (int r0 = 0; r0 < L.total; r0 += kAnisoSegs) {
         aniso_put(L, r0, W, lane | (F.minu << 5));
         __syncwarp(mask);
@@ -522,9 +525,10 @@ __device__ __forceinline__ float4 aniso_boundary_sum(const AnisoFoot& F, bool wa
             const float4 sg = W.seg[t];
             const int ow = W.own[t];
             const float2 a = make_float2(sg.x, sg.y), b = make_float2(sg.z, sg.w);
+            const int64_t base = (int64_t)W.row[ow & 31] * (ry * rx);
             float4 r;
-            if constexpr (kShared) r = segment_sum_shared<Tex>(a, b, ow >> 5, textures, tex_base, P, rx, ry, scale);
-            else r = segment_sum<Tex>(a, b, ow >> 5, textures, tex_base, P, rx, ry, scale);
+            if constexpr (kShared) r = segment_sum_shared<Tex>(a, b, ow >> 5, textures, base, P + base, rx, ry, scale);
+            else r = segment_sum<Tex>(a, b, ow >> 5, textures, base, P + base, rx, ry, scale);
             float* dst = reinterpret_cast<float*>(W.lane + (ow & 31));
             atomicAdd(dst, r.x);
             atomicAdd(dst + 1, r.y);
@@ -540,22 +544,25 @@ __device__ __forceinline__ float4 aniso_boundary_sum(const AnisoFoot& F, bool wa
 
 // Adjoint of aniso_boundary_sum: the gradient g of every lane with want set (already divided by the area)
 // scattered along its footprint's boundary, the segments spread over the warp.  Called by the full warp.
+// vt, vP: the first splat's rows.
 __device__ __forceinline__ void aniso_boundary_scatter(const AnisoFoot& F, float4 g, bool want, float* vt, float* vP,
-                                                       int rx, int ry, const AnisoWarp& W, unsigned mask) {
+                                                       int row, int rx, int ry, const AnisoWarp& W, unsigned mask) {
     const int lane = threadIdx.x & 31;
     want = want && F.maxu > F.minu && F.maxv > F.minv;
     if (!__any_sync(mask, want)) return;
     SegList L;
     aniso_segments(F, want, rx, ry, mask, L);
     W.lane[lane] = g;
+    W.row[lane] = row;
     for (int r0 = 0; r0 < L.total; r0 += kAnisoSegs) {
         aniso_put(L, r0, W, lane);
         __syncwarp(mask);
         const int n = min(kAnisoSegs, L.total - r0);
         for (int t = lane; t < n; t += 32) {
             const float4 sg = W.seg[t];
-            segment_scatter(make_float2(sg.x, sg.y), make_float2(sg.z, sg.w), W.lane[W.own[t] & 31], vt, vP, rx,
-                            ry);
+            const int ow = W.own[t] & 31;
+            const int64_t base = (int64_t)W.row[ow] * (4 * ry * rx);
+            segment_scatter(make_float2(sg.x, sg.y), make_float2(sg.z, sg.w), W.lane[ow], vt + base, vP + base, rx, ry);
         }
         __syncwarp(mask);  // the list is read before the next round rewrites it
     }
@@ -823,15 +830,14 @@ __device__ __forceinline__ void foot_cell(const AnisoFoot& F, int i, int& u, int
 // integrated; returns the lane's own integral (not yet divided by the area).
 // The warp must be full (mask = all 32 lanes).
 template <class Tex, bool kShared = false>
-__device__ __forceinline__ float4 aniso_coop_sum(const AnisoFoot& Fown, bool need, const void* textures,
-                                                 int64_t tex_base, int rx, float scale, unsigned mask,
-                                                 const float4* P = nullptr, int ry = 0, float4* s_warp = nullptr) {
+__device__ __forceinline__ float4 aniso_coop_sum(const AnisoFoot& Fown, bool need, const void* textures, int row,
+                                                 int rx, int ry, float scale, unsigned mask, const float4* P,
+                                                 float4* s_warp) {
     const int lane = threadIdx.x & 31;
     float4 mine = make_float4(0.f, 0.f, 0.f, 0.f);
-    // with the row-prefix table, convex footprints are integrated along their boundaries (P is the same for
-    // the whole warp); the others cell by cell
+    // with the row-prefix table, convex footprints are integrated along their boundaries; the others cell by cell
     if (P != nullptr) {
-        mine = aniso_boundary_sum<Tex, kShared>(Fown, need && Fown.convex, textures, tex_base, P, rx, ry, scale,
+        mine = aniso_boundary_sum<Tex, kShared>(Fown, need && Fown.convex, textures, row, P, rx, ry, scale,
                                                 aniso_warp(s_warp), mask);
         need = need && !Fown.convex;
     }
@@ -840,6 +846,7 @@ __device__ __forceinline__ float4 aniso_coop_sum(const AnisoFoot& Fown, bool nee
         const int L = __ffs(pending) - 1;
         pending &= pending - 1;
         const AnisoFoot F = shfl_foot(Fown, L, mask);
+        const int64_t tex_base = (int64_t)__shfl_sync(mask, row, L) * (ry * rx);
         // a footprint wholly outside the texture has an empty (possibly inverted) cell range: no cells
         const int n = (F.maxu > F.minu && F.maxv > F.minv) ? (F.maxu - F.minu) * (F.maxv - F.minv) : 0;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -866,12 +873,11 @@ __device__ __forceinline__ float4 aniso_coop_sum(const AnisoFoot& Fown, bool nee
 // Texel-gradient scatter of every lane's footprint (gown: the lane's gradient
 // already divided by the area; need: it has one), cells spread over the warp.
 template <bool kShared = false>
-__device__ __forceinline__ void aniso_coop_scatter(const AnisoFoot& Fown, float4 gown, bool need, float* vt, int rx,
-                                                   unsigned mask, float* vP = nullptr, int ry = 0,
-                                                   float4* s_warp = nullptr) {
+__device__ __forceinline__ void aniso_coop_scatter(const AnisoFoot& Fown, float4 gown, bool need, float* vt, int row,
+                                                   int rx, int ry, unsigned mask, float* vP, float4* s_warp) {
     const int lane = threadIdx.x & 31;
     if (vP != nullptr) {  // uniform over the warp
-        aniso_boundary_scatter(Fown, gown, need && Fown.convex, vt, vP, rx, ry, aniso_warp(s_warp), mask);
+        aniso_boundary_scatter(Fown, gown, need && Fown.convex, vt, vP, row, rx, ry, aniso_warp(s_warp), mask);
         need = need && !Fown.convex;
     }
     unsigned pending = __ballot_sync(mask, need);
@@ -881,6 +887,7 @@ __device__ __forceinline__ void aniso_coop_scatter(const AnisoFoot& Fown, float4
         const AnisoFoot F = shfl_foot(Fown, L, mask);
         const float4 g = make_float4(__shfl_sync(mask, gown.x, L), __shfl_sync(mask, gown.y, L),
                                      __shfl_sync(mask, gown.z, L), __shfl_sync(mask, gown.w, L));
+        float* vl = vt + (int64_t)__shfl_sync(mask, row, L) * (4 * ry * rx);
         // a footprint wholly outside the texture has an empty (possibly inverted) cell range: no cells
         const int n = (F.maxu > F.minu && F.maxv > F.minv) ? (F.maxu - F.minu) * (F.maxv - F.minv) : 0;
         for (int i = lane; i < n; i += 32) {
@@ -889,7 +896,7 @@ __device__ __forceinline__ void aniso_coop_scatter(const AnisoFoot& Fown, float4
             const float4 mo = aniso_cell<kShared>(F, u, v);
             if (mo.x == 0.f && mo.y == 0.f && mo.z == 0.f && mo.w == 0.f) continue;
             const float4 w = cell_weights(mo);
-            float4* t00 = reinterpret_cast<float4*>(vt + 4 * ((int64_t)v * rx + u));
+            float4* t00 = reinterpret_cast<float4*>(vl + 4 * ((int64_t)v * rx + u));
             atomicAdd(t00, make_float4(g.x * w.x, g.y * w.x, g.z * w.x, g.w * w.x));
             atomicAdd(t00 + 1, make_float4(g.x * w.y, g.y * w.y, g.z * w.y, g.w * w.y));
             atomicAdd(t00 + rx, make_float4(g.x * w.z, g.y * w.z, g.z * w.z, g.w * w.z));
@@ -898,25 +905,25 @@ __device__ __forceinline__ void aniso_coop_scatter(const AnisoFoot& Fown, float4
     }
 }
 
-// The anisotropic_bilinear pair evaluation for a whole (full) warp working on
-// one splat: every lane calls it, act = the lane has a pair to evaluate; the
-// footprints that need integrating are integrated by the warp together.
+// The anisotropic_bilinear pair evaluation for a whole (full) warp: every lane
+// calls it with its own splat (row: its texture row), act = the lane has a pair
+// to evaluate; the footprints that need integrating are integrated by the warp
+// together.  P: the row-prefix tables of all textures, or NULL.
 template <class Tex, bool kShared = false>
 __device__ __forceinline__ void eval_aniso_coop(PairEvalAniso& e, bool act, float px, float py, const float4 xyo,
                                                 const float4 m0, const float4 m1, const float4 m2,
-                                                const void* textures, int64_t tex_base, int rx, int ry, float range_x,
-                                                float range_y, float g_weight, unsigned mask,
-                                                const float4* P = nullptr, float4* s_warp = nullptr,
-                                                const float4* rec = nullptr) {
+                                                const void* textures, int row, int rx, int ry, float range_x,
+                                                float range_y, float g_weight, unsigned mask, const float4* P,
+                                                float4* s_warp, const float4* rec = nullptr) {
     e.valid = false;
     e.need = false;
     e.tex_valid = false;
     if (act)
-        eval_pair<Tex, FiltAniso>(e, px, py, xyo, m0, m1, m2, textures, tex_base, rx, ry, range_x, range_y, g_weight);
+        eval_pair<Tex, FiltAniso>(e, px, py, xyo, m0, m1, m2, textures, 0, rx, ry, range_x, range_y, g_weight);
     const bool need = act && e.valid && e.need;
     const bool have = need && rec != nullptr;  // rec: the forward's record of this footprint's integral
     if (need && (P == nullptr || !e.F.convex)) aniso_cells_setup(e.F);  // integrated (or scattered) cell by cell
-    float4 ts = aniso_coop_sum<Tex, kShared>(e.F, need && !have, textures, tex_base, rx, xyo.w, mask, P, ry, s_warp);
+    float4 ts = aniso_coop_sum<Tex, kShared>(e.F, need && !have, textures, row, rx, ry, xyo.w, mask, P, s_warp);
     if (have) ts = *rec;
     if (!(act && e.valid)) return;
     e.asf = 0.f;
@@ -1011,6 +1018,12 @@ __device__ __forceinline__ PixelSlot pixel_slot(int tid, int side) {
     const int lane = tid & 31, warp = tid >> 5, per_row = side >> 3;
     const int wy = warp / per_row, wx = warp - wy * per_row;
     return PixelSlot{wx * 8 + ((lane >> 3) & 1) * 4 + (lane & 3), wy * 4 + (lane >> 4) * 2 + ((lane >> 2) & 1)};
+}
+
+// The thread of pixel_slot that owns pixel (x, y) of the square.
+__device__ __forceinline__ int slot_of_pixel(int x, int y, int side) {
+    return ((y >> 2) * (side >> 3) + (x >> 3)) * 32 + (((y >> 1) & 1) << 4) + (((x >> 2) & 1) << 3) + ((y & 1) << 2) +
+           (x & 3);
 }
 
 // Bits of the 4x2 groups of row band k (two pixel rows) whose columns are set in `cols`, in the order
