@@ -472,6 +472,12 @@ typedef struct {
      * splats 32 k .. 32 k + 31 of tile t's list.  NULL: none (the adjoint then
      * tests every pair again).  No counterpart in the reference. */
     uint32_t* contrib_masks;
+    /* Scratch [n_entries,20] FP32, 16-byte aligned, or NULL: the forward packs
+     * what it stages of each entry into it first, and the adjoint, given the
+     * same pointer and unchanged inputs, reads it too.  n_entries = E (used
+     * only with entry_records).  No counterpart in the reference. */
+    float* entry_records;
+    int64_t n_entries;
 } tg_raster_fwd_args;
 TG_API int tg_rasterize_fwd(const tg_raster_fwd_args* a, tg_stream_t stream);
 

@@ -83,7 +83,7 @@ class RasterFwdArgs(ctypes.Structure):
                 ("batch_depth", I32), ("work_queue", P), ("mip_levels", I32), ("tex_coarse", P),
                 ("filter", I32), ("t_checkpoints", P), ("aniso_prefix", P),
                 ("aniso_records", P), ("aniso_record_count", P), ("aniso_record_cap", I32),
-                ("contrib_masks", P)]
+                ("contrib_masks", P), ("entry_records", P), ("n_entries", I64)]
 
 
 class RasterBwdArgs(ctypes.Structure):

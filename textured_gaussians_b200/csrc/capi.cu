@@ -157,6 +157,9 @@ int check_raster_common(const tg_raster_fwd_args& a) {
             break;
         default: return fail(TG_ERR_UNSUPPORTED, "unknown texture format %d", a.tex_format);
     }
+    TG_REQUIRE(a.entry_records == nullptr ||
+                   (aligned(a.entry_records, 16) && a.n_entries >= 0 && a.n_entries < (int64_t(1) << 31)),
+               TG_ERR_INVALID_ARG, "entry_records needs 16-byte alignment and n_entries");
     if (a.tex_format != TG_TEX_NONE)
         TG_REQUIRE(a.tex_rx >= 1 && a.tex_ry >= 1 && a.range_x > 0.f && a.range_y > 0.f, TG_ERR_INVALID_ARG,
                    "bad texture size or range");

@@ -14,7 +14,7 @@
 // Reductions:
 //  * per-splat gradients (colour, ray transform, means2d, opacity; with an upstream gradient for normals, distortion
 //    or median depth, or |means2d| asked for, also those) are summed over a group's eight lanes by a reduce-scatter
-//    (14 shuffles for 16 values, 21 for 24) that leaves consecutive values in consecutive lanes, which add them to
+//    (14 shuffles for 16 values, 21 for 24; of the ray transform its moments) that leaves consecutive values in consecutive lanes, which add them to
 //    the entry's row of a packed [E, slots] buffer -- 64 contiguous bytes, two per lane.  A splat meets 1.1 groups
 //    per tile that lists it, so collecting a tile's sums in shared memory first would not save adds; the rows are
 //    spread to the separate gradient arrays by one pass over the entries afterwards;
@@ -73,9 +73,13 @@ __device__ __forceinline__ int slot_base(int lane) {
 #ifndef TG_BWD_MIN_CTAS_ANISO
 #define TG_BWD_MIN_CTAS_ANISO 3
 #endif
-template <class Filt, bool kGeo>
+// Two CTAs (up to 128 registers) where three spill more than they hide: FP32 textures (1496 against 1560 us for 100k
+// splats of 50x50 texels, 800x800), mipmapped2 (687 against 703 us), the geometric sums and the UV term; with 16-bit
+// textures three are faster (9.31 against 10.18 ms for the 1M-splat mixture, four views), and four slower throughout.
+template <class Tex, class Filt, bool kGeo>
 struct BwdBounds {
-    static constexpr int kMinCtas = Filt::kAniso ? TG_BWD_MIN_CTAS_ANISO : (kGeo || Filt::kUV) ? 2 : TG_BWD_MIN_CTAS;
+    static constexpr bool kWide = kGeo || Filt::kUV || Filt::kMip || Tex::kFormat == TG_TEX_F32;
+    static constexpr int kMinCtas = Filt::kAniso ? TG_BWD_MIN_CTAS_ANISO : kWide ? 2 : TG_BWD_MIN_CTAS;
 };
 
 // Per-pixel state of the back-to-front sweep.  Everything behind the current splat enters its alpha's gradient
@@ -164,14 +168,14 @@ __device__ __forceinline__ void accumulate_pair(const tg_raster_bwd_args& a, con
             *aniso_g = make_float4(g.x * ia, g.y * ia, g.z * ia, g.w * ia);
         }
     } else if (kTextured && e.tex_valid && vt != nullptr) {
+        const float4 g = make_float4(D > 0 ? fac * P.v_c[0] : 0.f, D > 1 ? fac * P.v_c[D > 1 ? 1 : 0] : 0.f,
+                                     D > 2 ? fac * P.v_c[D > 2 ? 2 : 0] : 0.f,
+                                     (D > 3 ? fac * P.v_c[D > 3 ? 3 : 0] : 0.f) + tex_a_grad);
+        const bool any = g.x != 0.f || g.y != 0.f || g.z != 0.f || g.w != 0.f;
 #pragma unroll
         for (int q = 0; q < Filt::kTaps; ++q) {
-            float4 gq;
-            gq.x = 0 < D ? fac * e.w[q] * P.v_c[0] : 0.f;
-            gq.y = 1 < D ? fac * e.w[q] * P.v_c[1 < D ? 1 : 0] : 0.f;
-            gq.z = 2 < D ? fac * e.w[q] * P.v_c[2 < D ? 2 : 0] : 0.f;
-            gq.w = (3 < D ? fac * e.w[q] * P.v_c[3 < D ? 3 : 0] : 0.f) + e.w[q] * tex_a_grad;
-            if (gq.x != 0.f || gq.y != 0.f || gq.z != 0.f || gq.w != 0.f) {
+            if (any && e.w[q] != 0.f) {
+                const float4 gq = make_float4(e.w[q] * g.x, e.w[q] * g.y, e.w[q] * g.z, e.w[q] * g.w);
                 if constexpr (Filt::kMip) {  // pyramid coordinate: coarse levels, or level 0 = the texture
                     const int mc = e.toff[q];
                     float* dst = mc < mip_clen ? vct + 4 * (int64_t)mc : vt + 4 * (int64_t)(mc - mip_clen);
@@ -211,6 +215,12 @@ __device__ __forceinline__ void accumulate_pair(const tg_raster_bwd_args& a, con
         const float iz = 1.f / e.z.z;
         const float a_ = vsx * iz, b_ = vsy * iz;
         const f3 vz = mk3(a_, b_, -(a_ * e.sx + b_ * e.sy));
+        if (a.v_packed != nullptr) {  // the moments about the projected centre (see unpack_grads_kernel)
+            vals[GS::kM + 0] = vz.x; vals[GS::kM + 1] = vz.y; vals[GS::kM + 2] = vz.z;
+            vals[GS::kM + 3] = e.dx * vz.x; vals[GS::kM + 4] = e.dx * vz.y; vals[GS::kM + 5] = e.dx * vz.z;
+            vals[GS::kM + 6] = e.dy * vz.x; vals[GS::kM + 7] = e.dy * vz.y; vals[GS::kM + 8] = e.dy * vz.z;
+            return;
+        }
         const f3 vhu = cross(e.hv, vz), vhv = cross(vz, e.hu);
         vals[GS::kM + 0] = -vhu.x; vals[GS::kM + 1] = -vhu.y; vals[GS::kM + 2] = -vhu.z;
         vals[GS::kM + 3] = -vhv.x; vals[GS::kM + 4] = -vhv.y; vals[GS::kM + 5] = -vhv.z;
@@ -361,29 +371,20 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
             uint32_t reach = 0u;
             if (idx <= max_bin) {
                 const int32_t g = f.flatten_ids[idx];
-                const float2 xy = reinterpret_cast<const float2*>(f.means2d)[g];
-                const int32_t row = f.gaussian_ids ? (int32_t)f.gaussian_ids[g] : g % f.N;
-                const float op = f.opacities[g];
-                const float* m = f.ray_transforms + 9 * (int64_t)g;
-                const float4 m0 = make_float4(m[0], m[1], m[2], xy.x), m1 = make_float4(m[3], m[4], m[5], xy.y),
-                             m2 = make_float4(m[6], m[7], m[8], op);
-                S.m0[slot] = m0;
-                S.m1[slot] = m1;
-                S.m2[slot] = m2;
-                const float* c = f.colors + (int64_t)g * D;
-                S.col[slot] = make_float4(c[0], D > 1 ? c[D > 1 ? 1 : 0] : 0.f, D > 2 ? c[D > 2 ? 2 : 0] : 0.f,
-                                          D > 3 ? c[D > 3 ? 3 : 0] : 0.f);
-                if constexpr (D == 5) S.col5[slot] = c[4];
-                if constexpr (kGeo) {
-                    const float* n = f.normals + 3 * (int64_t)g;
-                    S.nrm[slot] = make_float4(n[0], n[1], n[2], 0.f);
-                }
+                const EntryRecord r = load_entry<D, kGeo>(f, g);
+                const int32_t row = __float_as_int(r.nrm.w);
+                S.m0[slot] = r.m0;
+                S.m1[slot] = r.m1;
+                S.m2[slot] = r.m2;
+                S.col[slot] = r.col;
+                if constexpr (D == 5) S.col5[slot] = f.colors[(int64_t)g * D + 4];
+                if constexpr (kGeo) S.nrm[slot] = r.nrm;
                 if constexpr (BwdSmem<D, Tex, kGeo>::kScale) S.scale[slot] = f.tex_scales[row];
                 S.row[slot] = row;
                 S.entry[slot] = g;
                 if (!have_bits)
-                    reach = group_mask(make_float4(xy.x, xy.y, op, 1.f), m0, m1, m2, kTextured, f.range_x, f.range_y,
-                                       f.g_weight, !Filt::kAniso, X0, Y0, side);
+                    reach = group_mask(make_float4(r.m0.w, r.m1.w, r.m2.w, 1.f), r.m0, r.m1, r.m2, kTextured, f.range_x,
+                                       f.range_y, f.g_weight, !Filt::kAniso, X0, Y0, side);
             }
             if (!have_bits) store_group_words(reach, S.words, n_words, slot >> 5, side);
         }
@@ -490,7 +491,7 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
 // CTA per work item, or (work_queue != NULL) a persistent grid whose CTAs take
 // items from the queue counter until none is left.
 template <int D, class Tex, bool kPersistent, class Filt, bool kGeo>
-__global__ void __launch_bounds__(256, BwdBounds<Filt, kGeo>::kMinCtas) raster_bwd_kernel(const tg_raster_bwd_args a,
+__global__ void __launch_bounds__(256, BwdBounds<Tex, Filt, kGeo>::kMinCtas) raster_bwd_kernel(const tg_raster_bwd_args a,
                                                                                           const float uv_scale,
                                                                                           const int bs,
                                                                                           const int64_t n_items) {
@@ -521,9 +522,39 @@ __global__ void densify_grad_kernel(const float* __restrict__ v_M, const float* 
     v_densify[2 * e + 1] = v_M[9 * e + 5] * depth;
 }
 
+// Gradient of the ray transform M from an entry's moments of v_zeta over its pairs: r = (S, X, Y) with S = sum v_zeta
+// and X, Y the sums weighted with the projected centre's offset (cx - px, cy - py).  h_u = px M2 - M0 and
+// h_v = py M2 - M1 are linear in the pixel, so the pairs' nine products
+//   v_h_u = h_v x v_zeta,  v_h_v = v_zeta x h_u,  v_M0 = -v_h_u,  v_M1 = -v_h_v,  v_M2 = px v_h_u + py v_h_v
+// sum to crosses of the moments with M (px py M2 x v_zeta cancels), formed here once per entry instead of once per
+// pair.  In FP64: M0 and M1 nearly cancel against the centre's multiple of M2.
+__device__ __forceinline__ void moments_to_transform(const float* __restrict__ M, float2 c, float* r) {
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) any = any || r[k] != 0.f;
+    if (!any) return;  // (and M may be anything)
+    struct d3 {
+        double x, y, z;
+    };
+    auto cross = [](d3 a, d3 b) { return d3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; };
+    const double cx = c.x, cy = c.y;
+    const d3 m2{M[6], M[7], M[8]};
+    const d3 m0{M[0] - cx * m2.x, M[1] - cx * m2.y, M[2] - cx * m2.z}, m1{M[3] - cy * m2.x, M[4] - cy * m2.y, M[5] - cy * m2.z};
+    const d3 s{r[0], r[1], r[2]}, sx{-(double)r[3], -(double)r[4], -(double)r[5]},
+        sy{-(double)r[6], -(double)r[7], -(double)r[8]};
+    const d3 a0 = cross(m2, sy), a1 = cross(m1, s), b0 = cross(sx, m2), b1 = cross(s, m0), e0 = cross(m0, sy),
+             e1 = cross(m1, sx);
+    const d3 A{a0.x - a1.x, a0.y - a1.y, a0.z - a1.z}, B{b0.x - b1.x, b0.y - b1.y, b0.z - b1.z};
+    r[0] = (float)-A.x; r[1] = (float)-A.y; r[2] = (float)-A.z;
+    r[3] = (float)-B.x; r[4] = (float)-B.y; r[5] = (float)-B.z;
+    r[6] = (float)(e0.x - e1.x + cx * A.x + cy * B.x);
+    r[7] = (float)(e0.y - e1.y + cx * A.y + cy * B.y);
+    r[8] = (float)(e0.z - e1.z + cx * A.z + cy * B.z);
+}
+
 // Spreads the entries' packed rows over the gradient arrays (every element is written, so none is cleared first)
-// and forms v_densify.  128 rows per CTA go through shared memory, so that both the reads and the writes of the
-// odd-sized arrays are coalesced; the pass moves its bytes once (HBM-bound).
+// and forms v_ray_transforms and v_densify.  128 rows per CTA go through shared memory, so that both the reads and
+// the writes of the odd-sized arrays are coalesced; the pass moves its bytes once (HBM-bound).
 template <int D, bool kGeo>
 __global__ void __launch_bounds__(128) unpack_grads_kernel(const tg_raster_bwd_args a) {
     using GS = GradSlots<D, kGeo>;
@@ -538,6 +569,14 @@ __global__ void __launch_bounds__(128) unpack_grads_kernel(const tg_raster_bwd_a
         d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
     }
     __syncthreads();
+    if ((int)threadIdx.x < n) {
+        const int64_t e = e0 + threadIdx.x;
+        const float* M = a.f.ray_transforms + 9 * e;
+        float* r = s + threadIdx.x * kPitch + GS::kM;
+        moments_to_transform(M, reinterpret_cast<const float2*>(a.f.means2d)[e], r);
+        reinterpret_cast<float2*>(a.v_densify)[e] = make_float2(r[2] * M[8], r[5] * M[8]);
+    }
+    __syncthreads();
     auto spread = [&](float* dst, int width, int off) {
         for (int k = threadIdx.x; k < n * width; k += kRows) dst[e0 * width + k] = s[(k / width) * kPitch + off + k % width];
     };
@@ -550,12 +589,6 @@ __global__ void __launch_bounds__(128) unpack_grads_kernel(const tg_raster_bwd_a
         if (a.v_means2d_abs) spread(a.v_means2d_abs, 2, GS::kAbs);
     } else {
         for (int k = threadIdx.x; k < n * 3; k += kRows) a.v_normals[e0 * 3 + k] = 0.f;
-    }
-    if ((int)threadIdx.x < n) {
-        const int64_t e = e0 + threadIdx.x;
-        const float depth = a.f.ray_transforms[9 * e + 8];
-        const float* r = s + threadIdx.x * kPitch + GS::kM;
-        reinterpret_cast<float2*>(a.v_densify)[e] = make_float2(r[2] * depth, r[5] * depth);
     }
 }
 

@@ -150,24 +150,16 @@ __device__ __forceinline__ void fwd_square(const tg_raster_fwd_args& a, const in
             uint32_t reach = 0u;
             if (idx < range_end) {
                 const int32_t g = a.flatten_ids[idx];
-                const float2 xy = reinterpret_cast<const float2*>(a.means2d)[g];
-                const int32_t row = a.gaussian_ids ? (int32_t)a.gaussian_ids[g] : g % a.N;
-                const float op = a.opacities[g];
-                const float* m = a.ray_transforms + 9 * (int64_t)g;
-                const float4 m0 = make_float4(m[0], m[1], m[2], xy.x), m1 = make_float4(m[3], m[4], m[5], xy.y),
-                             m2 = make_float4(m[6], m[7], m[8], op);
-                S.m0[slot] = m0;
-                S.m1[slot] = m1;
-                S.m2[slot] = m2;
-                const float* n = a.normals + 3 * (int64_t)g;
-                S.nrm[slot] = make_float4(n[0], n[1], n[2], __int_as_float(row));
-                const float* c = a.colors + (int64_t)g * D;
-                S.col[slot] = make_float4(c[0], D > 1 ? c[D > 1 ? 1 : 0] : 0.f, D > 2 ? c[D > 2 ? 2 : 0] : 0.f,
-                                          D > 3 ? c[D > 3 ? 3 : 0] : 0.f);
-                if constexpr (D == 5) S.col5[slot] = c[4];
-                if constexpr (FwdSmem<D, Tex>::kScale) S.scale[slot] = a.tex_scales[row];
-                reach = group_mask(make_float4(xy.x, xy.y, op, 1.f), m0, m1, m2, kTextured, a.range_x, a.range_y,
-                                   a.g_weight, !Filt::kAniso, X0, Y0, side);
+                const EntryRecord r = load_entry<D, true>(a, g);
+                S.m0[slot] = r.m0;
+                S.m1[slot] = r.m1;
+                S.m2[slot] = r.m2;
+                S.nrm[slot] = r.nrm;
+                S.col[slot] = r.col;
+                if constexpr (D == 5) S.col5[slot] = a.colors[(int64_t)g * D + 4];
+                if constexpr (FwdSmem<D, Tex>::kScale) S.scale[slot] = a.tex_scales[__float_as_int(r.nrm.w)];
+                reach = group_mask(make_float4(r.m0.w, r.m1.w, r.m2.w, 1.f), r.m0, r.m1, r.m2, kTextured, a.range_x,
+                                   a.range_y, a.g_weight, !Filt::kAniso, X0, Y0, side);
             }
             store_group_words(reach, S.words, n_words, slot >> 5, side);
         }
@@ -401,22 +393,14 @@ __device__ __forceinline__ void aniso_long_square(const tg_raster_fwd_args& a, c
             const int32_t idx = batch_start + slot;
             uint32_t reach = 0u;
             if (idx < range_end) {
-                const int32_t g = a.flatten_ids[idx];
-                const float2 xy = reinterpret_cast<const float2*>(a.means2d)[g];
-                const int32_t row = a.gaussian_ids ? (int32_t)a.gaussian_ids[g] : g % a.N;
-                const float op = a.opacities[g];
-                const float* m = a.ray_transforms + 9 * (int64_t)g;
-                const float4 m0 = make_float4(m[0], m[1], m[2], xy.x), m1 = make_float4(m[3], m[4], m[5], xy.y),
-                             m2 = make_float4(m[6], m[7], m[8], op);
-                S.m0[slot] = m0;
-                S.m1[slot] = m1;
-                S.m2[slot] = m2;
-                const float* n = a.normals + 3 * (int64_t)g;
-                S.nrm[slot] = make_float4(n[0], n[1], n[2], __int_as_float(row));
-                const float* c = a.colors + (int64_t)g * D;
-                S.col[slot] = make_float4(c[0], c[1], c[2], D > 3 ? c[D > 3 ? 3 : 0] : 0.f);
-                reach = group_mask(make_float4(xy.x, xy.y, op, 1.f), m0, m1, m2, true, a.range_x, a.range_y, a.g_weight,
-                                   false, X0, Y0, kAnisoSide);
+                const EntryRecord r = load_entry<D, true>(a, a.flatten_ids[idx]);
+                S.m0[slot] = r.m0;
+                S.m1[slot] = r.m1;
+                S.m2[slot] = r.m2;
+                S.nrm[slot] = r.nrm;
+                S.col[slot] = r.col;
+                reach = group_mask(make_float4(r.m0.w, r.m1.w, r.m2.w, 1.f), r.m0, r.m1, r.m2, true, a.range_x, a.range_y,
+                                   a.g_weight, false, X0, Y0, kAnisoSide);
             }
             store_group_words(reach, S.words, n_words, slot >> 5, kAnisoSide);
         }
@@ -638,6 +622,50 @@ cudaError_t launch_fwd_t(const tg_raster_fwd_args& a, cudaStream_t s) {
                                    : launch_fwd_kernel<D, Tex, false, FiltBilinear>(a, s);
 }
 
+// Packs the entries' records (see load_entry): a warp collects those of 32 entries in shared memory, reading every
+// array and writing the records in whole lines.
+template <int D>
+__global__ void __launch_bounds__(128) pack_entries_kernel(const tg_raster_fwd_args a) {
+    __shared__ float4 s4[4 * 32 * 5];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float* s = reinterpret_cast<float*>(s4 + warp * 32 * 5);
+    const int64_t e0 = ((int64_t)blockIdx.x * 4 + warp) * 32;
+    const int n = (int)min((int64_t)32, a.n_entries - e0);
+    if (n <= 0) return;  // (whole warps)
+    for (int i = lane; i < 9 * n; i += 32) s[(i / 9) * 20 + (i % 9) / 3 * 4 + i % 3] = a.ray_transforms[9 * e0 + i];
+    for (int i = lane; i < 3 * n; i += 32) s[(i / 3) * 20 + 16 + i % 3] = a.normals[3 * e0 + i];
+    for (int i = lane; i < D * n; i += 32)
+        if (i % D < 4) s[(i / D) * 20 + 12 + i % D] = a.colors[D * e0 + i];
+    if (lane < n) {
+        const int64_t e = e0 + lane;
+        const float2 xy = reinterpret_cast<const float2*>(a.means2d)[e];
+        float* r = s + lane * 20;
+        r[3] = xy.x;
+        r[7] = xy.y;
+        r[11] = a.opacities[e];
+        for (int k = D; k < 4; ++k) r[12 + k] = 0.f;
+        r[19] = __int_as_float(a.gaussian_ids ? (int)a.gaussian_ids[e] : (int)(e % a.N));
+    }
+    __syncwarp();
+    float4* dst = reinterpret_cast<float4*>(a.entry_records) + 5 * e0;
+    for (int i = lane; i < 5 * n; i += 32) dst[i] = reinterpret_cast<const float4*>(s)[i];
+}
+
+cudaError_t launch_pack_entries(const tg_raster_fwd_args& a, cudaStream_t s) {
+    if (a.entry_records == nullptr || a.n_entries == 0) return cudaSuccess;
+    const unsigned grid = (unsigned)((a.n_entries + 127) / 128);
+    switch (a.D) {
+        case 1: pack_entries_kernel<1><<<grid, 128, 0, s>>>(a); break;
+        case 2: pack_entries_kernel<2><<<grid, 128, 0, s>>>(a); break;
+        case 3: pack_entries_kernel<3><<<grid, 128, 0, s>>>(a); break;
+        case 4: pack_entries_kernel<4><<<grid, 128, 0, s>>>(a); break;
+        case 5: pack_entries_kernel<5><<<grid, 128, 0, s>>>(a); break;
+        default: return cudaErrorInvalidValue;
+    }
+    note_launches(1);
+    return cudaGetLastError();
+}
+
 template <class Tex>
 cudaError_t launch_fwd_d(const tg_raster_fwd_args& a, cudaStream_t s) {
     switch (a.D) {
@@ -661,6 +689,8 @@ cudaError_t launch_fwd_d34(const tg_raster_fwd_args& a, cudaStream_t s) {
 }
 
 cudaError_t launch_raster_fwd(const tg_raster_fwd_args& a, cudaStream_t s) {
+    const cudaError_t e = launch_pack_entries(a, s);
+    if (e != cudaSuccess) return e;
     switch (a.tex_format) {
         case TG_TEX_NONE: return launch_fwd_d<TexNone>(a, s);
         case TG_TEX_F32: return launch_fwd_d<TexF32>(a, s);

@@ -732,6 +732,8 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
         masks_buf = _contrib_masks(layout, isect_offsets, flatten_ids, tile_size, C, dev) if any(
             ctx.needs_input_grad) else None
         a.contrib_masks = B.ptr(masks_buf)
+        entries = _entry_records(means2d, flatten_ids)
+        a.entry_records, a.n_entries = B.ptr(entries), means2d.numel() // 2
         st = B.stream_of(means2d)
         prefix = _aniso_prefix(tex_store, tex_scales, st) if filter_code == B.TG_FILTER_ANISO_BILINEAR else None
         a.aniso_prefix = B.ptr(prefix)
@@ -756,6 +758,7 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
         ctx.aniso_prefix = prefix
         ctx.aniso_records = (records, counts)
         ctx.contrib_masks = masks_buf
+        ctx.entry_records = entries
         ctx.mark_non_differentiable(contrib_sum, contrib_count)
         ctx.set_materialize_grads(False)  # an output the loss does not use passes no gradient (NULL) to the adjoint
         return render_colors, render_alphas, render_normals, render_distort, render_median, contrib_sum, contrib_count
@@ -778,6 +781,7 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
                       0.0, g_weight, C, N, ctx.layout, ctx.n_isects_dev, *ctx.mip)
         f.t_checkpoints = B.ptr(ctx.t_checkpoints)
         f.contrib_masks = B.ptr(ctx.contrib_masks)
+        f.entry_records, f.n_entries = B.ptr(ctx.entry_records), means2d.numel() // 2
         f.aniso_prefix = B.ptr(ctx.aniso_prefix)
         if ctx.aniso_records[0] is not None:
             f.aniso_records, f.aniso_record_count = B.ptr(ctx.aniso_records[0]), B.ptr(ctx.aniso_records[1])
@@ -860,6 +864,24 @@ def _checkpoint_buffer(layout, isect_offsets, flatten_ids, tile_size, C, device)
 CONTRIB_MASK_BYTES = 8 << 30
 
 
+def _scratch(shape, dtype, device):
+    """An uninitialised tensor, or None where device memory does not allow it (the caller does without)."""
+    try:
+        return torch.empty(shape, dtype=dtype, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return None
+
+
+def _entry_records(means2d, flatten_ids):
+    """The entry_records scratch of tg_raster_fwd_args, or None where few of the entries are listed (less than one
+    listing in four entries: packing them all would cost more than gathering the listed ones) and for calls so small
+    that one launch more costs what the faster staging saves (10k entries: 4 us for 1)."""
+    E = means2d.numel() // 2
+    if E < 32768 or 4 * flatten_ids.numel() < E:
+        return None
+    return _scratch((E, 20), torch.float32, means2d.device)
+
+
 def _contrib_masks(layout, isect_offsets, flatten_ids, tile_size, C, device):
     """The contrib_masks buffer of tg_raster_fwd_args: [n_tiles + n_isects / 32 + 1, tile_size^2] int32, or None."""
     vt = None if layout is None else layout.get("view_table")
@@ -867,7 +889,7 @@ def _contrib_masks(layout, isect_offsets, flatten_ids, tile_size, C, device):
     rows = n_tiles + flatten_ids.numel() // 32 + 1
     if rows * tile_size * tile_size * 4 > CONTRIB_MASK_BYTES:
         return None
-    return torch.empty((rows, tile_size * tile_size), dtype=torch.int32, device=device)
+    return _scratch((rows, tile_size * tile_size), torch.int32, device)
 
 
 def _check_common(means2d, ray_transforms, colors, opacities, isect_offsets, tile_size, image_width, image_height,
