@@ -531,6 +531,33 @@ TG_API int tg_rasterize_bwd(const tg_raster_bwd_args* a, tg_stream_t stream);
 TG_API int tg_rotate_normals(const float* viewmats, int32_t C, const tg_view* views, int64_t view_pixels,
                              int64_t n_pixels, int32_t transpose, const float* in, float* out, tg_stream_t stream);
 
+/* ------------------------------------------------------------------ depth images
+ * The last step of the depth render modes (textured_gaussians/rendering.py:1296-1313,
+ * utils.py:81-168).  With `alphas` (and out_colors) the last of the D channels is
+ * divided by max(alpha, 1e-10).  out_normals ([C,H,W,3], or NULL): world-space
+ * normals of `depth` ([C,H,W]) or, where that is NULL, of the (divided) last
+ * channel, zero on the border; needs camtoworlds ([C,4,4]) and Ks ([C,3,3]),
+ * C <= 65535.  The adjoint takes the same inputs, the upstream gradients (either
+ * may be NULL: zero) and writes v_colors, v_alphas (with alphas) and v_depth
+ * (with depth), each if non-NULL. */
+typedef struct {
+    int32_t C, width, height, D;
+    const float* colors;       /* [C,H,W,D] */
+    const float* alphas;       /* [C,H,W] or NULL: no division */
+    const float* depth;        /* [C,H,W] or NULL */
+    const float* camtoworlds;
+    const float* Ks;
+    float* out_colors;         /* [C,H,W,D] or NULL */
+    float* out_normals;
+    const float* v_out_colors;
+    const float* v_normals;
+    float* v_colors;
+    float* v_alphas;
+    float* v_depth;
+} tg_depth_image_args;
+TG_API int tg_depth_image_fwd(const tg_depth_image_args* a, tg_stream_t stream);
+TG_API int tg_depth_image_bwd(const tg_depth_image_args* a, tg_stream_t stream);
+
 /* ------------------------------------------------------------------ spherical harmonics
  * Replaces compute_sh_fwd_tensor / compute_sh_bwd_tensor
  * (textured_gaussians/cuda/csrc/compute_sh_fwd.cu, compute_sh_bwd.cu).

@@ -95,6 +95,12 @@ class RasterBwdArgs(ctypes.Structure):
                 ("v_aniso_prefix", P), ("v_packed", P)]
 
 
+class DepthImageArgs(ctypes.Structure):
+    _fields_ = [("C", I32), ("width", I32), ("height", I32), ("D", I32), ("colors", P), ("alphas", P), ("depth", P),
+                ("camtoworlds", P), ("Ks", P), ("out_colors", P), ("out_normals", P), ("v_out_colors", P),
+                ("v_normals", P), ("v_colors", P), ("v_alphas", P), ("v_depth", P)]
+
+
 _lib = None
 _lock = threading.Lock()
 
@@ -138,6 +144,8 @@ def lib() -> ctypes.CDLL:
                 ("tg_generate_mipmap_bwd", [P, P, I64, I32, P]),
                 ("tg_aniso_prefix", [P, I32, P, I64, I32, I32, P, P]),
                 ("tg_rotate_normals", [P, I32, P, I64, I64, I32, P, P, P]),
+                ("tg_depth_image_fwd", [ctypes.POINTER(DepthImageArgs), P]),
+                ("tg_depth_image_bwd", [ctypes.POINTER(DepthImageArgs), P]),
                 ("tg_sh_bwd", [I64, I64, I32, I32, P, P, P, P, P, P, P]),
             ]:
                 fn = getattr(L, name)

@@ -61,6 +61,7 @@ cudaError_t launch_aniso_prefix_fold(const float* v_prefix, int64_t G, int ry, i
                                      cudaStream_t s);
 cudaError_t launch_rotate_normals(const float* viewmats, int C, const tg_view* views, int64_t view_pixels,
                                   int64_t n_pixels, int transpose, const float* in, float* out, cudaStream_t s);
+cudaError_t launch_depth_image(const tg_depth_image_args& a, bool adjoint, cudaStream_t s);
 int fail_with(int code, const char* msg);
 }  // namespace tg
 
@@ -566,6 +567,32 @@ int tg_rotate_normals(const float* viewmats, int32_t C, const tg_view* views, in
     TG_REQUIRE(viewmats && in && out, TG_ERR_INVALID_ARG, "null pointer");
     return cuda_status(tg::launch_rotate_normals(viewmats, C, views, view_pixels, n_pixels, transpose, in, out, stream),
                        "tg_rotate_normals");
+}
+
+namespace {
+int check_depth_image(const tg_depth_image_args* a) {
+    TG_REQUIRE(a != nullptr, TG_ERR_INVALID_ARG, "null args");
+    TG_REQUIRE(a->C >= 0 && a->C <= 65535 && a->width >= 0 && a->height >= 0 && a->D >= 1, TG_ERR_INVALID_ARG,
+               "bad sizes");
+    if ((int64_t)a->C * a->width * a->height == 0) return TG_OK;
+    TG_REQUIRE(a->colors, TG_ERR_INVALID_ARG, "null colors");
+    TG_REQUIRE((!a->out_normals && !a->v_normals) || (a->camtoworlds && a->Ks), TG_ERR_INVALID_ARG,
+               "depth normals need camtoworlds and Ks");
+    return TG_OK;
+}
+}  // namespace
+
+int tg_depth_image_fwd(const tg_depth_image_args* a, tg_stream_t stream) {
+    const int rc = check_depth_image(a);
+    if (rc != TG_OK || (int64_t)a->C * a->width * a->height == 0) return rc;
+    TG_REQUIRE(a->out_colors == nullptr || a->alphas, TG_ERR_INVALID_ARG, "out_colors needs alphas");
+    return cuda_status(tg::launch_depth_image(*a, false, stream), "tg_depth_image_fwd");
+}
+
+int tg_depth_image_bwd(const tg_depth_image_args* a, tg_stream_t stream) {
+    const int rc = check_depth_image(a);
+    if (rc != TG_OK || (int64_t)a->C * a->width * a->height == 0) return rc;
+    return cuda_status(tg::launch_depth_image(*a, true, stream), "tg_depth_image_bwd");
 }
 
 int tg_sh_fwd(int64_t n, int64_t coeff_rows, int32_t degree, int32_t K, const float* dirs, const float* coeffs,

@@ -1119,6 +1119,62 @@ def normals_to_world(normals: Tensor, viewmats: Tensor, view_table=None) -> Tens
     return _RotateNormals.apply(normals, viewmats.contiguous(), view_table.views, max(view_table.pix_count), 0)
 
 
+# --------------------------------------------------------------------------- depth images
+class _DepthImage(torch.autograd.Function):
+    """(colours with the expected depth, or None; world-space normals of the depth image, or None)."""
+
+    @staticmethod
+    def forward(ctx, colors, alphas, depth, camtoworlds, Ks):
+        x, al = (None if t is None else t.contiguous() for t in (colors, alphas))
+        # a copy of what the adjoint reads again and the caller holds (the compositor keeps colours and opacities itself)
+        z = None if depth is None else depth.clone(memory_format=torch.contiguous_format)
+        out = None if al is None else torch.empty_like(x)
+        normals = None if camtoworlds is None else x.new_empty(x.shape[:-1] + (3,))
+        ctx.save_for_backward(x, al, z, camtoworlds, Ks)
+        ctx.set_materialize_grads(False)
+        C, H, W, D = x.shape
+        a = B.DepthImageArgs(C, W, H, D, B.ptr(x), B.ptr(al), B.ptr(z), B.ptr(camtoworlds), B.ptr(Ks), B.ptr(out),
+                             B.ptr(normals))
+        st = B.stream_of(x)
+        B.call("tg_depth_image_fwd", st, B.lib().tg_depth_image_fwd, ctypes.byref(a), st)
+        return out, normals
+
+    @staticmethod
+    def backward(ctx, v_out, v_normals):
+        if v_out is None and v_normals is None:
+            return (None,) * 5
+        x, al, z, camtoworlds, Ks = ctx.saved_tensors
+        v_out, v_normals = (None if t is None else t.contiguous() for t in (v_out, v_normals))
+        v_x = torch.empty_like(x) if ctx.needs_input_grad[0] else None
+        v_al = torch.empty_like(al) if al is not None else None
+        v_z = torch.empty_like(z) if z is not None and ctx.needs_input_grad[2] else None
+        if v_x is None and al is not None:  # (the opacities' gradient is written beside the colours')
+            v_x = torch.empty_like(x)
+        C, H, W, D = x.shape
+        a = B.DepthImageArgs(C, W, H, D, B.ptr(x), B.ptr(al), B.ptr(z), B.ptr(camtoworlds), B.ptr(Ks), None, None,
+                             B.ptr(v_out), B.ptr(v_normals), B.ptr(v_x), B.ptr(v_al), B.ptr(v_z))
+        st = B.stream_of(x)
+        B.call("tg_depth_image_bwd", st, B.lib().tg_depth_image_bwd, ctypes.byref(a), st)
+        return v_x, v_al, v_z, None, None
+
+
+def depth_image_supported(colors: Tensor, viewmats: Tensor, Ks: Tensor) -> bool:
+    """Whether :func:`depth_image` takes these: FP32, cameras without gradients, images of at least 2x2 pixels (the
+    tensor expressions give smaller ones a border of their own shape) and at most 65535 views."""
+    return (colors.dim() == 4 and colors.dtype == viewmats.dtype == Ks.dtype == torch.float32 and
+            not viewmats.requires_grad and not Ks.requires_grad and
+            min(colors.shape[1:3]) >= 2 and colors.shape[0] <= 65535)
+
+
+def depth_image(colors: Tensor, alphas: Optional[Tensor], depth: Optional[Tensor] = None,
+                camtoworlds: Optional[Tensor] = None, Ks: Optional[Tensor] = None):
+    """Last step of the depth render modes on images [C,H,W,D]: with ``alphas`` the last channel over
+    max(alpha, 1e-10), and with ``camtoworlds`` world-space normals [C,H,W,3] of ``depth`` [C,H,W,1], or of the last
+    channel where that is None."""
+    cam = (None, None) if camtoworlds is None else (camtoworlds.contiguous(), Ks.contiguous())
+    return _DepthImage.apply(colors, alphas, depth, *cam)
+
+
 # --------------------------------------------------------------------------- gradient consumers
 _SHADOW_FORMAT = {None: B.TG_TEX_NONE, torch.bfloat16: B.TG_TEX_BF16, torch.float16: B.TG_TEX_F16}
 

@@ -36,6 +36,8 @@ import torch
 from torch import Tensor
 
 from .cuda._wrapper import (
+    depth_image,
+    depth_image_supported,
     fully_fused_projection_2dgs,
     isect_offset_encode,
     isect_tiles,
@@ -134,10 +136,18 @@ def _prepare(means, quats, scales, opacities, colors, viewmats, Ks, width, heigh
 def _finish(p, render_colors, render_alphas, render_normals, render_distort, render_median, gs_contrib_sum,
             gs_contrib_count, viewmats, Ks, width, height, tile_size, render_mode, depth_mode):
     render_normals_from_depth = None
-    if render_mode in ["ED", "RGB+ED"]:
+    expected, with_normals = render_mode in ["ED", "RGB+ED"], render_mode in ["RGB+ED", "RGB+D"]
+    if (expected or with_normals) and depth_image_supported(render_colors, viewmats, Ks):
+        cam = (_inverse(viewmats), Ks) if with_normals else ()
+        out, n = depth_image(render_colors, render_alphas if expected else None,
+                             None if depth_mode == "expected" else render_median, *cam)
+        render_colors = out if expected else render_colors
+        render_normals_from_depth = n.squeeze(0) if with_normals else None
+        expected = with_normals = False
+    if expected:
         render_colors = torch.cat(
             [render_colors[..., :-1], render_colors[..., -1:] / render_alphas.clamp(min=1e-10)], dim=-1)
-    if render_mode in ["RGB+ED", "RGB+D"]:
+    if with_normals:
         depth_for_normal = render_colors[..., -1:] if depth_mode == "expected" else render_median
         render_normals_from_depth = depth_to_normal(depth_for_normal, _inverse(viewmats), Ks).squeeze(0)
     meta = {
