@@ -75,6 +75,20 @@ def test_packed_projection_matches_dense_entries_bit_exact(make):
         s.near_plane, s.far_plane, 0.0)[1][sel[:, 0], sel[:, 1]])
 
 
+# The packed passes give a CTA 256 entries of a camera row up to 2 x 592 CTAs' worth over all cameras, multiples of 256
+# beyond, 4096 from 2,424,832 entries on; ragged ends on both sides of each line.
+@pytest.mark.parametrize("N", [1, 255, 257, 101_034, 101_035, 808_277, 808_609])
+def test_packed_projection_chunk_sizes(N):
+    s = scenes.mixture1m(N=N, R=1, n_cams=3, width=320, height=240, radius=25.0)
+    args = (T(s.viewmats), T(s.Ks), s.width, s.height, 0.3, s.near_plane, s.far_plane, 0.0)
+    dense = fully_fused_projection_2dgs(T(s.means), T(s.quats), T(s.scales), *args)
+    packed = fully_fused_projection_2dgs(T(s.means), T(s.quats), T(s.scales), *args, packed=True)
+    sel = (dense[0] > 0).nonzero()
+    assert torch.equal(packed[0], sel[:, 0]) and torch.equal(packed[1], sel[:, 1])
+    for d, p in zip(dense, packed[2:]):
+        assert torch.equal(d[sel[:, 0], sel[:, 1]], p)
+
+
 def test_packed_projection_empty_and_indptr():
     s = scene3()
     # near plane beyond every Gaussian: nnz = 0

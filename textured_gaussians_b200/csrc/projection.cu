@@ -300,8 +300,16 @@ __global__ void __launch_bounds__(32 * kProjWarps<NB>, 6) project_fwd_kernel(tg_
 
 // ------------------------------------------------------------------ packed forward
 constexpr int kPackThreads = 256;
-constexpr int kPackItems = 16;
-constexpr int kPackChunk = kPackThreads * kPackItems;  // entries of one camera row per CTA
+constexpr int kPackMaxItems = 16;
+constexpr int kPackCtas = 4 * 148;
+
+// Entries of one camera row per CTA, in units of 256.  Both passes are latency-bound a CTA (means, rotations, scales,
+// then an SH row per visible entry), so up to four CTAs an SM the entries are spread over more of them rather than
+// looped over; beyond, the chunks grow to 4096, which keeps the single-CTA scan of their counts short.  Emitting
+// 150,000 entries of degree 3 (37 CTAs of 4096, now 586 of 256): 105 -> 25 us; 1,200,000 of degree 0: 74 -> 44 us.
+inline int pack_items(int64_t C, int64_t len) {
+    return (int)std::min<int64_t>(std::max<int64_t>(C * len / ((int64_t)kPackThreads * kPackCtas), 1), kPackMaxItems);
+}
 
 // Row of camera c: Gaussians [g0, g0 + len) (all N, or the camera's scene in
 // the batching form, clamped to [0, N)) and its image size.
@@ -326,14 +334,14 @@ __device__ __forceinline__ PackRow pack_row(const tg_project_packed_args& a, int
 
 // Pass 1: number of visible entries in each chunk (blockIdx.x) of camera blockIdx.y.
 __global__ void __launch_bounds__(kPackThreads) project_packed_count_kernel(tg_project_packed_args a,
-                                                                           int64_t* chunk_counts) {
+                                                                           int items, int64_t* chunk_counts) {
     __shared__ int64_t s_warp[kPackThreads / 32];
     const int c = blockIdx.y;
     const PackRow row = pack_row(a, c);
-    const int64_t base = (int64_t)blockIdx.x * kPackChunk;
+    const int64_t base = (int64_t)blockIdx.x * items * kPackThreads;
     int64_t local = 0;
 #pragma unroll 1
-    for (int i = 0; i < kPackItems; ++i) {
+    for (int i = 0; i < items; ++i) {
         const int64_t k = base + (int64_t)i * kPackThreads + threadIdx.x;
         if (k >= row.len) break;
         Projected o;
@@ -358,16 +366,16 @@ __global__ void packed_indptr_kernel(const int64_t* chunk_offsets, const int64_t
 // warp ballot plus a CTA prefix over warps, and write them at chunk offset +
 // rank, so entries keep (camera, Gaussian) order.
 template <int NB>
-__global__ void __launch_bounds__(kPackThreads) project_packed_emit_kernel(tg_project_packed_args a,
+__global__ void __launch_bounds__(kPackThreads) project_packed_emit_kernel(tg_project_packed_args a, int items,
                                                                           const int64_t* chunk_offsets) {
     __shared__ int32_t s_warp[kPackThreads / 32];
     const int c = blockIdx.y;
     const PackRow row = pack_row(a, c);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t base = (int64_t)blockIdx.x * kPackChunk;
+    const int64_t base = (int64_t)blockIdx.x * items * kPackThreads;
     int64_t run = chunk_offsets[(int64_t)c * gridDim.x + blockIdx.x];
 #pragma unroll 1
-    for (int i = 0; i < kPackItems; ++i) {
+    for (int i = 0; i < items; ++i) {
         const int64_t slice = base + (int64_t)i * kPackThreads;
         if (slice >= row.len) break;  // uniform across the CTA
         const int64_t k = slice + threadIdx.x;
@@ -676,27 +684,34 @@ cudaError_t launch_project_bwd(const tg_project_bwd_args& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-size_t project_packed_workspace_bytes(int32_t C, int32_t N) {
-    const int64_t chunks = (int64_t)std::max(C, 0) * (((int64_t)std::max(N, 0) + kPackChunk - 1) / kPackChunk);
-    return align256(sizeof(int64_t) * (size_t)std::max<int64_t>(chunks, 1));
+// Chunks per camera row, for rows of at most len entries.
+inline int64_t packed_chunks_per_row(int64_t C, int64_t len) {
+    const int64_t chunk = (int64_t)kPackThreads * pack_items(C, len);
+    return (len + chunk - 1) / chunk;
+}
+inline int64_t packed_row_len(const tg_project_packed_args& a) {
+    return a.gauss_ranges ? std::min<int64_t>(a.max_range, a.N) : a.N;
 }
 
-// Chunks per camera row: the longest row over 4096.
-inline int64_t packed_chunks_per_row(const tg_project_packed_args& a) {
-    const int64_t len = a.gauss_ranges ? std::min<int64_t>(a.max_range, a.N) : a.N;
-    return (len + kPackChunk - 1) / kPackChunk;
+// One count per chunk, for the longest rows (C, N) allow or any shorter ones: a row has at most one partial chunk,
+// and whole ones number less than 2 kPackCtas in all, or one per 4096 entries where the chunks have that size.
+size_t project_packed_workspace_bytes(int32_t C, int32_t N) {
+    const int64_t c = std::max(C, 0), n = std::max(N, 0);
+    const int64_t whole = std::max<int64_t>(2 * kPackCtas, c * n / (kPackThreads * kPackMaxItems));
+    return align256(sizeof(int64_t) * (size_t)(c + std::min(whole, c * n / kPackThreads) + 1));
 }
 
 // Count pass: chunk counts, their scan (-> *nnz), indptr.  Three launches.
 cudaError_t launch_project_packed_count(const tg_project_packed_args& a, cudaStream_t s) {
-    const int64_t per_row = packed_chunks_per_row(a);
+    const int64_t len = packed_row_len(a), per_row = packed_chunks_per_row(a.C, len);
+    const int items = pack_items(a.C, len);
     if ((int64_t)a.C * per_row == 0) {
         cudaError_t e = cudaMemsetAsync(a.nnz, 0, sizeof(int64_t), s);
         if (e == cudaSuccess) e = cudaMemsetAsync(a.indptr, 0, sizeof(int32_t) * ((size_t)a.C + 1), s);
         return e;
     }
     int64_t* chunk = static_cast<int64_t*>(a.workspace);
-    project_packed_count_kernel<<<dim3((unsigned)per_row, (unsigned)a.C), kPackThreads, 0, s>>>(a, chunk);
+    project_packed_count_kernel<<<dim3((unsigned)per_row, (unsigned)a.C), kPackThreads, 0, s>>>(a, items, chunk);
     note_launches(1);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
@@ -709,17 +724,18 @@ cudaError_t launch_project_packed_count(const tg_project_packed_args& a, cudaStr
 
 // Emit pass; the chunk offsets left in the workspace by the count pass are reused.
 cudaError_t launch_project_packed_emit(const tg_project_packed_args& a, cudaStream_t s) {
-    const int64_t per_row = packed_chunks_per_row(a);
+    const int64_t len = packed_row_len(a), per_row = packed_chunks_per_row(a.C, len);
+    const int items = pack_items(a.C, len);
     if ((int64_t)a.C * per_row == 0 || a.nnz_host == 0) return cudaSuccess;
     const dim3 grid((unsigned)per_row, (unsigned)a.C);
     const int64_t* chunk = static_cast<const int64_t*>(a.workspace);
     switch (a.sh_coeffs ? a.sh_degree : -1) {
-        case 0: project_packed_emit_kernel<1><<<grid, kPackThreads, 0, s>>>(a, chunk); break;
-        case 1: project_packed_emit_kernel<4><<<grid, kPackThreads, 0, s>>>(a, chunk); break;
-        case 2: project_packed_emit_kernel<9><<<grid, kPackThreads, 0, s>>>(a, chunk); break;
-        case 3: project_packed_emit_kernel<16><<<grid, kPackThreads, 0, s>>>(a, chunk); break;
-        case 4: project_packed_emit_kernel<25><<<grid, kPackThreads, 0, s>>>(a, chunk); break;
-        default: project_packed_emit_kernel<0><<<grid, kPackThreads, 0, s>>>(a, chunk); break;
+        case 0: project_packed_emit_kernel<1><<<grid, kPackThreads, 0, s>>>(a, items, chunk); break;
+        case 1: project_packed_emit_kernel<4><<<grid, kPackThreads, 0, s>>>(a, items, chunk); break;
+        case 2: project_packed_emit_kernel<9><<<grid, kPackThreads, 0, s>>>(a, items, chunk); break;
+        case 3: project_packed_emit_kernel<16><<<grid, kPackThreads, 0, s>>>(a, items, chunk); break;
+        case 4: project_packed_emit_kernel<25><<<grid, kPackThreads, 0, s>>>(a, items, chunk); break;
+        default: project_packed_emit_kernel<0><<<grid, kPackThreads, 0, s>>>(a, items, chunk); break;
     }
     note_launches(1);
     if (a.overflow) {
