@@ -271,9 +271,10 @@ TG_API int tg_isect_emit(const tg_isect_args* a, tg_stream_t stream);
  * stably by the 32 + tile_bits + camera_bits low key bits): the entries are
  * sorted by depth, and the intersections, written in that order, by camera and
  * tile alone.
- * tg_isect_sorted_count: tiles_per_gauss, *n_isects and the entries' order
- * (left in order_ws); needs depths, not cum_tiles or scan_workspace.
- * tg_isect_sorted_lists: isect_ids and flatten_ids [n], n = *n_isects; in
+ * tg_isect_sorted_count: tiles_per_gauss and *n_isects (and, in order_ws, what
+ * the second call starts from); needs depths, not cum_tiles or scan_workspace.
+ * tg_isect_sorted_lists: the entries' order, then isect_ids and flatten_ids [n],
+ * n = *n_isects, from the same inputs and the counts of the first call; in
  * capacity mode (overflow != NULL) n = capacity and the tail as described at
  * `capacity`.  order_ws: what tg_isect_sorted_count filled, of
  * tg_isect_sorted_order_bytes(n_elems) bytes; list_ws:

@@ -388,8 +388,8 @@ int tg_isect_sorted_lists(const tg_isect_args* a, void* order_ws, int64_t n, voi
                "bad tile grid");
     TG_REQUIRE(a->isect_ids && a->flatten_ids, TG_ERR_INVALID_ARG, "null pointer");
     if (a->n_elems > 0)
-        TG_REQUIRE(a->means2d && a->radii && a->depths && order_ws && (a->camera_ids || a->N > 0), TG_ERR_INVALID_ARG,
-                   "null pointer");
+        TG_REQUIRE(a->means2d && a->radii && a->depths && a->tiles_per_gauss && order_ws && (a->camera_ids || a->N > 0),
+                   TG_ERR_INVALID_ARG, "null pointer");
     TG_REQUIRE(list_ws && aligned(list_ws, 16) && list_bytes >= tg::isect_lists_workspace_bytes(n, tb + cb),
                TG_ERR_WORKSPACE, "list workspace missing, misaligned or smaller than %zu bytes",
                tg::isect_lists_workspace_bytes(n, tb + cb));

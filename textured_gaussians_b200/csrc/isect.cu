@@ -401,7 +401,7 @@ struct OrderWorkspace {
     uint32_t* counter;  // [4] tiles taken, then the error flag
     uint32_t* status;   // [4][tiles][256]
     uint32_t *keys[2], *ids[2];  // ping-pong; the depth order ends in ids[1]
-    int64_t* chunks;    // [chunks + 1] intersections before each chunk of the depth order
+    int64_t* chunks;    // [chunks] intersections before each chunk of the depth order
     size_t zeroed, bytes;
 };
 inline OrderWorkspace carve_order_workspace(void* base, int64_t E) {
@@ -420,7 +420,7 @@ inline OrderWorkspace carve_order_workspace(void* base, int64_t E) {
     w.zeroed = off;
     for (int i = 0; i < 2; ++i) w.keys[i] = reinterpret_cast<uint32_t*>(take(4 * (size_t)(tiles ? E : 0)));
     for (int i = 0; i < 2; ++i) w.ids[i] = reinterpret_cast<uint32_t*>(take(4 * (size_t)(tiles || i ? E : 0)));
-    w.chunks = reinterpret_cast<int64_t*>(take(8 * ((E + kOrderChunk - 1) / kOrderChunk + 1)));
+    w.chunks = reinterpret_cast<int64_t*>(take(8 * ((E + kOrderChunk - 1) / kOrderChunk)));
     w.bytes = off;
     return w;
 }
@@ -438,9 +438,15 @@ __device__ __forceinline__ void count_digit(uint32_t* s, uint32_t d, bool ok) {
     }
 }
 
-// Tile counts of the entries, and the digit counts of their depths.
-__global__ void __launch_bounds__(256) order_count_kernel(tg_isect_args a, uint32_t* hist) {
+// Tile counts of the entries, their sum (added to the zeroed *n_isects), and the digit counts of their depths.  The
+// host waits for the sum alone: the entries' sort comes after its read, so a small call does not wait for it (35 us
+// of a 376 us frame, now 348; a plain training step of 150,000 splats 1774 -> 1687 us), and a large one is the same
+// (1,000,000 entries: 311 us).  Eight CTAs an SM: at 36 registers the 977 CTAs of a million entries need a second
+// wave (18.9 -> 25.1 us).
+__global__ void __launch_bounds__(256, 8) order_count_kernel(tg_isect_args a, uint32_t* hist) {
     __shared__ uint32_t s_hist[kDepthPasses * kRadix];
+    __shared__ int64_t s_warp[256 / 32];
+    int64_t local = 0;
     if (hist != nullptr) {
         for (int i = threadIdx.x; i < kDepthPasses * kRadix; i += 256) s_hist[i] = 0;
         __syncthreads();
@@ -461,6 +467,7 @@ __global__ void __launch_bounds__(256) order_count_kernel(tg_isect_args a, uint3
                 cnt = (int32_t)((y1 - y0) * (x1 - x0));
             }
             a.tiles_per_gauss[e] = cnt;
+            local += cnt;
         }
         if (hist != nullptr) {
             const uint32_t k = in ? __float_as_uint(a.depths[e]) : 0u;
@@ -468,9 +475,12 @@ __global__ void __launch_bounds__(256) order_count_kernel(tg_isect_args a, uint3
             for (int p = 0; p < kDepthPasses; ++p) count_digit(s_hist + p * kRadix, (k >> (8 * p)) & 0xffu, in);
         }
     }
+    int64_t sum;
+    block_excl_scan(local, s_warp, sum);
+    if (threadIdx.x == 0 && sum != 0)
+        atomicAdd(reinterpret_cast<unsigned long long*>(a.n_isects), (unsigned long long)sum);
     if (hist == nullptr) return;
-    __syncthreads();
-    for (int i = threadIdx.x; i < kDepthPasses * kRadix; i += 256)
+    for (int i = threadIdx.x; i < kDepthPasses * kRadix; i += 256)  // (the scan above is a barrier)
         if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
 }
 
@@ -494,12 +504,38 @@ __global__ void __launch_bounds__(kSortThreads, 4) order_pass_kernel(const float
         n, 8 * pass, 8, hist, status, counter, error);
 }
 
-// The whole entry order by one CTA, for n <= kSmallSort.
-__global__ void __launch_bounds__(kSmallThreads) order_small_kernel(const float* __restrict__ depths, int n,
-                                                                    uint32_t* __restrict__ ids) {
+// The whole entry order and its chunk offsets by one CTA, for n <= kSmallSort (entries without tiles anywhere).
+__global__ void __launch_bounds__(kSmallThreads) order_small_kernel(const float* __restrict__ depths,
+                                                                    const int32_t* __restrict__ counts, int n,
+                                                                    uint32_t* __restrict__ ids, int64_t* chunks) {
+    static_assert(kSmallThreads == kOrderChunk && kSmallItems <= 32, "item i of all threads is chunk i");
+    __shared__ int64_t s_part[kSmallItems][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, items = (n + kSmallThreads - 1) / kSmallThreads;
     uint32_t *s_keys, *s_idx;
-    sort_small([&](int i) { return __float_as_uint(depths[i]); }, n, 32, s_keys, s_idx);
-    for (int i = threadIdx.x; i < n; i += kSmallThreads) ids[i] = s_idx[i];
+    sort_small(
+        [&](int i, bool& matters) {
+            matters = counts[i] > 0;
+            return __float_as_uint(depths[i]);
+        },
+        n, 32, s_keys, s_idx);
+    for (int c = 0; c < items; ++c) {
+        const int i = c * kSmallThreads + threadIdx.x;
+        int64_t v = 0;
+        if (i < n) {
+            const uint32_t id = s_idx[i];
+            ids[i] = id;
+            v = counts[id];
+        }
+        v = warp_incl_scan(v);
+        if (lane == 31) s_part[c][warp] = v;
+    }
+    __syncthreads();
+    if (warp != 0) return;
+    int64_t v = 0;
+    if (lane < items)
+        for (int w = 0; w < 32; ++w) v += s_part[lane][w];
+    const int64_t incl = warp_incl_scan(v);
+    if (lane < items) chunks[lane] = incl - v;
 }
 
 // Intersections of each chunk of the depth order.
@@ -518,9 +554,8 @@ __global__ void __launch_bounds__(256) order_sums_kernel(const uint32_t* __restr
     if (threadIdx.x == 0) chunks[blockIdx.x] = total;
 }
 
-// Exclusive scan of the chunk sums by one CTA of 1024 threads, four sums each; the total goes to chunks[n_chunks]
-// and *n_total.
-__global__ void __launch_bounds__(1024) order_scan_kernel(int64_t* chunks, int64_t n_chunks, int64_t* n_total) {
+// Exclusive scan of the chunk sums by one CTA of 1024 threads, four sums each.
+__global__ void __launch_bounds__(1024) order_scan_kernel(int64_t* chunks, int64_t n_chunks) {
     __shared__ int64_t s_warp[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int64_t carry = 0;
@@ -546,27 +581,33 @@ __global__ void __launch_bounds__(1024) order_scan_kernel(int64_t* chunks, int64
         carry += s_warp[31];
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        chunks[n_chunks] = carry;
-        *n_total = carry;
-    }
 }
 
+// Counts of the entries' tiles and their sum.
 cudaError_t launch_isect_order(const tg_isect_args& a, void* workspace, cudaStream_t s) {
     const int64_t E = a.n_elems;
-    if (E == 0) return cudaMemsetAsync(a.n_isects, 0, sizeof(int64_t), s);
+    cudaError_t e = cudaMemsetAsync(a.n_isects, 0, sizeof(int64_t), s);
+    if (e != cudaSuccess || E == 0) return e;
     const OrderWorkspace w = carve_order_workspace(workspace, E);
     const int64_t chunks = (E + kOrderChunk - 1) / kOrderChunk;
     const bool small = E <= kSmallSort;
-    cudaError_t e = cudaSuccess;
     if (!small && (e = cudaMemsetAsync(workspace, 0, w.zeroed, s)) != cudaSuccess) return e;
     order_count_kernel<<<(unsigned)chunks, 256, 0, s>>>(a, small ? nullptr : w.hist);
-    if (small) {
+    note_launches(1);
+    return cudaGetLastError();
+}
+
+// The entries by depth and the offsets of its chunks.
+cudaError_t launch_entry_sort(const tg_isect_args& a, const OrderWorkspace& w, cudaStream_t s) {
+    const int64_t E = a.n_elems, chunks = (E + kOrderChunk - 1) / kOrderChunk;
+    cudaError_t e;
+    if (E <= kSmallSort) {
         if ((e = cudaFuncSetAttribute(order_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)kSmallSmem)) != cudaSuccess)
             return e;
-        order_small_kernel<<<1, kSmallThreads, kSmallSmem, s>>>(a.depths, (int)E, w.ids[1]);
-        note_launches(2);
+        order_small_kernel<<<1, kSmallThreads, kSmallSmem, s>>>(a.depths, a.tiles_per_gauss, (int)E, w.ids[1],
+                                                                w.chunks);
+        note_launches(1);
     } else {
         constexpr size_t smem = sort_pass_smem<uint32_t>();
         if ((e = cudaFuncSetAttribute(order_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
@@ -577,11 +618,10 @@ cudaError_t launch_isect_order(const tg_isect_args& a, void* workspace, cudaStre
             order_pass_kernel<<<(unsigned)tiles, kSortThreads, smem, s>>>(
                 a.depths, w.keys[(p + 1) & 1], w.ids[(p + 1) & 1], w.keys[p & 1], w.ids[p & 1], E, p,
                 w.hist + p * kRadix, w.status + (size_t)p * tiles * kRadix, w.counter + p, w.counter + kDepthPasses);
-        note_launches(1 + kDepthPasses);
+        order_sums_kernel<<<(unsigned)chunks, 256, 0, s>>>(w.ids[1], a.tiles_per_gauss, E, w.chunks);
+        order_scan_kernel<<<1, 1024, 0, s>>>(w.chunks, chunks);
+        note_launches(kDepthPasses + 2);
     }
-    order_sums_kernel<<<(unsigned)chunks, 256, 0, s>>>(w.ids[1], a.tiles_per_gauss, E, w.chunks);
-    order_scan_kernel<<<1, 1024, 0, s>>>(w.chunks, chunks, a.n_isects);
-    note_launches(2);
     return cudaGetLastError();
 }
 
@@ -782,6 +822,7 @@ cudaError_t launch_isect_lists(const tg_isect_args& a, void* order_ws, int64_t n
     cudaError_t e = cudaMemsetAsync(ws, 0, w.zeroed, s);
     if (e != cudaSuccess) return e;
     if (E > 0) {
+        if ((e = launch_entry_sort(a, o, s)) != cudaSuccess) return e;
         isect_expand_kernel<<<(unsigned)((E + kOrderChunk - 1) / kOrderChunk), 256, 0, s>>>(
             a, o.ids[1], o.chunks, n, tile_bits, passes, pass_bits, w.keys[0], w.ids[0], w.hist);
         note_launches(1);
@@ -825,8 +866,8 @@ __global__ void __launch_bounds__(kSmallThreads) tile_order_small_kernel(const i
                                                                          int64_t n_isects, const int64_t* n_dev,
                                                                          uint32_t bound, int end_bit, int32_t* order) {
     uint32_t *s_keys, *s_idx;
-    sort_small([&](int i) { return tile_key(offsets, i, n_tiles, n_isects, n_dev, bound); }, n_tiles, end_bit, s_keys,
-               s_idx);
+    sort_small([&](int i, bool&) { return tile_key(offsets, i, n_tiles, n_isects, n_dev, bound); }, n_tiles, end_bit,
+               s_keys, s_idx);
     for (int i = threadIdx.x; i < n_tiles; i += kSmallThreads) order[i] = (int32_t)s_idx[i];
 }
 
