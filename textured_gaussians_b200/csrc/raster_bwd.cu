@@ -249,24 +249,22 @@ __device__ __forceinline__ void scatter_slot(const tg_raster_bwd_args& a, int64_
 template <int D, class Tex, bool kGeo>
 struct BwdSmem {
     static constexpr bool kScale = Tex::kFormat == TG_TEX_FP8_E4M3;
-    float4 *m0, *m1, *m2, *col, *nrm;
-    int *row, *entry;
+    static constexpr int kVec = kGeo ? 6 : 5;
+    float4* rec;  // [bs][kVec]: three rows, colour, (texture row, entry), and with kGeo the normal
     float *col5, *scale;
     uint32_t *words;   // [groups][n_words]
     uint32_t *pixels;  // [n_words][threads]: the pixels' own bits
     float4* extra;     // anisotropic_bilinear: the boundary integration's per-warp areas
     __device__ __forceinline__ BwdSmem(float4* base, int bs, int side) {
-        m0 = base; m1 = m0 + bs; m2 = m1 + bs; col = m2 + bs; nrm = col + bs;
-        row = reinterpret_cast<int*>(nrm + (kGeo ? bs : 0));
-        entry = row + bs;
-        scale = reinterpret_cast<float*>(entry + bs);
+        rec = base;
+        scale = reinterpret_cast<float*>(rec + kVec * bs);
         col5 = scale + (kScale ? bs : 0);
         words = reinterpret_cast<uint32_t*>(col5 + (D == 5 ? bs : 0));
         pixels = words + (side * side / kGroupLanes) * (bs / 32);
         extra = reinterpret_cast<float4*>(pixels + side * side * (bs / 32));
     }
     static size_t bytes(int bs, int side) {
-        return (size_t)bs * ((kGeo ? 5 : 4) * sizeof(float4) + 8 + (kScale ? 4 : 0) + (D == 5 ? 4 : 0)) +
+        return (size_t)bs * (kVec * sizeof(float4) + (kScale ? 4 : 0) + (D == 5 ? 4 : 0)) +
                (size_t)(side * side / kGroupLanes + side * side) * (bs / 32) * 4;
     }
 };
@@ -285,6 +283,7 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
     const int nt = blockDim.x;  // one thread per pixel of the square
     const int ts = f.tile_size, side = square_side(ts), subs = squares_per_tile(ts);
     const BwdSmem<D, Tex, kGeo> S(smem4, bs, side);
+    constexpr int kVec = BwdSmem<D, Tex, kGeo>::kVec;
     float4* s_aniso = Filt::kAniso ? S.extra + (threadIdx.x >> 5) * kAnisoWarpF4 : nullptr;
 
     const TileWork tc = tile_work(f, subs == 1 ? item : item / subs);
@@ -308,7 +307,7 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
     P.rest = 0.f;
     P.ck_batch = -1;
     int32_t bin_final = -1;
-    int32_t rec = -1;  // anisotropic_bilinear: the forward's record of the next footprint integral (counting down)
+    int32_t record = -1;  // anisotropic_bilinear: the forward's record of the next footprint integral (counting down)
 #pragma unroll
     for (int k = 0; k < D; ++k) P.v_c[k] = 0.f;
     if constexpr (kGeo) {
@@ -345,7 +344,7 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
             P.acc_w_buf = P.acc_w = alpha_out;
         }
         if (Filt::kAniso && f.aniso_records != nullptr && f.contrib_masks != nullptr)
-            rec = f.aniso_record_count[pix] - 1;
+            record = f.aniso_record_count[pix] - 1;
     }
     // last contributor over the CTA
     const int32_t warp_bin_final = __reduce_max_sync(kFull, bin_final);
@@ -373,15 +372,15 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
                 const int32_t g = f.flatten_ids[idx];
                 const EntryRecord r = load_entry<D, kGeo>(f, g);
                 const int32_t row = __float_as_int(r.nrm.w);
-                S.m0[slot] = r.m0;
-                S.m1[slot] = r.m1;
-                S.m2[slot] = r.m2;
-                S.col[slot] = r.col;
+                float4* rec = S.rec + kVec * slot;
+                rec[0] = r.m0;
+                rec[1] = r.m1;
+                rec[2] = r.m2;
+                rec[3] = r.col;
+                rec[4] = make_float4(r.nrm.w, __int_as_float(g), 0.f, 0.f);
                 if constexpr (D == 5) S.col5[slot] = f.colors[(int64_t)g * D + 4];
-                if constexpr (kGeo) S.nrm[slot] = r.nrm;
+                if constexpr (kGeo) rec[5] = r.nrm;
                 if constexpr (BwdSmem<D, Tex, kGeo>::kScale) S.scale[slot] = f.tex_scales[row];
-                S.row[slot] = row;
-                S.entry[slot] = g;
                 if (!have_bits)
                     reach = group_mask(make_float4(r.m0.w, r.m1.w, r.m2.w, 1.f), r.m0, r.m1, r.m2, kTextured, f.range_x,
                                        f.range_y, f.g_weight, !Filt::kAniso, X0, Y0, side);
@@ -414,13 +413,14 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
             const int t = w * 32 + bit;
             const int32_t idx = batch_start + t;
             const bool act = listed && ((own >> bit) & 1u) != 0u && idx <= bin_final;
+            const float4* rec = S.rec + kVec * t;
             float vals[NS];
 #pragma unroll
             for (int k = 0; k < NS; ++k) vals[k] = 0.f;
             if (Filt::kAniso || act) {
-                const float4 m0 = S.m0[t], m1 = S.m1[t], m2 = S.m2[t];
+                const float4 m0 = rec[0], m1 = rec[1], m2 = rec[2];
                 const float4 xyo = make_float4(m0.w, m1.w, m2.w, BwdSmem<D, Tex, kGeo>::kScale ? S.scale[t] : 1.f);
-                const int row = S.row[t];
+                const int row = __float_as_int(rec[4].x);
                 const int64_t tex_base = (int64_t)row * tex_stride;
                 float* vt = a.v_textures != nullptr ? a.v_textures + 4 * tex_base : nullptr;
                 float* vct = Filt::kMip && a.v_tex_coarse != nullptr ? a.v_tex_coarse + 4 * (int64_t)row * mip_clen
@@ -429,14 +429,14 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
                 if constexpr (Filt::kAniso) {  // every lane takes part: the warp integrates footprints together
                     // the forward's integral of this pair's footprint, if it has one (it keeps the first
                     // aniso_record_cap contributors of each pixel, in order; this walks them back to front)
-                    const float4* r = act && rec >= 0 && rec < f.aniso_record_cap
+                    const float4* r = act && record >= 0 && record < f.aniso_record_cap
                                           ? reinterpret_cast<const float4*>(f.aniso_records) +
-                                                pix * f.aniso_record_cap + rec
+                                                pix * f.aniso_record_cap + record
                                           : nullptr;
                     eval_aniso_coop<Tex, true>(e, act, P.px, P.py, xyo, m0, m1, m2, f.textures, row, f.tex_rx, f.tex_ry,
                                                f.range_x, f.range_y, f.g_weight, kFull,
                                                reinterpret_cast<const float4*>(f.aniso_prefix), s_aniso, r);
-                    if (act) --rec;
+                    if (act) --record;
                 } else {
                     eval_pair<Tex, Filt>(e, P.px, P.py, xyo, m0, m1, m2, f.textures, tex_base, f.tex_rx, f.tex_ry,
                                          f.range_x, f.range_y, f.g_weight,
@@ -453,11 +453,11 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
                         P.T = f.t_checkpoints[((int64_t)tc.t + range_start / bs + b) * (int64_t)(ts * ts) +
                                               (i - tc.ty * ts) * ts + (j - tc.tx * ts)];
                     }
-                    const float4 c4 = S.col[t];
+                    const float4 c4 = rec[3];
                     float cp[D];
 #pragma unroll
                     for (int k = 0; k < D; ++k) cp[k] = k < 4 ? f4get(c4, k) : S.col5[t];
-                    const float4 nn = kGeo ? S.nrm[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    const float4 nn = kGeo ? rec[kVec - 1] : make_float4(0.f, 0.f, 0.f, 0.f);
                     accumulate_pair<D, Tex, Filt, kGeo, NS>(a, e, P, xyo.z, nn, cp, idx, vt, uv_scale, vals, vct,
                                                             mip_clen, &g4);
                 }
@@ -468,7 +468,7 @@ __device__ __forceinline__ void bwd_tile(const tg_raster_bwd_args& a, const floa
                                              a.v_textures, row, f.tex_rx, f.tex_ry, kFull, a.v_aniso_prefix, s_aniso);
             }
             reduce_scatter8<NS>(vals);
-            const int64_t g = S.entry[t];
+            const int64_t g = __float_as_int(rec[4].y);
             const int slot = slot_base<NS>(lane);
             if (a.v_packed != nullptr) {
                 float* dst = a.v_packed + g * NS + slot;

@@ -1183,6 +1183,13 @@ __device__ __forceinline__ float warp_sum(float v, unsigned mask) {
 // views, every entry staged by 7.5 tiles).
 struct EntryRecord {
     float4 m0, m1, m2, col, nrm;
+    __device__ __forceinline__ void store(float4* p) const {
+        p[0] = m0;
+        p[1] = m1;
+        p[2] = m2;
+        p[3] = col;
+        p[4] = nrm;
+    }
 };
 template <int D, bool kNormals>
 __device__ __forceinline__ EntryRecord load_entry(const tg_raster_fwd_args& a, int32_t g) {
