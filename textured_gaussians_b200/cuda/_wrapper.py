@@ -1105,10 +1105,10 @@ class _RotateNormals(torch.autograd.Function):
 def normals_to_world(normals: Tensor, viewmats: Tensor, view_table=None) -> Tensor:
     """Camera-space normal images [C,H,W,3] (or flat [n_pixels,3] with ``view_table``) in world space.
 
-    View matrices that need a gradient, or other than FP32, take the torch expression (one matrix product per
-    view), as does a call on more views than the kernel's grid holds."""
+    View matrices that need a gradient, types other than FP32 and images on the host take the torch expression (one
+    matrix product per view), as does a call on more views than the kernel's grid holds."""
     if viewmats.requires_grad or viewmats.dtype != torch.float32 or normals.dtype != torch.float32 or \
-            viewmats.shape[0] > 65535 or viewmats.dim() != 3:
+            viewmats.shape[0] > 65535 or viewmats.dim() != 3 or not (normals.is_cuda and viewmats.is_cuda):
         inv = torch.linalg.inv_ex(viewmats)[0][..., :3, :3]
         if view_table is None:
             return torch.einsum("...ij,...hwj->...hwi", inv, normals)
@@ -1159,9 +1159,10 @@ class _DepthImage(torch.autograd.Function):
 
 
 def depth_image_supported(colors: Tensor, viewmats: Tensor, Ks: Tensor) -> bool:
-    """Whether :func:`depth_image` takes these: FP32, cameras without gradients, images of at least 2x2 pixels (the
-    tensor expressions give smaller ones a border of their own shape) and at most 65535 views."""
-    return (colors.dim() == 4 and colors.dtype == viewmats.dtype == Ks.dtype == torch.float32 and
+    """Whether :func:`depth_image` takes these: FP32 on the GPU, cameras without gradients, images of at least 2x2
+    pixels (the tensor expressions give smaller ones a border of their own shape) and at most 65535 views."""
+    return (colors.is_cuda and viewmats.is_cuda and Ks.is_cuda and colors.dim() == 4 and
+            colors.dtype == viewmats.dtype == Ks.dtype == torch.float32 and
             not viewmats.requires_grad and not Ks.requires_grad and
             min(colors.shape[1:3]) >= 2 and colors.shape[0] <= 65535)
 
