@@ -14,8 +14,8 @@
 // Reductions:
 //  * per-splat gradients (colour, ray transform, means2d, opacity; with an upstream gradient for normals, distortion
 //    or median depth, or |means2d| asked for, also those) are summed over a group's eight lanes by a reduce-scatter
-//    (14 shuffles for 16 values, 21 for 24; of the ray transform its moments) that leaves consecutive values in consecutive lanes, which add them to
-//    the entry's row of a packed [E, slots] buffer -- 64 contiguous bytes, two per lane.  A splat meets 1.1 groups
+//    (14 shuffles for 16 values, 21 for 24; of the ray transform its moments) that leaves consecutive values in
+//    consecutive lanes, which add them to the entry's row of a packed [E, slots] buffer -- 64 contiguous bytes, two per lane.  A splat meets 1.1 groups
 //    per tile that lists it, so collecting a tile's sums in shared memory first would not save adds; the rows are
 //    spread to the separate gradient arrays by one pass over the entries afterwards;
 //  * per-texel gradients are RGBA float4 vector atomics, one per bilinear tap

@@ -997,10 +997,6 @@ __device__ __forceinline__ float4 cull_box(const float4 xyo, const float4 m0, co
     return box;
 }
 
-__device__ __forceinline__ bool in_box(const float4 b, float px, float py) {
-    return px >= b.x && px <= b.z && py >= b.y && py <= b.w;
-}
-
 // ---------------------------------------------------------------- pixel groups
 // A CTA composites a square of side 8 (64 threads) or 16 (256 threads) pixels; warp w owns an 8x4 block of it and
 // each 8 lanes of the warp a 4x2 group of that block, so neighbouring lanes stay neighbouring pixels.  Each group
@@ -1162,18 +1158,6 @@ template <int NT>
 __device__ __forceinline__ float tex_color_adj(const PairEvalT<NT>& e, int k) { return tex_color(e, k); }
 __device__ __forceinline__ float tex_color_adj(const PairEvalAniso& e, int k) {
     return (k >= 4 || !e.tex_valid) ? 0.f : f4get(e.tsum, k);
-}
-
-// Sum over the lanes in `mask`; lanes outside it contribute zero.  The
-// butterfly reads lane^o, which exists whenever the mask is a prefix of
-// lanes whose count is a power of two, or the full warp.
-__device__ __forceinline__ float warp_sum(float v, unsigned mask) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float u = __shfl_xor_sync(mask, v, o);
-        if (((threadIdx.x & 31) ^ o) < 32 && (mask >> ((threadIdx.x & 31) ^ o)) & 1u) v += u;
-    }
-    return v;
 }
 
 // What the compositor stages of a splat: rows of the ray transform with the projected centre and the opacity
