@@ -748,7 +748,7 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
         B.call("tg_rasterize_fwd", st, B.lib().tg_rasterize_fwd, ctypes.byref(a), st)
         ctx.save_for_backward(means2d, ray_transforms, colors, opacities, textures, normals, densify, backgrounds, m,
                               tex_store, tex_scales, isect_offsets, flatten_ids, render_colors, render_alphas,
-                              last_ids, median_ids, gaussian_ids)
+                              last_ids, median_ids, gaussian_ids, masks_buf, entries)
         ctx.cfg = (range_x, range_y, width, height, tile_size, absgrad, g_weight, adjoint, bg_grad_index_ok,
                    gs_contrib_threshold, N, n_contrib, C, pshape)
         ctx.layout = layout
@@ -757,8 +757,6 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
         ctx.t_checkpoints = ckpt
         ctx.aniso_prefix = prefix
         ctx.aniso_records = (records, counts)
-        ctx.contrib_masks = masks_buf
-        ctx.entry_records = entries
         ctx.mark_non_differentiable(contrib_sum, contrib_count)
         ctx.set_materialize_grads(False)  # an output the loss does not use passes no gradient (NULL) to the adjoint
         return render_colors, render_alphas, render_normals, render_distort, render_median, contrib_sum, contrib_count
@@ -768,7 +766,7 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
                  v_contrib_sum, v_contrib_count):
         (means2d, ray_transforms, colors, opacities, textures, normals, densify, backgrounds, m, tex_store, tex_scales,
          isect_offsets, flatten_ids, render_colors, render_alphas, last_ids, median_ids,
-         gaussian_ids) = ctx.saved_tensors
+         gaussian_ids, masks_buf, entries) = ctx.saved_tensors
         (range_x, range_y, width, height, tile_size, absgrad, g_weight, adjoint, bg_grad_index_ok,
          gs_contrib_threshold, N, n_contrib, C, pshape) = ctx.cfg
         dev = means2d.device
@@ -780,8 +778,8 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
                       backgrounds, m, width, height, tile_size, isect_offsets, flatten_ids, gaussian_ids, n_contrib,
                       0.0, g_weight, C, N, ctx.layout, ctx.n_isects_dev, *ctx.mip)
         f.t_checkpoints = B.ptr(ctx.t_checkpoints)
-        f.contrib_masks = B.ptr(ctx.contrib_masks)
-        f.entry_records, f.n_entries = B.ptr(ctx.entry_records), means2d.numel() // 2
+        f.contrib_masks = B.ptr(masks_buf)
+        f.entry_records, f.n_entries = B.ptr(entries), means2d.numel() // 2
         f.aniso_prefix = B.ptr(ctx.aniso_prefix)
         if ctx.aniso_records[0] is not None:
             f.aniso_records, f.aniso_record_count = B.ptr(ctx.aniso_records[0]), B.ptr(ctx.aniso_records[1])
