@@ -14,8 +14,8 @@
 // Reductions:
 //  * per-splat gradients (colour, ray transform, means2d, opacity; with an upstream gradient for normals, distortion
 //    or median depth, or |means2d| asked for, also those) are summed over a group's eight lanes by a reduce-scatter
-//    (14 shuffles for 16 values, 21 for 24; of the ray transform its moments) that leaves consecutive values in
-//    consecutive lanes, which add them to the entry's row of a packed [E, slots] buffer -- 64 contiguous bytes, two per lane.  A splat meets 1.1 groups
+//    (14 shuffles for 16 values, 21 for 24) that leaves consecutive values in consecutive lanes, which add them to
+//    the entry's row of a packed [E, slots] buffer -- 64 contiguous bytes, two per lane.  A splat meets 1.1 groups
 //    per tile that lists it, so collecting a tile's sums in shared memory first would not save adds; the rows are
 //    spread to the separate gradient arrays by one pass over the entries afterwards;
 //  * per-texel gradients are RGBA float4 vector atomics, one per bilinear tap
@@ -215,12 +215,10 @@ __device__ __forceinline__ void accumulate_pair(const tg_raster_bwd_args& a, con
         const float iz = 1.f / e.z.z;
         const float a_ = vsx * iz, b_ = vsy * iz;
         const f3 vz = mk3(a_, b_, -(a_ * e.sx + b_ * e.sy));
-        if (a.v_packed != nullptr) {  // the moments about the projected centre (see unpack_grads_kernel)
-            vals[GS::kM + 0] = vz.x; vals[GS::kM + 1] = vz.y; vals[GS::kM + 2] = vz.z;
-            vals[GS::kM + 3] = e.dx * vz.x; vals[GS::kM + 4] = e.dx * vz.y; vals[GS::kM + 5] = e.dx * vz.z;
-            vals[GS::kM + 6] = e.dy * vz.x; vals[GS::kM + 7] = e.dy * vz.y; vals[GS::kM + 8] = e.dy * vz.z;
-            return;
-        }
+        // The pair's nine products themselves.  As moments of vz about the projected centre (one sum less to form a pair,
+        // expanded once per entry) FP32 loses a pixel's place beside a centre far off the image: gradients of splats
+        // whose plane passes near the camera were 3e-2 off against 6e-7 (median over 96, 160x120), and the step was
+        // no faster (20.11 and 20.17 ms for the 1M-splat mixture, four views).
         const f3 vhu = cross(e.hv, vz), vhv = cross(vz, e.hu);
         vals[GS::kM + 0] = -vhu.x; vals[GS::kM + 1] = -vhu.y; vals[GS::kM + 2] = -vhu.z;
         vals[GS::kM + 3] = -vhv.x; vals[GS::kM + 4] = -vhv.y; vals[GS::kM + 5] = -vhv.z;
@@ -522,39 +520,9 @@ __global__ void densify_grad_kernel(const float* __restrict__ v_M, const float* 
     v_densify[2 * e + 1] = v_M[9 * e + 5] * depth;
 }
 
-// Gradient of the ray transform M from an entry's moments of v_zeta over its pairs: r = (S, X, Y) with S = sum v_zeta
-// and X, Y the sums weighted with the projected centre's offset (cx - px, cy - py).  h_u = px M2 - M0 and
-// h_v = py M2 - M1 are linear in the pixel, so the pairs' nine products
-//   v_h_u = h_v x v_zeta,  v_h_v = v_zeta x h_u,  v_M0 = -v_h_u,  v_M1 = -v_h_v,  v_M2 = px v_h_u + py v_h_v
-// sum to crosses of the moments with M (px py M2 x v_zeta cancels), formed here once per entry instead of once per
-// pair.  In FP64: M0 and M1 nearly cancel against the centre's multiple of M2.
-__device__ __forceinline__ void moments_to_transform(const float* __restrict__ M, float2 c, float* r) {
-    bool any = false;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) any = any || r[k] != 0.f;
-    if (!any) return;  // (and M may be anything)
-    struct d3 {
-        double x, y, z;
-    };
-    auto cross = [](d3 a, d3 b) { return d3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; };
-    const double cx = c.x, cy = c.y;
-    const d3 m2{M[6], M[7], M[8]};
-    const d3 m0{M[0] - cx * m2.x, M[1] - cx * m2.y, M[2] - cx * m2.z}, m1{M[3] - cy * m2.x, M[4] - cy * m2.y, M[5] - cy * m2.z};
-    const d3 s{r[0], r[1], r[2]}, sx{-(double)r[3], -(double)r[4], -(double)r[5]},
-        sy{-(double)r[6], -(double)r[7], -(double)r[8]};
-    const d3 a0 = cross(m2, sy), a1 = cross(m1, s), b0 = cross(sx, m2), b1 = cross(s, m0), e0 = cross(m0, sy),
-             e1 = cross(m1, sx);
-    const d3 A{a0.x - a1.x, a0.y - a1.y, a0.z - a1.z}, B{b0.x - b1.x, b0.y - b1.y, b0.z - b1.z};
-    r[0] = (float)-A.x; r[1] = (float)-A.y; r[2] = (float)-A.z;
-    r[3] = (float)-B.x; r[4] = (float)-B.y; r[5] = (float)-B.z;
-    r[6] = (float)(e0.x - e1.x + cx * A.x + cy * B.x);
-    r[7] = (float)(e0.y - e1.y + cx * A.y + cy * B.y);
-    r[8] = (float)(e0.z - e1.z + cx * A.z + cy * B.z);
-}
-
 // Spreads the entries' packed rows over the gradient arrays (every element is written, so none is cleared first)
-// and forms v_ray_transforms and v_densify.  128 rows per CTA go through shared memory, so that both the reads and
-// the writes of the odd-sized arrays are coalesced; the pass moves its bytes once (HBM-bound).
+// and forms v_densify.  128 rows per CTA go through shared memory, so that both the reads and the writes of the
+// odd-sized arrays are coalesced; the pass moves its bytes once (HBM-bound).
 template <int D, bool kGeo>
 __global__ void __launch_bounds__(128) unpack_grads_kernel(const tg_raster_bwd_args a) {
     using GS = GradSlots<D, kGeo>;
@@ -571,10 +539,9 @@ __global__ void __launch_bounds__(128) unpack_grads_kernel(const tg_raster_bwd_a
     __syncthreads();
     if ((int)threadIdx.x < n) {
         const int64_t e = e0 + threadIdx.x;
-        const float* M = a.f.ray_transforms + 9 * e;
-        float* r = s + threadIdx.x * kPitch + GS::kM;
-        moments_to_transform(M, reinterpret_cast<const float2*>(a.f.means2d)[e], r);
-        reinterpret_cast<float2*>(a.v_densify)[e] = make_float2(r[2] * M[8], r[5] * M[8]);
+        const float depth = a.f.ray_transforms[9 * e + 8];
+        const float* r = s + threadIdx.x * kPitch + GS::kM;
+        reinterpret_cast<float2*>(a.v_densify)[e] = make_float2(r[2] * depth, r[5] * depth);
     }
     __syncthreads();
     auto spread = [&](float* dst, int width, int off) {
