@@ -42,3 +42,18 @@ def test_large_and_small_images_agree(tile, depth, n):
     gs = torch.autograd.grad(small[0], small_leaves, up)
     for k, (a, b) in enumerate(zip(gb, gs)):
         assert rel_l2(to_np(a), to_np(b)) < 2.0 ** -24 / 1e-4, k  # (test_gpu_groups: the stored alpha's last place)
+
+
+@pytest.mark.parametrize("tile,depth", [(8, 608), (8, 640), (8, 1024), (16, 640), (16, 1024)])
+def test_deep_batches_agree_with_shallow_ones(tile, depth):
+    """Batches of up to 1024 splats, of which four squares' do not fit one CTA's shared memory together above 608."""
+    s = scenes.tiny(seed=22, N=1500, R=16)
+    s.means[:1200] *= 0.02  # lists longer than a batch
+    deep_leaves, deep = _render(s, 800, 800, tile, 1500, depth)
+    leaves, ref = _render(s, 800, 800, tile, 1500, 32)
+    for k in (0, 1, 2, 5):
+        assert_close(to_np(deep[k]), to_np(ref[k]), 1e-6, 1e-6, 1e-3, name=f"output {k}")
+    up = torch.randn_like(ref[0])
+    for k, (a, b) in enumerate(zip(torch.autograd.grad(deep[0], deep_leaves, up),
+                                   torch.autograd.grad(ref[0], leaves, up))):
+        assert rel_l2(to_np(a), to_np(b)) < 2.0 ** -24 / 1e-4, k

@@ -304,9 +304,10 @@ __global__ void __launch_bounds__(256, TG_FWD_MIN_CTAS) raster_fwd_kernel(const 
 // for 60k splats, 800x600, the SMs busy for half of it at 16 % occupancy; 3.25 ms so).  But the halves wait for one
 // another, and where every SM is full anyway that costs: 22.1 against 20.5 ms for 300k splats in two 1600x1200
 // views.  So only the first kLongTiles squares are taken so, the others four to a CTA, two warps each; and from
-// kFullSquares squares on all take the other filters' kernel.
+// kFullSquares squares on, or where a batch is too deep for that, all take the other filters' kernel.
 constexpr int kFullSquares = 128 * kNumSMs;  // eight times what the device holds at once
 constexpr int kLongTiles = 3 * kNumSMs;  // of 1, 3 and 6 per SM (60k splats: 3.96, 3.25, 3.32 ms)
+constexpr size_t kMaxSmem = 227 * 1024;  // of a CTA
 constexpr int kAnisoWarps = 8;
 constexpr int kAnisoThreads = 32 * kAnisoWarps;
 constexpr int kAnisoItems = 64;  // 32, 48, 64: 3.63, 3.45, 3.25 ms; more leaves the walk's reads less L1
@@ -588,7 +589,8 @@ cudaError_t launch_aniso_fwd(const tg_raster_fwd_args& a, cudaStream_t s) {
     const int64_t subs = (a.tile_size / kAnisoSide) * (a.tile_size / kAnisoSide), squares = tiles * subs;
     if (squares == 0) return cudaSuccess;
     if (squares > 0x7fffffff) return cudaErrorInvalidValue;
-    if (squares >= kFullSquares) return launch_fwd_kernel<D, Tex, false, FiltAniso>(a, s);
+    // (batches deeper than 608 splats do not fit a CTA's shared memory four times)
+    if (squares >= kFullSquares || smem > kMaxSmem) return launch_fwd_kernel<D, Tex, false, FiltAniso>(a, s);
     const int64_t n_long = std::min<int64_t>(squares, (kLongTiles + subs - 1) / subs * subs);
     const int64_t items = n_long + (squares - n_long + 3) / 4;
     const cudaError_t err = cudaFuncSetAttribute(aniso_fwd_kernel<D, Tex>, cudaFuncAttributeMaxDynamicSharedMemorySize,
