@@ -10,7 +10,7 @@ import pytest
 import torch
 
 from textured_gaussians_b200.cuda._wrapper import depth_image
-from textured_gaussians_b200.utils import depth_to_normal
+from textured_gaussians_b200.utils import depth_image_expression, depth_to_normal
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -55,3 +55,28 @@ def test_depth_image(W, H, C, D, expected, median):
     for a, b in zip(got[1], ref[1]):
         assert (a is None or a.abs().max() == 0) if b is None else (
             (a.double() - b).abs().max() <= 5e-4 * b.abs().max())
+
+
+@pytest.mark.parametrize("expected,median", [(True, False), (False, False), (True, True)])
+def test_second_derivatives(expected, median):
+    """A derivative of the gradient: taken of the same FP32 expressions on either side, so alike but for the order in
+    which a few shares of a gradient are added (a handful of roundings of 2^-24: 1e-5 of the largest is ample)."""
+    W, H, D = 40, 21, 4
+    g = torch.Generator().manual_seed(3)
+    rnd = lambda *s: torch.rand(*s, generator=g).to(DEV)  # noqa: E731
+    colors, al, med = rnd(2, H, W, D) + 1, 0.25 + 0.75 * rnd(2, H, W, 1), rnd(2, H, W, 1) + 1
+    cam = (torch.eye(4, device=DEV).repeat(2, 1, 1),
+           torch.tensor([[50.0, 0, W / 2], [0, 50.0, H / 2], [0, 0, 1]], device=DEV).repeat(2, 1, 1))
+    ups = [rnd(2, H, W, D), rnd(2, H, W, 3)]
+    res = []
+    for fn in (depth_image, depth_image_expression):
+        t = [v.clone().requires_grad_() for v in ((colors, al) if expected else (colors,)) + ((med,) if median else ())]
+        out, n = fn(t[0], t[1] if expected else None, t[-1] if median else None, *cam)
+        loss = sum((o * u).sum() for o, u in zip((out, n), ups) if o is not None)
+        first = torch.autograd.grad(loss, t, create_graph=True)
+        assert all(f.requires_grad for f in first if f.abs().max() > 0)
+        second = torch.autograd.grad(sum((f * f).sum() for f in first), t)
+        res.append((first, second))
+    for a, b in zip(res[0][0] + res[0][1], res[1][0] + res[1][1]):
+        assert (a - b).abs().max() <= 1e-5 * b.abs().max()
+    assert all(s.abs().max() > 0 for s in res[0][1])

@@ -31,6 +31,7 @@ from torch import Tensor
 
 from .. import _backend as B
 from ..graph import active_plan
+from ..utils import depth_image_expression
 
 _FILTER_ADJOINT = {
     "bilinear": B.TG_ADJ_REFERENCE,
@@ -1119,21 +1120,20 @@ def normals_to_world(normals: Tensor, viewmats: Tensor, view_table=None) -> Tens
 
 # --------------------------------------------------------------------------- depth images
 class _DepthImage(torch.autograd.Function):
-    """(colours with the expected depth, or None; world-space normals of the depth image, or None)."""
+    """(colours with the expected depth, or None; world-space normals of the depth image, or None), of contiguous
+    inputs.  Where the gradient itself is to be differentiated (``create_graph``) it comes from the tensor
+    expressions: the kernel's has no graph."""
 
     @staticmethod
     def forward(ctx, colors, alphas, depth, camtoworlds, Ks):
-        x, al = (None if t is None else t.contiguous() for t in (colors, alphas))
-        # a copy of what the adjoint reads again and the caller holds (the compositor keeps colours and opacities itself)
-        z = None if depth is None else depth.clone(memory_format=torch.contiguous_format)
-        out = None if al is None else torch.empty_like(x)
-        normals = None if camtoworlds is None else x.new_empty(x.shape[:-1] + (3,))
-        ctx.save_for_backward(x, al, z, camtoworlds, Ks)
+        out = None if alphas is None else torch.empty_like(colors)
+        normals = None if camtoworlds is None else colors.new_empty(colors.shape[:-1] + (3,))
+        ctx.save_for_backward(colors, alphas, depth, camtoworlds, Ks)
         ctx.set_materialize_grads(False)
-        C, H, W, D = x.shape
-        a = B.DepthImageArgs(C, W, H, D, B.ptr(x), B.ptr(al), B.ptr(z), B.ptr(camtoworlds), B.ptr(Ks), B.ptr(out),
-                             B.ptr(normals))
-        st = B.stream_of(x)
+        C, H, W, D = colors.shape
+        a = B.DepthImageArgs(C, W, H, D, B.ptr(colors), B.ptr(alphas), B.ptr(depth), B.ptr(camtoworlds), B.ptr(Ks),
+                             B.ptr(out), B.ptr(normals))
+        st = B.stream_of(colors)
         B.call("tg_depth_image_fwd", st, B.lib().tg_depth_image_fwd, ctypes.byref(a), st)
         return out, normals
 
@@ -1142,6 +1142,17 @@ class _DepthImage(torch.autograd.Function):
         if v_out is None and v_normals is None:
             return (None,) * 5
         x, al, z, camtoworlds, Ks = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            outs = depth_image_expression(x, al, z, camtoworlds, Ks)
+            pairs = [(o, v) for o, v in zip(outs, (v_out, v_normals)) if v is not None and o.requires_grad]
+            want = [k for k in range(3) if ctx.needs_input_grad[k]]
+            grads = [None] * 5
+            if pairs:
+                found = torch.autograd.grad([o for o, _ in pairs], [(x, al, z)[k] for k in want],
+                                            [v for _, v in pairs], create_graph=True, allow_unused=True)
+                for k, g in zip(want, found):
+                    grads[k] = g
+            return tuple(grads)
         v_out, v_normals = (None if t is None else t.contiguous() for t in (v_out, v_normals))
         v_x = torch.empty_like(x) if ctx.needs_input_grad[0] else None
         v_al = torch.empty_like(al) if al is not None else None
@@ -1171,7 +1182,9 @@ def depth_image(colors: Tensor, alphas: Optional[Tensor], depth: Optional[Tensor
     max(alpha, 1e-10), and with ``camtoworlds`` world-space normals [C,H,W,3] of ``depth`` [C,H,W,1], or of the last
     channel where that is None."""
     cam = (None, None) if camtoworlds is None else (camtoworlds.contiguous(), Ks.contiguous())
-    return _DepthImage.apply(colors, alphas, depth, *cam)
+    # a copy of what the adjoint reads again and the caller holds (the compositor keeps colours and opacities itself)
+    depth = None if depth is None else depth.clone(memory_format=torch.contiguous_format)
+    return _DepthImage.apply(colors.contiguous(), None if alphas is None else alphas.contiguous(), depth, *cam)
 
 
 # --------------------------------------------------------------------------- gradient consumers

@@ -49,7 +49,7 @@ from .cuda._wrapper import (
     spherical_harmonics,
     spherical_harmonics_shared,
 )
-from .utils import depth_to_normal
+from .utils import depth_image_expression
 
 _RENDER_MODES = ["RGB", "D", "ED", "RGB+D", "RGB+ED"]
 
@@ -137,19 +137,13 @@ def _finish(p, render_colors, render_alphas, render_normals, render_distort, ren
             gs_contrib_count, viewmats, Ks, width, height, tile_size, render_mode, depth_mode):
     render_normals_from_depth = None
     expected, with_normals = render_mode in ["ED", "RGB+ED"], render_mode in ["RGB+ED", "RGB+D"]
-    if (expected or with_normals) and depth_image_supported(render_colors, viewmats, Ks):
-        cam = (_inverse(viewmats), Ks) if with_normals else ()
-        out, n = depth_image(render_colors, render_alphas if expected else None,
-                             None if depth_mode == "expected" else render_median, *cam)
+    if expected or with_normals:
+        step = depth_image if depth_image_supported(render_colors, viewmats, Ks) else depth_image_expression
+        cam = (_inverse(viewmats), Ks) if with_normals else (None, None)
+        out, n = step(render_colors, render_alphas if expected else None,
+                      None if depth_mode == "expected" else render_median, *cam)
         render_colors = out if expected else render_colors
         render_normals_from_depth = n.squeeze(0) if with_normals else None
-        expected = with_normals = False
-    if expected:
-        render_colors = torch.cat(
-            [render_colors[..., :-1], render_colors[..., -1:] / render_alphas.clamp(min=1e-10)], dim=-1)
-    if with_normals:
-        depth_for_normal = render_colors[..., -1:] if depth_mode == "expected" else render_median
-        render_normals_from_depth = depth_to_normal(depth_for_normal, _inverse(viewmats), Ks).squeeze(0)
     meta = {
         "camera_ids": p["camera_ids"],
         "gaussian_ids": p["gaussian_ids"],

@@ -7,6 +7,8 @@ the border.  Plain torch on the GPU tensors (post-processing glue).
 """
 from __future__ import annotations
 
+from typing import Optional
+
 import torch
 import torch.nn.functional as F
 from torch import Tensor
@@ -45,3 +47,18 @@ def depth_to_normal(depths: Tensor, camtoworlds: Tensor, Ks: Tensor, z_depth: bo
     d_cols = pts[..., 1:-1, 2:, :] - pts[..., 1:-1, :-2, :]
     n = F.normalize(torch.cross(d_rows, d_cols, dim=-1), dim=-1)
     return F.pad(n, (0, 0, 1, 1, 1, 1), value=0.0)
+
+
+def depth_image_expression(colors: Tensor, alphas: Optional[Tensor], depth: Optional[Tensor],
+                           camtoworlds: Optional[Tensor], Ks: Optional[Tensor]):
+    """Last step of the depth render modes as tensor expressions (any type and device, differentiable at will): with
+    ``alphas`` the colours with their last channel over max(alpha, 1e-10), else None; with ``camtoworlds`` the normals
+    of ``depth``, or of the (divided) last channel where that is None, else None."""
+    out = None
+    if alphas is not None:
+        out = torch.cat([colors[..., :-1], colors[..., -1:] / alphas.clamp(min=1e-10)], dim=-1)
+    if camtoworlds is None:
+        return out, None
+    if depth is None:
+        depth = (colors if out is None else out)[..., -1:]
+    return out, depth_to_normal(depth, camtoworlds, Ks)
