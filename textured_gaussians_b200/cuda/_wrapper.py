@@ -699,7 +699,9 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
     def forward(ctx, means2d, ray_transforms, colors, opacities, textures, normals, densify, backgrounds, masks,
                 tex_store, tex_scales, range_x, range_y, width, height, tile_size, isect_offsets, flatten_ids,
                 absgrad, gs_contrib_threshold, g_weight, adjoint, bg_grad_index_ok, gaussian_ids, n_rows, layout,
-                mip_levels=0, filter_code=0):
+                grad_mode, mip_levels=0, filter_code=0):
+        # grad_mode: the caller's torch.is_grad_enabled() (off in here); needs_input_grad is set without it too
+        differentiable = grad_mode and any(ctx.needs_input_grad)
         dev = means2d.device
         coarse = _coarse_pyramid(textures, mip_levels) if mip_levels else None
         vt = None if layout is None else layout.get("view_table")
@@ -730,8 +732,8 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
         a.contrib_sum, a.contrib_count = B.ptr(contrib_sum), B.ptr(contrib_count)
         ckpt = _checkpoint_buffer(layout, isect_offsets, flatten_ids, tile_size, C, dev)
         a.t_checkpoints = B.ptr(ckpt)
-        masks_buf = _contrib_masks(layout, isect_offsets, flatten_ids, tile_size, C, dev) if any(
-            ctx.needs_input_grad) else None
+        masks_buf = (_contrib_masks(layout, isect_offsets, flatten_ids, tile_size, C, dev) if differentiable
+                     else None)
         a.contrib_masks = B.ptr(masks_buf)
         entries = _entry_records(means2d, flatten_ids)
         a.entry_records, a.n_entries = B.ptr(entries), means2d.numel() // 2
@@ -742,7 +744,7 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
         records = counts = None
         n_pix = math.prod(pshape)
         cap = min(ANISO_RECORDS, ANISO_RECORDS_BYTES // max(1, 16 * n_pix))
-        if prefix is not None and cap > 0 and any(ctx.needs_input_grad):
+        if prefix is not None and cap > 0 and differentiable:
             records = torch.empty((n_pix, cap, 4), dtype=torch.float32, device=dev)
             counts = torch.empty((n_pix,), dtype=torch.int32, device=dev)
             a.aniso_records, a.aniso_record_count, a.aniso_record_cap = B.ptr(records), B.ptr(counts), cap
@@ -827,7 +829,7 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
             v_textures = v_textures.to(textures.dtype)
         return (v_means2d, v_ray_transforms, v_colors, v_opacities, v_textures, v_normals, v_densify, v_backgrounds,
                 None, None, None, None, None, None, None, None, None, None, None, None, None, None, None, None, None,
-                None, None, None)
+                None, None, None, None)
 
 
 _TRANSMITTANCE = ("divide", "checkpoint")
@@ -1014,8 +1016,7 @@ def rasterize_to_pixels_textured_gaussians(
         _FILTER_ADJOINT[filtering], False, gaussian_ids, textures.shape[0],
         _layout(tile_order, view_table,
                 batch_depth or (ANISO_BATCH_DEPTH if filter_code == B.TG_FILTER_ANISO_BILINEAR else 0), persistent,
-                means2d.device, transmittance), mip_levels,
-        filter_code)
+                means2d.device, transmittance), torch.is_grad_enabled(), mip_levels, filter_code)
     render_colors = out[0]
     if padded > 0:
         render_colors = render_colors[..., :-padded]
@@ -1074,7 +1075,8 @@ def rasterize_to_pixels_2dgs(
         normals.contiguous(), densify.contiguous(), None if backgrounds is None else backgrounds.contiguous(), masks,
         None, None, 3.0, 3.0, int(image_width), int(image_height), int(tile_size), isect_offsets.contiguous(),
         flatten_ids.contiguous(), absgrad, gs_contrib_threshold, 1.0, B.TG_ADJ_REFERENCE, True, gaussian_ids,
-        int(n_gaussians), _layout(tile_order, view_table, batch_depth, persistent, means2d.device))
+        int(n_gaussians), _layout(tile_order, view_table, batch_depth, persistent, means2d.device),
+        torch.is_grad_enabled())
     render_colors = out[0]
     if padded > 0:
         render_colors = render_colors[..., :-padded]
