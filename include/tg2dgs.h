@@ -286,6 +286,15 @@ TG_API size_t tg_isect_sorted_lists_bytes(int64_t n, int32_t key_bits);
 TG_API int tg_isect_sorted_lists(const tg_isect_args* a, void* order_ws, int64_t n, void* list_ws, size_t list_bytes,
                                  tg_stream_t stream);
 
+/* Diagnostic, as tg_sort_lookback_selftest: tg_isect_sorted_lists where nobody
+ * takes the first 4096 pairs of the entries' depth sort (sort = 1) or of the
+ * lists' sort (sort = 2), so that every look-back of that pass waits for them
+ * and gives up.  The lists come out wrong, with entries in range wherever
+ * they are written (a place may be left unwritten).  More than 16,384 entries
+ * (sort = 1) or intersections (2).  No counterpart in the reference. */
+TG_API int tg_isect_sorted_lookback_selftest(const tg_isect_args* a, void* order_ws, int64_t n, void* list_ws,
+                                             size_t list_bytes, int32_t sort, tg_stream_t stream);
+
 /* Work order for the compositor (tg_raster_fwd_args.tile_order): the tiles by
  * descending list length, ties by index.  offsets [n_tiles] as from
  * tg_isect_offset_encode; n_isects (or, if not NULL, *n_isects_dev, at most

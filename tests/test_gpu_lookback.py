@@ -1,0 +1,65 @@
+"""Sorted lists whose look-back waits give up (nobody takes the first 4096 pairs of a sort): the call ends, what it
+writes stays in range, and the next call on the same buffers is right.  The scratch is filled with 0xff first, so that
+places the broken sort leaves unwritten hold ids of no entry.
+"""
+import ctypes
+
+import pytest
+import torch
+
+from textured_gaussians_b200 import _backend as B
+from textured_gaussians_b200.cuda._wrapper import isect_tiles
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+W, H, TILE, E = 500, 300, 16, 40000
+TW, TH = -(-W // TILE), -(-H // TILE)
+KEY_BITS = (TW * TH).bit_length() + 1
+
+
+def _entries():
+    g = torch.Generator(device=DEV).manual_seed(9)
+    xy = torch.rand(1, E, 2, generator=g, device=DEV) * torch.tensor([float(W), float(H)], device=DEV)
+    radii = (torch.rand(1, E, generator=g, device=DEV) ** 4 * 30).int()
+    return xy, radii, torch.rand(1, E, generator=g, device=DEV) + 0.1
+
+
+class Call:
+    """One tg_isect_sorted_count / _lists pair on buffers of its own."""
+
+    def __init__(self, xy, radii, depths):
+        self.L, self.st = B.lib(), B.stream_of(xy)
+        u8 = lambda n: torch.full((n,), 0xff, dtype=torch.uint8, device=DEV)  # noqa: E731
+        self.order_ws = u8(self.L.tg_isect_sorted_order_bytes(E))
+        self.counts = torch.empty((1, E), dtype=torch.int32, device=DEV)
+        self.n_dev = torch.empty((1,), dtype=torch.int64, device=DEV)
+        self.a = B.IsectArgs(E, E, None, B.ptr(xy), B.ptr(radii), B.ptr(depths), TILE, TW, TH, 1, B.ptr(self.counts),
+                             None, B.ptr(self.n_dev))
+        self.count()
+        self.n = int(self.n_dev.item())
+        self.list_ws = u8(self.L.tg_isect_sorted_lists_bytes(self.n, KEY_BITS))
+        self.ids = torch.zeros((self.n,), dtype=torch.int64, device=DEV)
+        self.flat = torch.zeros((self.n,), dtype=torch.int32, device=DEV)
+        self.a.isect_ids, self.a.flatten_ids = B.ptr(self.ids), B.ptr(self.flat)
+
+    def count(self):
+        B.check(self.L.tg_isect_sorted_count(ctypes.byref(self.a), B.ptr(self.order_ws), self.order_ws.numel(),
+                                             self.st), "count")
+
+    def lists(self, lost=0):
+        args = [ctypes.byref(self.a), B.ptr(self.order_ws), self.n, B.ptr(self.list_ws), self.list_ws.numel()]
+        fn = self.L.tg_isect_sorted_lookback_selftest if lost else self.L.tg_isect_sorted_lists
+        B.check(fn(*args, *([lost] if lost else []), self.st), "lists")
+
+
+@pytest.mark.parametrize("lost", [1, 2])
+def test_lists_stay_in_range_and_the_next_call_is_right(lost):
+    inputs = _entries()
+    c = Call(*inputs)
+    c.lists(lost)
+    torch.cuda.synchronize()
+    assert int(c.flat.min()) >= 0 and int(c.flat.max()) < E
+    c.count()
+    c.lists()
+    _, ids, flat = isect_tiles(*inputs, TILE, TW, TH)
+    assert torch.equal(c.ids, ids) and torch.equal(c.flat, flat)

@@ -129,6 +129,8 @@ def lib() -> ctypes.CDLL:
                 ("tg_isect_emit", [ctypes.POINTER(IsectArgs), P]),
                 ("tg_isect_sorted_count", [ctypes.POINTER(IsectArgs), P, ctypes.c_size_t, P]),
                 ("tg_isect_sorted_lists", [ctypes.POINTER(IsectArgs), P, I64, P, ctypes.c_size_t, P]),
+                ("tg_isect_sorted_lookback_selftest",
+                 [ctypes.POINTER(IsectArgs), P, I64, P, ctypes.c_size_t, I32, P]),
                 ("tg_tile_order", [P, I64, I64, P, P, P, ctypes.c_size_t, P]),
                 ("tg_sort_pairs", [P, P, P, P, I64, I32, P, ctypes.c_size_t, ctypes.POINTER(I32), P]),
                 ("tg_sort_status", [P, I64, I32, P]),

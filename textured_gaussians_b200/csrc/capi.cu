@@ -26,7 +26,7 @@ size_t isect_order_workspace_bytes(int64_t E);
 cudaError_t launch_isect_order(const tg_isect_args& a, void* workspace, cudaStream_t s);
 size_t isect_lists_workspace_bytes(int64_t n, int key_bits);
 cudaError_t launch_isect_lists(const tg_isect_args& a, void* order_ws, int64_t n, int tile_bits, int key_bits, void* ws,
-                               cudaStream_t s);
+                               int lost, cudaStream_t s);
 size_t tile_order_workspace_bytes(int64_t n_tiles);
 cudaError_t launch_tile_order(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, const int64_t* n_dev,
                               int32_t* order, void* ws, cudaStream_t s);
@@ -375,8 +375,9 @@ int tg_isect_sorted_count(const tg_isect_args* a, void* order_ws, size_t order_b
     return cuda_status(tg::launch_isect_order(*a, order_ws, stream), "tg_isect_sorted_count");
 }
 
-int tg_isect_sorted_lists(const tg_isect_args* a, void* order_ws, int64_t n, void* list_ws, size_t list_bytes,
-                          tg_stream_t stream) {
+namespace {
+int sorted_lists(const tg_isect_args* a, void* order_ws, int64_t n, void* list_ws, size_t list_bytes, int lost,
+                 tg_stream_t stream) {
     TG_REQUIRE(a != nullptr, TG_ERR_INVALID_ARG, "null args");
     TG_REQUIRE(n >= 0 && n < (int64_t(1) << 30) && a->n_elems >= 0 && a->n_elems < (int64_t(1) << 30),
                TG_ERR_INVALID_ARG, "sort supports up to 2^30 pairs");
@@ -393,7 +394,21 @@ int tg_isect_sorted_lists(const tg_isect_args* a, void* order_ws, int64_t n, voi
     TG_REQUIRE(list_ws && aligned(list_ws, 16) && list_bytes >= tg::isect_lists_workspace_bytes(n, tb + cb),
                TG_ERR_WORKSPACE, "list workspace missing, misaligned or smaller than %zu bytes",
                tg::isect_lists_workspace_bytes(n, tb + cb));
-    return cuda_status(tg::launch_isect_lists(*a, order_ws, n, tb, tb + cb, list_ws, stream), "tg_isect_sorted_lists");
+    return cuda_status(tg::launch_isect_lists(*a, order_ws, n, tb, tb + cb, list_ws, lost, stream),
+                       "tg_isect_sorted_lists");
+}
+}  // namespace
+
+int tg_isect_sorted_lists(const tg_isect_args* a, void* order_ws, int64_t n, void* list_ws, size_t list_bytes,
+                          tg_stream_t stream) {
+    return sorted_lists(a, order_ws, n, list_ws, list_bytes, 0, stream);
+}
+
+int tg_isect_sorted_lookback_selftest(const tg_isect_args* a, void* order_ws, int64_t n, void* list_ws,
+                                      size_t list_bytes, int32_t sort, tg_stream_t stream) {
+    TG_REQUIRE(a != nullptr && (sort == 1 || sort == 2), TG_ERR_INVALID_ARG, "bad sort %d", sort);
+    TG_REQUIRE((sort == 1 ? a->n_elems : n) > 16384, TG_ERR_INVALID_ARG, "more than 16384 entries or intersections");
+    return sorted_lists(a, order_ws, n, list_ws, list_bytes, sort, stream);
 }
 
 size_t tg_tile_order_workspace_bytes(int64_t n_tiles) { return tg::tile_order_workspace_bytes(std::max<int64_t>(n_tiles, 0)); }

@@ -538,7 +538,8 @@ __global__ void __launch_bounds__(kSmallThreads) order_small_kernel(const float*
     if (lane < items) chunks[lane] = incl - v;
 }
 
-// Intersections of each chunk of the depth order.
+// Intersections of each chunk of the depth order.  (Here and below an id that is no entry's is passed over: a sort whose
+// look-back gave up leaves places unwritten.)
 __global__ void __launch_bounds__(256) order_sums_kernel(const uint32_t* __restrict__ ids,
                                                          const int32_t* __restrict__ counts, int64_t n,
                                                          int64_t* chunks) {
@@ -547,7 +548,8 @@ __global__ void __launch_bounds__(256) order_sums_kernel(const uint32_t* __restr
 #pragma unroll
     for (int i = 0; i < kOrderChunk; i += 256) {
         const int64_t k = (int64_t)blockIdx.x * kOrderChunk + i + threadIdx.x;
-        if (k < n) local += counts[ids[k]];
+        const uint32_t e = k < n ? ids[k] : 0xffffffffu;
+        if ((int64_t)e < n) local += counts[e];
     }
     int64_t total;
     block_excl_scan(local, s_warp, total);
@@ -597,8 +599,8 @@ cudaError_t launch_isect_order(const tg_isect_args& a, void* workspace, cudaStre
     return cudaGetLastError();
 }
 
-// The entries by depth and the offsets of its chunks.
-cudaError_t launch_entry_sort(const tg_isect_args& a, const OrderWorkspace& w, cudaStream_t s) {
+// The entries by depth and the offsets of its chunks.  lost: nobody takes the first tile of the first pass.
+cudaError_t launch_entry_sort(const tg_isect_args& a, const OrderWorkspace& w, bool lost, cudaStream_t s) {
     const int64_t E = a.n_elems, chunks = (E + kOrderChunk - 1) / kOrderChunk;
     cudaError_t e;
     if (E <= kSmallSort) {
@@ -614,8 +616,9 @@ cudaError_t launch_entry_sort(const tg_isect_args& a, const OrderWorkspace& w, c
             cudaSuccess)
             return e;
         const int64_t tiles = (E + kSortTile - 1) / kSortTile;
+        if (lost) set_u32_kernel<<<1, 1, 0, s>>>(w.counter, 1u);
         for (int p = 0; p < kDepthPasses; ++p)
-            order_pass_kernel<<<(unsigned)tiles, kSortThreads, smem, s>>>(
+            order_pass_kernel<<<(unsigned)(tiles - (lost && p == 0)), kSortThreads, smem, s>>>(
                 a.depths, w.keys[(p + 1) & 1], w.ids[(p + 1) & 1], w.keys[p & 1], w.ids[p & 1], E, p,
                 w.hist + p * kRadix, w.status + (size_t)p * tiles * kRadix, w.counter + p, w.counter + kDepthPasses);
         order_sums_kernel<<<(unsigned)chunks, 256, 0, s>>>(w.ids[1], a.tiles_per_gauss, E, w.chunks);
@@ -683,7 +686,7 @@ __global__ void __launch_bounds__(256) isect_expand_kernel(tg_isect_args a, cons
         cnt[i] = 0;
         if (k < a.n_elems) {
             const uint32_t e = order[k];
-            const int32_t r = a.radii[e];
+            const int32_t r = (int64_t)e < a.n_elems ? a.radii[e] : 0;
             uint32_t tw, th;
             if (r > 0 && camera_grid(a, e, tw, th)) {
                 const float2 m = reinterpret_cast<const float2*>(a.means2d)[e];
@@ -788,7 +791,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) list_pass_kernel(const uint32
                                                                  const uint32_t* __restrict__ ids_in,
                                                                  uint32_t* __restrict__ keys_out,
                                                                  uint32_t* __restrict__ ids_out,
-                                                                 const float* __restrict__ depths,
+                                                                 const float* __restrict__ depths, int64_t n_elems,
                                                                  int64_t* __restrict__ isect_ids,
                                                                  int32_t* __restrict__ flatten_ids, int64_t n,
                                                                  int shift, int bits, const uint32_t* hist,
@@ -800,7 +803,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) list_pass_kernel(const uint32
         },
         [&](int64_t i, uint32_t k, uint32_t v) {
             if constexpr (kLast) {
-                const bool pad = v == 0xffffffffu;
+                const bool pad = (int64_t)v >= n_elems;  // (padding has the id 0xffffffff)
                 const uint32_t low = pad ? 0xffffffffu : __float_as_uint(__ldg(depths + v));
                 isect_ids[i] = (int64_t)(((uint64_t)k << 32) | low);
                 flatten_ids[i] = pad ? 0 : (int32_t)v;
@@ -812,8 +815,9 @@ __global__ void __launch_bounds__(kSortThreads, 4) list_pass_kernel(const uint32
         n, shift, bits, hist, status, counter, error);
 }
 
+// lost: the sort whose first tile nobody takes, as in sort_lookback_selftest (1: the entries', 2: the lists', 0: none).
 cudaError_t launch_isect_lists(const tg_isect_args& a, void* order_ws, int64_t n, int tile_bits, int key_bits, void* ws,
-                               cudaStream_t s) {
+                               int lost, cudaStream_t s) {
     const int64_t E = a.n_elems;
     if (n == 0) return cudaSuccess;
     const int passes = list_passes(key_bits), pass_bits = list_pass_bits(key_bits);
@@ -822,7 +826,7 @@ cudaError_t launch_isect_lists(const tg_isect_args& a, void* order_ws, int64_t n
     cudaError_t e = cudaMemsetAsync(ws, 0, w.zeroed, s);
     if (e != cudaSuccess) return e;
     if (E > 0) {
-        if ((e = launch_entry_sort(a, o, s)) != cudaSuccess) return e;
+        if ((e = launch_entry_sort(a, o, lost == 1, s)) != cudaSuccess) return e;
         isect_expand_kernel<<<(unsigned)((E + kOrderChunk - 1) / kOrderChunk), 256, 0, s>>>(
             a, o.ids[1], o.chunks, n, tile_bits, passes, pass_bits, w.keys[0], w.ids[0], w.hist);
         note_launches(1);
@@ -840,11 +844,12 @@ cudaError_t launch_isect_lists(const tg_isect_args& a, void* order_ws, int64_t n
             cudaSuccess)
         return e;
     const int64_t tiles = (n + kSortTile - 1) / kSortTile;
+    if (lost == 2) set_u32_kernel<<<1, 1, 0, s>>>(w.counter, 1u);
     for (int p = 0; p < passes; ++p) {
         const int shift = p * pass_bits, bits = std::min(pass_bits, key_bits - shift);
         const auto fn = p == passes - 1 ? list_pass_kernel<true> : list_pass_kernel<false>;
-        fn<<<(unsigned)tiles, kSortThreads, smem, s>>>(w.keys[p & 1], w.ids[p & 1], w.keys[(p + 1) & 1],
-                                                       w.ids[(p + 1) & 1], a.depths, a.isect_ids, a.flatten_ids, n,
+        fn<<<(unsigned)(tiles - (lost == 2 && p == 0)), kSortThreads, smem, s>>>(w.keys[p & 1], w.ids[p & 1], w.keys[(p + 1) & 1],
+                                                       w.ids[(p + 1) & 1], a.depths, E, a.isect_ids, a.flatten_ids, n,
                                                        shift, bits, w.hist + p * kRadix,
                                                        w.status + (size_t)p * tiles * kRadix, w.counter + p,
                                                        w.counter + 4);

@@ -83,6 +83,8 @@ constexpr size_t sort_pass_smem() {
 // One pass of a stable LSD radix sort over digit bits [shift, shift + bits), bits <= 8: the CTA takes the next
 // 4096-pair tile, ranks it, exchanges it through shared memory and writes each digit's run where the digit's earlier
 // pairs end.  load(pos, key, value) / store(pos, key, value); hist: the pass's digit counts over all keys.
+// After a look-back that gave up, some places of the output are not written, and the next pass finds digits there that
+// hist has not counted: its places are held below n.
 template <class Key, class Load, class Store>
 __device__ __forceinline__ void sort_pass(Load load, Store store, int64_t n, int shift, int bits,
                                           const uint32_t* __restrict__ hist, uint32_t* status, uint32_t* tile_counter,
@@ -165,7 +167,8 @@ __device__ __forceinline__ void sort_pass(Load load, Store store, int64_t n, int
     const int tile_n = rem < kSortTile ? (int)rem : kSortTile;
     for (int j = tid; j < tile_n; j += kSortThreads) {
         const Key key = s_keys[j];
-        store((int64_t)(s_gbase[(uint32_t)(key >> shift) & digit_mask] + (uint32_t)j), key, s_vals[j]);
+        const int64_t pos = (int64_t)(s_gbase[(uint32_t)(key >> shift) & digit_mask] + (uint32_t)j);
+        if (pos < n) store(pos, key, s_vals[j]);
     }
 }
 
