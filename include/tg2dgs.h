@@ -276,7 +276,8 @@ TG_API int tg_isect_emit(const tg_isect_args* a, tg_stream_t stream);
  * tg_isect_sorted_lists: the entries' order, then isect_ids and flatten_ids [n],
  * n = *n_isects, from the same inputs and the counts of the first call; in
  * capacity mode (overflow != NULL) n = capacity and the tail as described at
- * `capacity`.  order_ws: what tg_isect_sorted_count filled, of
+ * `capacity`.  order_ws: what tg_isect_sorted_count filled (one call's worth:
+ * count again before the next lists), of
  * tg_isect_sorted_order_bytes(n_elems) bytes; list_ws:
  * tg_isect_sorted_lists_bytes(n, tile_bits + camera_bits) bytes, both 16-byte
  * aligned.  n_elems and n below 2^30. */
@@ -285,6 +286,13 @@ TG_API int tg_isect_sorted_count(const tg_isect_args* a, void* order_ws, size_t 
 TG_API size_t tg_isect_sorted_lists_bytes(int64_t n, int32_t key_bits);
 TG_API int tg_isect_sorted_lists(const tg_isect_args* a, void* order_ws, int64_t n, void* list_ws, size_t list_bytes,
                                  tg_stream_t stream);
+
+/* Waits for the stream; TG_ERR_TIMEOUT if a bounded look-back wait of the sorts
+ * of the last tg_isect_sorted_lists on these workspaces gave up (its lists are
+ * then not to be used), TG_OK otherwise.  Sizes as given to that call; key_bits
+ * = tile_bits + camera_bits.  Synchronising: for checks and tests. */
+TG_API int tg_isect_sorted_status(const void* order_ws, int64_t n_elems, const void* list_ws, int64_t n,
+                                  int32_t key_bits, tg_stream_t stream);
 
 /* Diagnostic, as tg_sort_lookback_selftest: tg_isect_sorted_lists where nobody
  * takes the first 4096 pairs of the entries' depth sort (sort = 1) or of the
@@ -302,6 +310,11 @@ TG_API int tg_isect_sorted_lookback_selftest(const tg_isect_args* a, void* order
 TG_API size_t tg_tile_order_workspace_bytes(int64_t n_tiles);
 TG_API int tg_tile_order(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, const int64_t* n_isects_dev,
                          int32_t* order, void* ws, size_t ws_bytes, tg_stream_t stream);
+/* As tg_isect_sorted_status, for the last tg_tile_order on ws. */
+TG_API int tg_tile_order_status(const void* ws, int64_t n_tiles, tg_stream_t stream);
+/* As tg_isect_sorted_lookback_selftest, for more than 16,384 tiles. */
+TG_API int tg_tile_order_lookback_selftest(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, int32_t* order,
+                                           void* ws, size_t ws_bytes, tg_stream_t stream);
 
 /* Stable LSD onesweep radix sort of (int64 key, int32 value) pairs on key bits
  * [0, end_bit), ping-ponging between (keys, vals) and (keys_alt, vals_alt).

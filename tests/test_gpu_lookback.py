@@ -8,7 +8,7 @@ import pytest
 import torch
 
 from textured_gaussians_b200 import _backend as B
-from textured_gaussians_b200.cuda._wrapper import isect_tiles
+from textured_gaussians_b200.cuda._wrapper import isect_tiles, tile_order_heaviest_first
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -63,3 +63,48 @@ def test_lists_stay_in_range_and_the_next_call_is_right(lost):
     c.lists()
     _, ids, flat = isect_tiles(*inputs, TILE, TW, TH)
     assert torch.equal(c.ids, ids) and torch.equal(c.flat, flat)
+
+
+def _status(c):
+    return c.L.tg_isect_sorted_status(B.ptr(c.order_ws), E, B.ptr(c.list_ws), c.n, KEY_BITS, c.st)
+
+
+@pytest.mark.parametrize("lost", [1, 2])
+def test_lists_report_it(lost):
+    inputs = _entries()
+    c = Call(*inputs)
+    c.lists()
+    assert _status(c) == 0
+    c.count()
+    c.lists(lost)
+    assert _status(c) == -5 and b"gave up" in c.L.tg_last_error()
+    c.count()
+    c.lists()
+    assert _status(c) == 0
+    assert torch.equal(isect_tiles(*inputs, TILE, TW, TH, check=True)[2], c.flat)
+
+
+@pytest.mark.parametrize("entries", [0, 5, 16384, 16385])
+def test_status_of_every_size(entries):
+    """The sizes whose entries one CTA sorts keep no flag: nothing else of the scratch is taken for one."""
+    args = [x[:, :entries].contiguous() for x in _entries()]
+    for sort in (True, False):
+        isect_tiles(*args, TILE, TW, TH, sort=sort, check=True)
+
+
+@pytest.mark.parametrize("n_tiles", [1, 16384, 16385, 50000])
+def test_tile_order_reports_it(n_tiles):
+    off = torch.arange(n_tiles, dtype=torch.int32, device=DEV) * 3
+    total = 3 * n_tiles
+    want = torch.arange(n_tiles, dtype=torch.int32, device=DEV)
+    assert torch.equal(tile_order_heaviest_first(off, total, check=True), want)
+    L, st = B.lib(), B.stream_of(off)
+    ws = torch.full((L.tg_tile_order_workspace_bytes(n_tiles),), 0xff, dtype=torch.uint8, device=DEV)
+    order = torch.empty_like(off)
+    rc = L.tg_tile_order_lookback_selftest(B.ptr(off), n_tiles, total, B.ptr(order), B.ptr(ws), ws.numel(), st)
+    if n_tiles <= 16384:
+        assert rc == -1
+    else:
+        assert rc == 0 and L.tg_tile_order_status(B.ptr(ws), n_tiles, st) == -5
+    assert L.tg_tile_order(B.ptr(off), n_tiles, total, None, B.ptr(order), B.ptr(ws), ws.numel(), st) == 0
+    assert L.tg_tile_order_status(B.ptr(ws), n_tiles, st) == 0 and torch.equal(order, want)

@@ -131,7 +131,10 @@ def lib() -> ctypes.CDLL:
                 ("tg_isect_sorted_lists", [ctypes.POINTER(IsectArgs), P, I64, P, ctypes.c_size_t, P]),
                 ("tg_isect_sorted_lookback_selftest",
                  [ctypes.POINTER(IsectArgs), P, I64, P, ctypes.c_size_t, I32, P]),
+                ("tg_isect_sorted_status", [P, I64, P, I64, I32, P]),
                 ("tg_tile_order", [P, I64, I64, P, P, P, ctypes.c_size_t, P]),
+                ("tg_tile_order_status", [P, I64, P]),
+                ("tg_tile_order_lookback_selftest", [P, I64, I64, P, P, ctypes.c_size_t, P]),
                 ("tg_sort_pairs", [P, P, P, P, I64, I32, P, ctypes.c_size_t, ctypes.POINTER(I32), P]),
                 ("tg_sort_status", [P, I64, I32, P]),
                 ("tg_sort_lookback_selftest", [P, P, P, P, P, ctypes.c_size_t, P]),

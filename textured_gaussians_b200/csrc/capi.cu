@@ -29,7 +29,10 @@ cudaError_t launch_isect_lists(const tg_isect_args& a, void* order_ws, int64_t n
                                int lost, cudaStream_t s);
 size_t tile_order_workspace_bytes(int64_t n_tiles);
 cudaError_t launch_tile_order(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, const int64_t* n_dev,
-                              int32_t* order, void* ws, cudaStream_t s);
+                              int32_t* order, void* ws, bool lost, cudaStream_t s);
+const uint32_t* entry_sort_error(const void* order_ws, int64_t E);
+const uint32_t* list_sort_error(const void* list_ws, int64_t n, int key_bits);
+const uint32_t* tile_order_error(const void* ws, int64_t n_tiles);
 uint32_t* sort_error_flag(void* workspace, int64_t n, int end_bit);
 int sort_lookback_selftest(int64_t* keys, int32_t* vals, int64_t* keys_alt, int32_t* vals_alt, void* workspace,
                            size_t ws_bytes, cudaStream_t s, cudaError_t& cerr);
@@ -413,15 +416,53 @@ int tg_isect_sorted_lookback_selftest(const tg_isect_args* a, void* order_ws, in
 
 size_t tg_tile_order_workspace_bytes(int64_t n_tiles) { return tg::tile_order_workspace_bytes(std::max<int64_t>(n_tiles, 0)); }
 
-int tg_tile_order(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, const int64_t* n_isects_dev,
-                  int32_t* order, void* ws, size_t ws_bytes, tg_stream_t stream) {
+namespace {
+int tile_order(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, const int64_t* n_isects_dev, int32_t* order,
+               void* ws, size_t ws_bytes, bool lost, tg_stream_t stream) {
     TG_REQUIRE(n_tiles >= 0 && n_tiles < (int64_t(1) << 30) && n_isects >= 0, TG_ERR_INVALID_ARG, "bad sizes");
     if (n_tiles == 0) return TG_OK;
     TG_REQUIRE(offsets && order && ws && aligned(ws, 16), TG_ERR_INVALID_ARG, "null or misaligned pointer");
     TG_REQUIRE(ws_bytes >= tg::tile_order_workspace_bytes(n_tiles), TG_ERR_WORKSPACE, "workspace smaller than %zu bytes",
                tg::tile_order_workspace_bytes(n_tiles));
-    return cuda_status(tg::launch_tile_order(offsets, n_tiles, n_isects, n_isects_dev, order, ws, stream),
+    return cuda_status(tg::launch_tile_order(offsets, n_tiles, n_isects, n_isects_dev, order, ws, lost, stream),
                        "tg_tile_order");
+}
+
+// TG_ERR_TIMEOUT if one of the flags (NULL: none) is set once the stream's work is done.
+int read_flags(std::initializer_list<const uint32_t*> flags, const char* what, tg_stream_t stream) {
+    cudaError_t e = cudaStreamSynchronize(stream);
+    for (const uint32_t* f : flags) {
+        uint32_t h = 0;
+        if (e == cudaSuccess && f != nullptr) e = cudaMemcpy(&h, f, sizeof(h), cudaMemcpyDeviceToHost);
+        TG_REQUIRE(h == 0, TG_ERR_TIMEOUT, "%s: a look-back wait gave up", what);
+    }
+    return cuda_status(e, what);
+}
+}  // namespace
+
+int tg_tile_order(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, const int64_t* n_isects_dev,
+                  int32_t* order, void* ws, size_t ws_bytes, tg_stream_t stream) {
+    return tile_order(offsets, n_tiles, n_isects, n_isects_dev, order, ws, ws_bytes, false, stream);
+}
+
+int tg_tile_order_lookback_selftest(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, int32_t* order, void* ws,
+                                    size_t ws_bytes, tg_stream_t stream) {
+    TG_REQUIRE(n_tiles > 16384, TG_ERR_INVALID_ARG, "more than 16384 tiles");
+    return tile_order(offsets, n_tiles, n_isects, nullptr, order, ws, ws_bytes, true, stream);
+}
+
+int tg_isect_sorted_status(const void* order_ws, int64_t n_elems, const void* list_ws, int64_t n, int32_t key_bits,
+                           tg_stream_t stream) {
+    TG_REQUIRE(n_elems >= 0 && n >= 0 && key_bits >= 1 && key_bits <= 32, TG_ERR_INVALID_ARG, "bad sizes");
+    if (n == 0) return TG_OK;  // (nothing was sorted)
+    TG_REQUIRE((order_ws || n_elems == 0) && list_ws, TG_ERR_INVALID_ARG, "null workspace");
+    return read_flags({tg::entry_sort_error(order_ws, n_elems), tg::list_sort_error(list_ws, n, key_bits)},
+                      "tg_isect_sorted_lists", stream);
+}
+
+int tg_tile_order_status(const void* ws, int64_t n_tiles, tg_stream_t stream) {
+    TG_REQUIRE(n_tiles >= 0 && (ws || n_tiles == 0), TG_ERR_INVALID_ARG, "null workspace");
+    return read_flags({tg::tile_order_error(ws, n_tiles)}, "tg_tile_order", stream);
 }
 
 int tg_sort_lookback_selftest(int64_t* keys, int32_t* vals, int64_t* keys_alt, int32_t* vals_alt, void* workspace,

@@ -12,8 +12,9 @@
 // is a single kernel whose CTAs take 4096-key tiles in launch order, rank the
 // keys with warp ballots, publish their digit counts and resolve their
 // global digit offsets by decoupled look-back over earlier tiles (sort.cuh).
-// Every look-back wait is bounded; a wait that gives up raises a workspace
-// error flag that the host turns into TG_ERR_TIMEOUT.
+// Every look-back wait is bounded; a wait that gives up raises an error flag in
+// the sort's workspace, which tg_sort_status, tg_isect_sorted_status and
+// tg_tile_order_status turn into TG_ERR_TIMEOUT.
 //
 // Sorted intersection lists (the renderer's path) do not sort the 64-bit keys.
 // An entry's intersections share its depth, so the entries are sorted by depth
@@ -858,6 +859,17 @@ cudaError_t launch_isect_lists(const tg_isect_args& a, void* order_ws, int64_t n
     return cudaGetLastError();
 }
 
+// Where the host finds whether a look-back of the call's sorts gave up (NULL: the size takes a sort without any).
+const uint32_t* entry_sort_error(const void* order_ws, int64_t E) {
+    return E > kSmallSort ? carve_order_workspace(const_cast<void*>(order_ws), E).counter + kDepthPasses : nullptr;
+}
+const uint32_t* list_sort_error(const void* list_ws, int64_t n, int key_bits) {
+    return n > 0 ? carve_list_workspace(const_cast<void*>(list_ws), n, list_passes(key_bits)).counter + 4 : nullptr;
+}
+const uint32_t* tile_order_error(const void* ws, int64_t n_tiles) {
+    return n_tiles > kSmallSort ? carve_list_workspace(const_cast<void*>(ws), n_tiles, 4).counter + 4 : nullptr;
+}
+
 // ------------------------------------------------------------------ tile order
 // Tiles by descending list length (stable): keys bound - length, bound >= every length.
 __device__ __forceinline__ uint32_t tile_key(const int32_t* __restrict__ offsets, int64_t t, int64_t n_tiles,
@@ -916,8 +928,9 @@ size_t tile_order_workspace_bytes(int64_t n_tiles) {
     return n_tiles <= kSmallSort ? 256 : carve_list_workspace(nullptr, n_tiles, 4).bytes;
 }
 
+// lost: nobody takes the first tile of the first pass, as in sort_lookback_selftest.
 cudaError_t launch_tile_order(const int32_t* offsets, int64_t n_tiles, int64_t n_isects, const int64_t* n_dev,
-                              int32_t* order, void* ws, cudaStream_t s) {
+                              int32_t* order, void* ws, bool lost, cudaStream_t s) {
     if (n_tiles == 0) return cudaSuccess;
     const uint32_t bound = (uint32_t)std::min<int64_t>(std::max<int64_t>(n_isects, 1), 0x7fffffff);
     int end_bit = 0;
@@ -942,9 +955,10 @@ cudaError_t launch_tile_order(const int32_t* offsets, int64_t n_tiles, int64_t n
     if ((e = cudaFuncSetAttribute(tile_order_pass_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
         cudaSuccess)
         return e;
+    if (lost) set_u32_kernel<<<1, 1, 0, s>>>(w.counter, 1u);
     for (int p = 0; p < passes; ++p) {
         uint32_t* out = p == passes - 1 ? reinterpret_cast<uint32_t*>(order) : w.ids[(p + 1) & 1];
-        tile_order_pass_kernel<<<(unsigned)tiles, kSortThreads, smem, s>>>(
+        tile_order_pass_kernel<<<(unsigned)(tiles - (lost && p == 0)), kSortThreads, smem, s>>>(
             offsets, n_isects, n_dev, bound, w.keys[p & 1], w.ids[p & 1], w.keys[(p + 1) & 1], out, n_tiles, p,
             std::min(8, end_bit - 8 * p), w.hist + p * kRadix, w.status + (size_t)p * tiles * kRadix, w.counter + p,
             w.counter + 4);

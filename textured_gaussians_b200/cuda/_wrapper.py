@@ -374,6 +374,7 @@ def isect_tiles(
     gaussian_ids: Optional[Tensor] = None,
     *,
     view_table=None,
+    check: bool = False,
 ) -> Tuple[Tensor, Tensor, Tensor]:
     """Maps projected Gaussians to intersecting tiles (reference: cuda/_wrapper.py:349-420).
 
@@ -381,7 +382,9 @@ def isect_tiles(
     flatten_ids int32 [n_isects])``, sorted stably by isect id when ``sort``.
     ``view_table`` (batching form, :class:`textured_gaussians_b200.batch.ViewTable`)
     gives every camera its own tile grid; tile_width / tile_height are then
-    ignored and the key's tile bits come from the largest grid.
+    ignored and the key's tile bits come from the largest grid.  ``check=True``
+    waits for the sort and raises if one of its bounded look-back waits gave up
+    (not while a graph is captured).
     """
     if view_table is not None:
         tile_width, tile_height = view_table.key_tiles, 1
@@ -426,6 +429,7 @@ def isect_tiles(
         B.call("tg_isect_count", stream, L.tg_isect_count, ctypes.byref(a), stream)
     plan = active_plan()
     capture = plan is not None and plan.mode == "capture"
+    assert not (capture and check), "check reads the sort's status on the host"
     if capture:  # no host read: capacity-sized keys (tail padded to sort last), device count attached to flatten_ids
         n_isects = plan.next_capacity()
         a.capacity, a.overflow = n_isects, B.ptr(plan.new_flag(dev))
@@ -442,10 +446,13 @@ def isect_tiles(
             list_ws = torch.empty((wsb,), dtype=torch.uint8, device=dev)
             B.call("tg_isect_sorted_lists", stream, L.tg_isect_sorted_lists, ctypes.byref(a), B.ptr(ws), n_isects,
                    B.ptr(list_ws), wsb, stream)
+            if check:
+                B.check(L.tg_isect_sorted_status(B.ptr(ws), E, B.ptr(list_ws), n_isects, key_bits, stream),
+                        "tg_isect_sorted_status")
         else:
             B.call("tg_isect_emit", stream, L.tg_isect_emit, ctypes.byref(a), stream)
             if sort:
-                isect_ids, flatten_ids = sort_pairs(isect_ids, flatten_ids, 32 + key_bits)
+                isect_ids, flatten_ids = sort_pairs(isect_ids, flatten_ids, 32 + key_bits, check)
     if capture:
         flatten_ids._tg_n_isects = n_dev
     return tiles_per_gauss, isect_ids, flatten_ids
@@ -504,9 +511,10 @@ def isect_offset_encode_views(isect_ids: Tensor, view_table) -> Tensor:
 
 
 @torch.no_grad()
-def tile_order_heaviest_first(isect_offsets: Tensor, n_isects: int) -> Tensor:
+def tile_order_heaviest_first(isect_offsets: Tensor, n_isects: int, check: bool = False) -> Tensor:
     """Permutation of the flat tiles by descending intersection count (stable),
-    so the longest tiles start first and the tail of the launch is short."""
+    so the longest tiles start first and the tail of the launch is short.
+    ``check`` as in :func:`isect_tiles`."""
     flat = isect_offsets.reshape(-1).to(torch.int32).contiguous()
     n = flat.numel()
     order = torch.empty((n,), dtype=torch.int32, device=flat.device)
@@ -519,6 +527,8 @@ def tile_order_heaviest_first(isect_offsets: Tensor, n_isects: int) -> Tensor:
     ws = torch.empty((wsb,), dtype=torch.uint8, device=flat.device)
     st = B.stream_of(flat)
     B.call("tg_tile_order", st, L.tg_tile_order, B.ptr(flat), n, bound, B.ptr(n_dev), B.ptr(order), B.ptr(ws), wsb, st)
+    if check:
+        B.check(L.tg_tile_order_status(B.ptr(ws), n, st), "tg_tile_order_status")
     return order
 
 
