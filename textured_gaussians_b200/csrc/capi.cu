@@ -344,7 +344,8 @@ int tg_isect_emit(const tg_isect_args* a, tg_stream_t stream) {
     }
     if (a->n_elems == 0 && !(a->overflow && a->capacity > 0)) return TG_OK;
     if (a->n_elems > 0) {
-        TG_REQUIRE(a->means2d && a->radii && a->depths && a->cum_tiles && a->isect_ids && a->flatten_ids,
+        const bool no_room = a->overflow && a->capacity == 0;  // nothing is written but the overflow
+        TG_REQUIRE(a->means2d && a->radii && a->depths && a->cum_tiles && (no_room || (a->isect_ids && a->flatten_ids)),
                    TG_ERR_INVALID_ARG, "null pointer");
         TG_REQUIRE(a->camera_ids != nullptr || a->N > 0, TG_ERR_INVALID_ARG, "dense layout needs N > 0");
     }
@@ -386,7 +387,8 @@ int sorted_lists(const tg_isect_args* a, void* order_ws, int64_t n, void* list_w
                TG_ERR_INVALID_ARG, "sort supports up to 2^30 pairs");
     TG_REQUIRE(!a->overflow || (a->capacity == n && a->n_isects), TG_ERR_INVALID_ARG,
                "capacity mode needs n = capacity and n_isects");
-    if (n == 0) return TG_OK;
+    if (n == 0)  // nothing to list, but in capacity mode something to report
+        return cuda_status(tg::launch_isect_lists(*a, nullptr, 0, 0, 1, nullptr, 0, stream), "tg_isect_sorted_lists");
     const int tb = bit_width((int64_t)a->tile_width * a->tile_height), cb = bit_width(a->n_cameras);
     TG_REQUIRE(a->tile_width > 0 && a->tile_height > 0 && a->n_cameras > 0 && tb + cb <= 32, TG_ERR_INVALID_ARG,
                "bad tile grid");

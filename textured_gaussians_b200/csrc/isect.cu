@@ -786,6 +786,11 @@ __global__ void __launch_bounds__(256) isect_expand_pad_kernel(const int64_t* n_
     ids[i] = 0xffffffffu;
 }
 
+// A capacity of zero intersections: any at all are too many.
+__global__ void overflow_if_any_kernel(const int64_t* n_dev, uint32_t* overflow) {
+    if (*n_dev > 0) atomicOr(overflow, 1u);
+}
+
 // One pass over the (camera, tile) keys; the last writes the 64-bit keys and the entries.
 template <bool kLast>
 __global__ void __launch_bounds__(kSortThreads, 4) list_pass_kernel(const uint32_t* __restrict__ keys_in,
@@ -820,7 +825,12 @@ __global__ void __launch_bounds__(kSortThreads, 4) list_pass_kernel(const uint32
 cudaError_t launch_isect_lists(const tg_isect_args& a, void* order_ws, int64_t n, int tile_bits, int key_bits, void* ws,
                                int lost, cudaStream_t s) {
     const int64_t E = a.n_elems;
-    if (n == 0) return cudaSuccess;
+    if (n == 0) {
+        if (!a.overflow) return cudaSuccess;
+        overflow_if_any_kernel<<<1, 1, 0, s>>>(a.n_isects, a.overflow);
+        note_launches(1);
+        return cudaGetLastError();
+    }
     const int passes = list_passes(key_bits), pass_bits = list_pass_bits(key_bits);
     const OrderWorkspace o = carve_order_workspace(order_ws, E);
     const ListWorkspace w = carve_list_workspace(ws, n, passes);

@@ -439,7 +439,7 @@ def isect_tiles(
             plan.sizes.append(n_isects)
     isect_ids = torch.empty((n_isects,), dtype=torch.int64, device=dev)
     flatten_ids = torch.empty((n_isects,), dtype=torch.int32, device=dev)
-    if n_isects:
+    if n_isects or capture:  # (a capacity of 0 has an overflow to report)
         a.isect_ids, a.flatten_ids = B.ptr(isect_ids), B.ptr(flatten_ids)
         if by_depth:
             wsb = L.tg_isect_sorted_lists_bytes(n_isects, key_bits)
