@@ -34,6 +34,7 @@ from . import _backend as B
 from .cuda._wrapper import (
     _FILTER_ADJOINT,
     _FullyFusedProjectionPacked2DGS,
+    gather_rows,
     isect_offset_encode_views,
     isect_tiles,
     n_isects_of,
@@ -169,7 +170,7 @@ def rasterization_textured_gaussians_batch(
         means.contiguous(), quats.contiguous(), scales.contiguous(), viewmats.contiguous(), Ks.contiguous(), 0, 0,
         eps2d, near_plane, far_plane, radius_clip, False, mode, (vt.views, ranges, max_range), *sh)
     camera_ids, gaussian_ids, radii, means2d, depths, ray_transforms, normals = proj[:7]
-    opac = opacities.index_select(0, gaussian_ids)
+    opac = gather_rows(opacities, gaussian_ids)
     if fuse:
         cols = proj[-1]
     elif sh_degree is not None:
@@ -178,7 +179,7 @@ def rasterization_textured_gaussians_batch(
         cols = spherical_harmonics(sh_degree, dirs, colors[gaussian_ids], masks=radii > 0)
         cols = torch.clamp_min(cols + 0.5, 0.0)
     else:
-        cols = colors.index_select(0, gaussian_ids)
+        cols = gather_rows(colors, gaussian_ids)
     if render_mode in ("RGB+D", "RGB+ED"):
         cols = torch.cat((cols, depths[..., None]), dim=-1)
     elif render_mode in ("D", "ED"):

@@ -39,6 +39,7 @@ from .cuda._wrapper import (
     depth_image,
     depth_image_supported,
     fully_fused_projection_2dgs,
+    gather_rows,
     isect_offset_encode,
     isect_tiles,
     n_isects_of,
@@ -90,7 +91,7 @@ def _prepare(means, quats, scales, opacities, colors, viewmats, Ks, width, heigh
         sh_degree=sh_degree if fuse else None)
     if packed:
         camera_ids, gaussian_ids, radii, means2d, depths, ray_transforms, normals = proj[:7]
-        opacities = opacities.index_select(0, gaussian_ids)  # (its adjoint adds with atomics instead of sorting the ids)
+        opacities = gather_rows(opacities, gaussian_ids)
     else:
         radii, means2d, depths, ray_transforms, normals = proj[:5]
         opacities = opacities.repeat(C, 1)
@@ -118,7 +119,7 @@ def _prepare(means, quats, scales, opacities, colors, viewmats, Ks, width, heigh
             colors = spherical_harmonics_shared(sh_degree, dirs, colors, masks=radii > 0)  # [C, N, 3]
         colors = torch.clamp_min(colors + 0.5, 0.0)
     elif colors.dim() == 2:
-        colors = colors.index_select(0, gaussian_ids) if packed else colors.expand(C, *([-1] * colors.dim()))
+        colors = gather_rows(colors, gaussian_ids) if packed else colors.expand(C, *([-1] * colors.dim()))
     elif packed:
         colors = colors[camera_ids, gaussian_ids, :]
 
