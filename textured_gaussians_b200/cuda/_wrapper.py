@@ -528,6 +528,8 @@ def tile_order_heaviest_first(isect_offsets: Tensor, n_isects: int, check: bool 
     n = flat.numel()
     order = torch.empty((n,), dtype=torch.int32, device=flat.device)
     if isinstance(n_isects, Tensor):  # device count (graph capture)
+        if n_isects.device != flat.device:
+            raise RuntimeError(f"offsets on {flat.device}, their count on {n_isects.device}")
         n_dev, bound = n_isects.reshape(1).to(torch.int64), (1 << 31) - 1
     else:
         n_dev, bound = None, int(n_isects)
