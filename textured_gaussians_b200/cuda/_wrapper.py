@@ -827,7 +827,13 @@ class _RasterizeToPixelsTextured(torch.autograd.Function):
         a.v_tex_coarse = B.ptr(v_coarse)
         v_prefix = torch.empty_like(ctx.aniso_prefix) if ctx.aniso_prefix is not None and want_tex else None
         a.v_aniso_prefix = B.ptr(v_prefix)
-        packed_rows = torch.empty((means2d.numel() // 2, 24), dtype=torch.float32, device=dev)
+        packed_rows = _scratch((means2d.numel() // 2, 24), torch.float32, dev)
+        if packed_rows is None:  # without the rows every upstream gradient has to be there
+            v_rc, v_ra, v_rn, v_rd, v_rm = (
+                torch.zeros(pshape + (k,), dtype=torch.float32, device=dev) if t is None else t
+                for t, k in zip((v_rc, v_ra, v_rn, v_rd, v_rm), (D, 1, 3, 1, 1)))
+            a.v_render_colors, a.v_render_alphas, a.v_render_normals = B.ptr(v_rc), B.ptr(v_ra), B.ptr(v_rn)
+            a.v_render_distort, a.v_render_median = B.ptr(v_rd), B.ptr(v_rm)
         a.v_packed = B.ptr(packed_rows)
         st = B.stream_of(means2d)
         B.call("tg_rasterize_bwd", st, B.lib().tg_rasterize_bwd, ctypes.byref(a), st)
