@@ -69,7 +69,12 @@ typedef struct {
     int64_t pix_base;                /* first flat pixel of the view */
 } tg_view;
 
-TG_API int tg_version(void);
+/* Version of the argument structs' layout, raised with every change to it: a
+ * host built against another header than the library has another number.
+ * 2: contrib_masks, entry_records and n_entries end tg_raster_fwd_args, which
+ * moves what follows it in tg_raster_bwd_args, and v_packed ends that. */
+#define TG_ABI_VERSION 2
+TG_API int tg_version(void); /* the library's TG_ABI_VERSION */
 TG_API const char* tg_last_error(void);
 /* Number of kernels this library has launched in this process (all devices,
  * all threads); lets a harness count the launches inside a timed region.

@@ -202,7 +202,7 @@ int check_raster_common(const tg_raster_fwd_args& a) {
 
 extern "C" {
 
-int tg_version(void) { return 1; }
+int tg_version(void) { return TG_ABI_VERSION; }
 
 const char* tg_last_error(void) { return g_last_error.c_str(); }
 
