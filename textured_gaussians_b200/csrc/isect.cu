@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(256) order_sums_kernel(const uint32_t* __restr
     for (int i = 0; i < kOrderChunk; i += 256) {
         const int64_t k = (int64_t)blockIdx.x * kOrderChunk + i + threadIdx.x;
         const uint32_t e = k < n ? ids[k] : 0xffffffffu;
-        if ((int64_t)e < n) local += counts[e];
+        if (e < (uint32_t)n) local += counts[e];
     }
     int64_t total;
     block_excl_scan(local, s_warp, total);
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(256) isect_expand_kernel(tg_isect_args a, cons
         cnt[i] = 0;
         if (k < a.n_elems) {
             const uint32_t e = order[k];
-            const int32_t r = (int64_t)e < a.n_elems ? a.radii[e] : 0;
+            const int32_t r = e < (uint32_t)a.n_elems ? a.radii[e] : 0;
             uint32_t tw, th;
             if (r > 0 && camera_grid(a, e, tw, th)) {
                 const float2 m = reinterpret_cast<const float2*>(a.means2d)[e];
@@ -797,7 +797,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) list_pass_kernel(const uint32
                                                                  const uint32_t* __restrict__ ids_in,
                                                                  uint32_t* __restrict__ keys_out,
                                                                  uint32_t* __restrict__ ids_out,
-                                                                 const float* __restrict__ depths, int64_t n_elems,
+                                                                 const float* __restrict__ depths, uint32_t n_elems,
                                                                  int64_t* __restrict__ isect_ids,
                                                                  int32_t* __restrict__ flatten_ids, int64_t n,
                                                                  int shift, int bits, const uint32_t* hist,
@@ -809,7 +809,7 @@ __global__ void __launch_bounds__(kSortThreads, 4) list_pass_kernel(const uint32
         },
         [&](int64_t i, uint32_t k, uint32_t v) {
             if constexpr (kLast) {
-                const bool pad = (int64_t)v >= n_elems;  // (padding has the id 0xffffffff)
+                const bool pad = v >= n_elems;  // (padding has the id 0xffffffff)
                 const uint32_t low = pad ? 0xffffffffu : __float_as_uint(__ldg(depths + v));
                 isect_ids[i] = (int64_t)(((uint64_t)k << 32) | low);
                 flatten_ids[i] = pad ? 0 : (int32_t)v;
@@ -860,7 +860,7 @@ cudaError_t launch_isect_lists(const tg_isect_args& a, void* order_ws, int64_t n
         const int shift = p * pass_bits, bits = std::min(pass_bits, key_bits - shift);
         const auto fn = p == passes - 1 ? list_pass_kernel<true> : list_pass_kernel<false>;
         fn<<<(unsigned)(tiles - (lost == 2 && p == 0)), kSortThreads, smem, s>>>(w.keys[p & 1], w.ids[p & 1], w.keys[(p + 1) & 1],
-                                                       w.ids[(p + 1) & 1], a.depths, E, a.isect_ids, a.flatten_ids, n,
+                                                       w.ids[(p + 1) & 1], a.depths, (uint32_t)E, a.isect_ids, a.flatten_ids, n,
                                                        shift, bits, w.hist + p * kRadix,
                                                        w.status + (size_t)p * tiles * kRadix, w.counter + p,
                                                        w.counter + 4);

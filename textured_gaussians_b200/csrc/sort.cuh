@@ -167,8 +167,8 @@ __device__ __forceinline__ void sort_pass(Load load, Store store, int64_t n, int
     const int tile_n = rem < kSortTile ? (int)rem : kSortTile;
     for (int j = tid; j < tile_n; j += kSortThreads) {
         const Key key = s_keys[j];
-        const int64_t pos = (int64_t)(s_gbase[(uint32_t)(key >> shift) & digit_mask] + (uint32_t)j);
-        if (pos < n) store(pos, key, s_vals[j]);
+        const uint32_t pos = s_gbase[(uint32_t)(key >> shift) & digit_mask] + (uint32_t)j;
+        store((int64_t)min(pos, (uint32_t)n - 1u), key, s_vals[j]);  // (a branch here: 57 -> 65 us for the last list pass)
     }
 }
 
