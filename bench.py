@@ -449,14 +449,17 @@ def _run_ours(args, rank, world, local, dev):
     peaks, peaks_kind = load_peaks()
     bwd_ms = statistics.mean(stages_bf16["tg_rasterize_bwd"])
     achieved = bwd_b / (bwd_ms / 1e3) / 1e9
-    roofline = {"kernel": "tg_rasterize_bwd (compositor adjoint: gradient zero-fill + adjoint kernel + densify)",
+    earlier = traffic_bytes(args, N, C, R, tile, depth)
+    measured_here = earlier is not None and args.traffic_bytes is None  # the workload the captures are of
+    roofline = {"kernel": "tg_rasterize_bwd (compositor adjoint: zero-fills + adjoint kernel + spread of its rows)",
                 "bound": "hbm", "achieved": round(achieved, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": round(achieved / peaks["hbm_gbs"], 4), "peak_source": peaks_kind,
-                "traffic": traffic_bytes(args, N, C, R, tile, depth), "algorithmic_bytes": bwd_b,
+                "traffic": ADJOINT_CALL_DRAM_BYTES if measured_here else earlier,
+                "traffic_earlier_form": earlier if measured_here else None, "algorithmic_bytes": bwd_b,
                 "launch_ms": round(bwd_ms, 4)}
     # the forward compositor beside it: algorithmic and (headline workload) measured bytes over its event time
     fwd_ms = statistics.mean(stages_bf16["tg_rasterize_fwd"])
-    fwd_traffic = FORWARD_KERNEL_DRAM_BYTES if traffic_bytes(args, N, C, R, tile, depth) is not None else None
+    fwd_traffic = FORWARD_CALL_DRAM_BYTES if measured_here else None
     roofline_fwd = {"kernel": "tg_rasterize_fwd (compositor forward)", "bound": "hbm",
                     "achieved": round(fwd_b / (fwd_ms / 1e3) / 1e9, 1), "peak": peaks["hbm_gbs"], "unit": "GB/s",
                     "frac": round(fwd_b / (fwd_ms / 1e3) / 1e9 / peaks["hbm_gbs"], 4), "traffic": fwd_traffic,
@@ -513,15 +516,19 @@ def _run_ours(args, rank, world, local, dev):
 
 # DRAM bytes of one compositor-adjoint call on the headline workload (1M splats, 32x32 textures, four 1600x1200
 # views, tile 8, batch depth 64), measured with ncu in one pass (dram__bytes_read.sum + dram__bytes_write.sum):
-# adjoint kernel 53.763 GB read + 9.741 GB written, densification kernel 0.288 + 0.022 GB; the gradient zero-fill
-# (a memset, not a kernel) writes its N * R^2 * 16 bytes.
+# adjoint kernel 33.876 GB read + 9.052 GB written, the pass that spreads the gradient rows 0.400 + 0.266 GB; the
+# zero-fills (memsets, not kernels) of the rows, 4,000,000 * 64 bytes, and of the texture gradient, 16.384 GB
+ADJOINT_CALL_DRAM_BYTES = 33.876109e9 + 9.051906e9 + 0.400016e9 + 0.266023e9 + 0.256e9 + 16.384e9
+# the forward on the same workload, same capture: compositor kernel 27.178 GB read + 1.116 GB written, packing of the
+# entry records 0.288 + 0.269 GB
+FORWARD_CALL_DRAM_BYTES = 27.178072e9 + 1.116073e9 + 0.288105e9 + 0.268758e9
+# the adjoint's kernels in the form with one warp per 8x4 block and no contributor bits, reported beside it: adjoint
+# kernel 53.763 GB read + 9.741 GB written, densification kernel 0.288 + 0.022 GB
 ADJOINT_KERNEL_DRAM_BYTES = 53.763221e9 + 9.741255e9 + 0.288009e9 + 0.021744e9
-# the forward compositor kernel on the same workload, same capture: 36.358 GB read + 0.806 GB written
-FORWARD_KERNEL_DRAM_BYTES = 36.358471e9 + 0.806166e9
 
 
 def traffic_bytes(args, N, C, R, tile, depth):
-    """Measured DRAM traffic of the adjoint call for the workload it was measured on, else the --traffic-bytes
+    """DRAM traffic of the adjoint call's earlier form for the workload it was measured on, else the --traffic-bytes
     value (None when absent)."""
     if args.traffic_bytes is not None:
         return args.traffic_bytes

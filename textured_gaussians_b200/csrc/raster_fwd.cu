@@ -6,8 +6,8 @@
 // (tg_raster_fwd_args.entry_records).  A warp is four groups of 4x2 pixels; staging leaves each group a bit list of
 // the batch's splats whose bounds meet it (group_mask), and the four groups walk their own lists, so one warp
 // iteration works on four splats.  A warp per 8x4 block and a box test took 1.13 iterations a listed splat on the
-// 1M-splat mixture, the groups take 0.34 (four 1600x1200 views: forward 9.2 -> 6.7 ms).  What bounds it: issue
-// (72-77 % of the cycles) at 64 registers.
+// 1M-splat mixture, the groups take 0.49 (four 1600x1200 views: forward 9.2 -> 6.7 ms).  What bounds it: issue (58-78 %
+// of the cycles from 100,000 splats on, 44-50 % of the warps resident at 64 registers) and the reads it waits for between.
 // Each pixel samples its splat's RGBA texture with one 16-byte (FP32), 8-byte (BF16/FP16) or 4-byte (FP8) load per
 // bilinear tap and reuses the four taps for the alpha scale and every colour channel.  Lists end early for saturated
 // pixels, and a square at the next batch boundary once all are.  The contribution statistics are reduced per group,
