@@ -302,9 +302,9 @@ TG_API int tg_isect_sorted_status(const void* order_ws, int64_t n_elems, const v
 /* Diagnostic, as tg_sort_lookback_selftest: tg_isect_sorted_lists where nobody
  * takes the first 4096 pairs of the entries' depth sort (sort = 1) or of the
  * lists' sort (sort = 2), so that every look-back of that pass waits for them
- * and gives up.  The lists come out wrong, with entries in range wherever
- * they are written (a place may be left unwritten).  More than 16,384 entries
- * (sort = 1) or intersections (2).  No counterpart in the reference. */
+ * and gives up.  The lists come out wrong, with entries in range.  More than
+ * 16,384 entries (sort = 1) or intersections (2).  No counterpart in the
+ * reference. */
 TG_API int tg_isect_sorted_lookback_selftest(const tg_isect_args* a, void* order_ws, int64_t n, void* list_ws,
                                              size_t list_bytes, int32_t sort, tg_stream_t stream);
 

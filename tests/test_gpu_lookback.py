@@ -65,6 +65,27 @@ def test_lists_stay_in_range_and_the_next_call_is_right(lost):
     assert torch.equal(c.ids, ids) and torch.equal(c.flat, flat)
 
 
+@pytest.mark.parametrize("lost", [1, 2])
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("spare", [None, 0, 5000])
+def test_every_place_holds_an_entry(lost, shift, spare):
+    """Also the places nothing was sorted into, whatever the buffer's alignment, with exact sizes (None) and in
+    capacity mode with so many places to spare: a compositor given such lists stays within the entries."""
+    c = Call(*_entries())
+    if spare is not None:
+        flag = torch.zeros((1,), dtype=torch.int32, device=DEV)
+        c.n += spare
+        c.a.capacity, c.a.overflow = c.n, B.ptr(flag)
+        c.list_ws = torch.full((c.L.tg_isect_sorted_lists_bytes(c.n, KEY_BITS),), 0xff, dtype=torch.uint8, device=DEV)
+        c.ids = torch.zeros((c.n,), dtype=torch.int64, device=DEV)
+        c.a.isect_ids = B.ptr(c.ids)
+    flat = torch.full((c.n + 4,), -1, dtype=torch.int32, device=DEV)[shift:shift + c.n]
+    c.a.flatten_ids = B.ptr(flat)
+    c.lists(lost)
+    torch.cuda.synchronize()
+    assert int(flat.min()) >= 0 and int(flat.max()) < E
+
+
 def _status(c):
     return c.L.tg_isect_sorted_status(B.ptr(c.order_ws), E, B.ptr(c.list_ws), c.n, KEY_BITS, c.st)
 

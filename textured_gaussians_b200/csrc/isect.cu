@@ -665,7 +665,8 @@ size_t isect_lists_workspace_bytes(int64_t n, int key_bits) {
 
 // Writes the intersections in depth order and counts their keys' digits.  A CTA expands 1024 entries: their tile
 // boxes go to shared memory, and each thread fills four consecutive list places at a time (one search for the
-// first, then stepping), so that the writes are whole vectors whatever the entries' sizes.
+// first, then stepping), so that the writes are whole vectors whatever the entries' sizes.  flatten_ids gets an entry
+// in every place beforehand, so that whoever reads the lists of a sort that gave up stays within the entries.
 __global__ void __launch_bounds__(256) isect_expand_kernel(tg_isect_args a, const uint32_t* __restrict__ order,
                                                            const int64_t* __restrict__ chunks, int64_t limit,
                                                            int tile_bits, int passes, int pass_bits,
@@ -724,6 +725,7 @@ __global__ void __launch_bounds__(256) isect_expand_kernel(tg_isect_args a, cons
     const int64_t base = chunks[blockIdx.x];
     const int64_t end = min(base + (int64_t)s_off[kOrderChunk], limit);
     const uint32_t digit_mask = (1u << pass_bits) - 1u;
+    const bool whole = (reinterpret_cast<uintptr_t>(a.flatten_ids) & 15) == 0;
     for (int64_t p4 = (base >> 2) + tid; p4 * 4 < end; p4 += 256) {  // four places from 4 * p4 on
         const int64_t lo = max(p4 * 4, base), hi = min(p4 * 4 + 4, end);
         uint32_t rel = (uint32_t)(lo - base);
@@ -755,6 +757,9 @@ __global__ void __launch_bounds__(256) isect_expand_kernel(tg_isect_args a, cons
         if (hi - lo == 4) {
             reinterpret_cast<uint4*>(keys)[p4] = make_uint4(key[0], key[1], key[2], key[3]);
             reinterpret_cast<uint4*>(ids)[p4] = make_uint4(id[0], id[1], id[2], id[3]);
+        }
+        if (hi - lo == 4 && whole) {
+            reinterpret_cast<int4*>(a.flatten_ids)[p4] = make_int4(0, 0, 0, 0);
         } else {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -762,8 +767,16 @@ __global__ void __launch_bounds__(256) isect_expand_kernel(tg_isect_args a, cons
                 if (pos >= lo && pos < hi) {
                     keys[pos] = key[q];
                     ids[pos] = id[q];
+                    a.flatten_ids[pos] = 0;
                 }
             }
+        }
+    }
+    if (blockIdx.x == gridDim.x - 1) {  // an entry sort that gave up can leave fewer intersections than were counted
+        const int64_t counted = a.overflow ? min(*a.n_isects, limit) : limit;
+        for (int64_t pos = end + tid; pos < counted; pos += 256) {
+            keys[pos] = ids[pos] = 0xffffffffu;
+            a.flatten_ids[pos] = 0;
         }
     }
     __syncthreads();
@@ -775,7 +788,7 @@ __global__ void __launch_bounds__(256) isect_expand_kernel(tg_isect_args a, cons
 // Capacity mode: the places past the valid count get the largest key (they sort last) and no entry.
 __global__ void __launch_bounds__(256) isect_expand_pad_kernel(const int64_t* n_dev, int64_t capacity, uint32_t pad_key,
                                                                int passes, int pass_bits, uint32_t* keys, uint32_t* ids,
-                                                               uint32_t* hist) {
+                                                               int32_t* flatten_ids, uint32_t* hist) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, n = min(max(*n_dev, (int64_t)0), capacity);
     if (i == 0 && n < capacity)
         for (int p = 0; p < passes; ++p)
@@ -784,6 +797,7 @@ __global__ void __launch_bounds__(256) isect_expand_pad_kernel(const int64_t* n_
     if (i < n || i >= capacity) return;
     keys[i] = pad_key;
     ids[i] = 0xffffffffu;
+    flatten_ids[i] = 0;
 }
 
 // A capacity of zero intersections: any at all are too many.
@@ -845,7 +859,7 @@ cudaError_t launch_isect_lists(const tg_isect_args& a, void* order_ws, int64_t n
     if (a.overflow) {
         const uint32_t pad = key_bits >= 32 ? 0xffffffffu : (1u << key_bits) - 1u;
         isect_expand_pad_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a.n_isects, n, pad, passes, pass_bits,
-                                                                           w.keys[0], w.ids[0], w.hist);
+                                                                           w.keys[0], w.ids[0], a.flatten_ids, w.hist);
         note_launches(1);
     }
     constexpr size_t smem = sort_pass_smem<uint32_t>();
