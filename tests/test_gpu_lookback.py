@@ -28,6 +28,7 @@ class Call:
     """One tg_isect_sorted_count / _lists pair on buffers of its own."""
 
     def __init__(self, xy, radii, depths):
+        self.inputs = (xy, radii, depths)  # (read by every call)
         self.L, self.st = B.lib(), B.stream_of(xy)
         u8 = lambda n: torch.full((n,), 0xff, dtype=torch.uint8, device=DEV)  # noqa: E731
         self.order_ws = u8(self.L.tg_isect_sorted_order_bytes(E))
