@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(256, TG_FWD_MIN_CTAS) raster_fwd_kernel(const 
 // another, and where every SM is full anyway that costs: 22.1 against 20.5 ms for 300k splats in two 1600x1200
 // views.  So only the first kLongTiles squares are taken so, the others four to a CTA, two warps each; and from
 // kFullSquares squares on, or where a batch is too deep for that, all take the other filters' kernel.
-constexpr int kFullSquares = 128 * kNumSMs;  // eight times what the device holds at once
+constexpr int kFullSquares = 128 * kNumSMs;  // eight times what the device holds at once (no size between the two timed)
 constexpr int kLongTiles = 3 * kNumSMs;  // of 1, 3 and 6 per SM (60k splats: 3.96, 3.25, 3.32 ms)
 constexpr size_t kMaxSmem = 227 * 1024;  // of a CTA
 constexpr int kAnisoWarps = 8;
